@@ -1,0 +1,853 @@
+// The recurrences of recurrent.cu for prompts and portions in bfloat16, by chunks of 64 tokens on the tensor cores:
+//
+//   S_t = a_t S_(t-1) + b_t k_t v_t^T          o_t = S_t^T q_t
+//
+// with the head's fixed decay (retention) or the gates of an mlstm.  With S_0 the state ahead of a chunk and
+// D(t, s) = a_(s+1) ... a_t b_s,
+//   o_t = D(t, 0) S_0^T q_t + sum_(s<=t) D(t, s) (q_t . k_s) v_s          S_n = D(n, 0) S_0 + sum_s D(n, s) k_s v_s^T
+// Token by token the recurrence is a chain over all tokens whose steps leave most of the chip idle; by chunks only the state
+// is a chain, one short step per 64 tokens:
+//   gates   (mlstm) a block per (sequence, head): every token's logarithms and running maximum
+//   state   a block per (sequence, head, some value columns) walks the chunks in order: four warps hold their share of S in
+//           registers and multiply, eight others stage the next chunk's scaled keys; S_0 of every chunk goes to scratch
+//   output  a block per (chunk, head), all at once
+// The state kernel is bound by what a block does per chunk (its products where heads are of 128, its stagers' copies of cosines
+// and sines where they are rotated), the output kernel by the latencies of eight to twelve warps a multiprocessor (tensor cores
+// busy a quarter of the time).  2,048 tokens of 32 heads, both kernels (and gates), us: heads of 64 rotated 491 token by token
+// (recurrent.cu), 75 here; with gates 731 and 87; heads of 128 rotated 1,165 and 236; with gates 1,264 and 160.
+//
+// Precision: what the recurrence holds in 32 bits stays so.  A float32 operand enters the products as three bfloat16 terms
+// (its 24 bits), a pair of such operands as the six products that reach 2^-24; bfloat16 operands enter as they are.  The
+// tensor cores cut their sums off where float32 rounds, so no sum of theirs is longer than one step of 16 terms: each
+// starts from zero, least terms first, and joins the float32 accumulator by an ordinary addition.  The decays' logarithms add up
+// in float64, so that their differences keep their digits.  Distance from the recurrence in float64, 2,048 tokens, outputs / state:
+// 1.3e-7 / 1.0e-7 with a fixed decay (token by token 2.2e-7 / 2.2e-7), 2.0e-7 / 1.7e-7 with gates (3.9e-7 / 3.0e-7).
+#include "common.cuh"
+#include <math_constants.h>
+
+namespace {
+
+constexpr int CC = 64;          // tokens of a chunk
+constexpr int PAD = 8;          // bfloat16 behind a row of shared memory: rows of ldmatrix start in different banks
+enum Mode { HEAD, GATED };      // a fixed decay per head; gates per head and token
+
+typedef __nv_bfloat16 bf;
+
+struct ChunkArgs {
+    const bf* rows;              // [rows, stride]: q at q_off, k at k_off (H heads of dk each), v at v_off (H heads of dv)
+    int stride, q_off, k_off, v_off;
+    const float* cos_t;          // [positions, dk / 2] or null: q and k are rotated over the whole head
+    const float* sin_t;
+    const int* tok_pos;
+    const float* gate_pre;       // GATED: [rows, 2H] input gates' pre-activations (H), forget gates' (H), no bias
+    const float* gate_bias;      // GATED: [2H]
+    float gate_cap;
+    const float* decay;          // HEAD: [H]
+    float q_scale, k_scale;
+    float* state;                // [slots][H][dk (+1)][dv (+1)]; GATED's extra row holds the running maximum (in every column)
+    long long slot_stride;
+    const int* cu_rows;          // [B + 1]
+    const int* slots;            // [B]
+    float* out;                  // [rows, H, dv (+1)]
+    float* exp_neg_m;            // GATED: [rows, H]
+    float* s0;                   // scratch [places][H][dk][ld]: the state ahead of every chunk, column c of 32 at 4 (c % 8) + c / 8,
+                                 // the normaliser behind the columns
+    float* gates;                // GATED, scratch [places][H][GATE_FLOATS]: see GateRecord
+    int H, dk, dv, ld, B;
+    int first, places;           // the chunk places that this set of launches works on
+};
+
+// Where the chunks of sequence b lie: unique and never overlapping, whatever the sequences' lengths are.
+__device__ __forceinline__ int first_place(const int* cu_rows, int b) { return cu_rows[b] / CC + b; }
+
+__device__ __forceinline__ void ldsm_x4(const bf* p, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm_x4_t(const bf* p, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// 16 (or 4) bytes to shared memory without a register between; zeros where `in` is false.
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy4(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float low_f32(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float high_f32(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// (x, y) as three pairs of bfloat16 whose sums are x and y to 24 bits.
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        p[i] = *reinterpret_cast<const uint32_t*>(&v);
+        x -= low_f32(p[i]);
+        y -= high_f32(p[i]);
+    }
+}
+
+__device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
+
+// What the gates make of a chunk.  With F_t = f_1 + ... + f_t over the chunk and the running maximum
+// m_t = F_t + max(m_0, max_(s<=t)(i_s - F_s)), rounded to float32 once and used as such everywhere:
+struct GateRecord {
+    double up[CC];               // F_t - m_t
+    double down[CC];             // i_s - F_s (minus infinity behind the last token): D(t, s) = exp(up_t + down_s)
+    float last[CC];              // D(n, s)
+    float first[CC];             // exp(F_t + m_0 - m_t), what is left of S_0 at token t
+    float keep, m_end;           // the same at the chunk's end; the maximum there
+    float unused[2];
+};
+constexpr int GATE_FLOATS = sizeof(GateRecord) / sizeof(float);
+
+// decay^0 .. decay^CC, by multiplication in float64.
+__device__ __forceinline__ void decay_powers(float decay, float* pw, int tid, int threads) {
+    for (int j = tid; j <= CC; j += threads) {
+        double x = 1.0, d = decay;
+        for (int e = j; e; e >>= 1, d *= d)
+            if (e & 1) x *= d;
+        pw[j] = (float)x;
+    }
+}
+
+// ------------------------------------------------------------------ gates
+// Eight chunks at a time, a warp each, two tokens a lane; only the maxima of the chunks are a chain.
+__global__ void __launch_bounds__(256) chunk_gates_kernel(const __grid_constant__ ChunkArgs a) {
+    pdl_launch_dependents();
+    __shared__ double F_sum[8], i_top[8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = blockIdx.x, h = blockIdx.y, H = a.H;
+    pdl_wait();
+    const int row0 = a.cu_rows[b], row1 = a.cu_rows[b + 1], base = first_place(a.cu_rows, b);
+    const int c_lo = max(0, a.first - base), c_hi = min((row1 - row0 + CC - 1) / CC, a.first + a.places - base);
+    if (c_lo >= c_hi) return;
+    float m = a.state[(long long)a.slots[b] * a.slot_stride + ((size_t)h * (a.dk + 1) + a.dk) * (a.dv + 1)];
+    const float cap = a.gate_cap, bias_i = a.gate_bias[h], bias_f = a.gate_bias[H + h];
+    for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
+        const int c = c0 + warp, row = row0 + c * CC, n = c < c_hi ? min(CC, row1 - row) : 0;
+        float i[2] = {-CUDART_INF_F, -CUDART_INF_F};
+        double f[2] = {0.0, 0.0};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = 2 * lane + j;
+            if (t < n) {
+                const float* g = a.gate_pre + (size_t)(row + t) * 2 * H;
+                i[j] = cap * tanhf((g[h] + bias_i) / cap);
+                f[j] = log_sigmoid(cap * tanhf((g[H + h] + bias_f) / cap));
+            }
+        }
+        double run = f[0] + f[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += up;
+        }
+        const double F[2] = {run - f[1], run};
+        const double down[2] = {(double)i[0] - F[0], (double)i[1] - F[1]};
+        double top = fmax(down[0], down[1]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, top, o);
+            if (lane >= o) top = fmax(top, up);
+        }
+        double before = __shfl_up_sync(0xffffffffu, top, 1);
+        if (lane == 0) before = -CUDART_INF;
+        if (lane == 31) { F_sum[warp] = run; i_top[warp] = top; }
+        __syncthreads();
+        float m0 = m;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            if (w == warp) m0 = m;
+            if (c0 + w < c_hi) m = (float)(F_sum[w] + fmax((double)m, i_top[w]));
+        }
+        if (n > 0) {
+            const double F_end = F_sum[warp];
+            const float m_end = (float)(F_end + fmax((double)m0, i_top[warp]));
+            GateRecord& r = reinterpret_cast<GateRecord*>(a.gates)[(size_t)(base + c - a.first) * H + h];
+            const double tops[2] = {fmax(before, down[0]), top};
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int t = 2 * lane + j;
+                const float mt = (float)(F[j] + fmax((double)m0, tops[j]));
+                r.up[t] = F[j] - (double)mt;
+                r.down[t] = down[j];
+                r.last[t] = expf((float)(F_end - (double)m_end + down[j]));
+                r.first[t] = expf((float)(F[j] + (double)m0 - (double)mt));
+                if (t < n) a.exp_neg_m[(size_t)(row + t) * H + h] = expf(-mt);
+            }
+            if (lane == 0) {
+                r.keep = expf((float)(F_end + (double)m0 - (double)m_end));
+                r.m_end = m_end;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------ state
+// 8 NTL value columns a block.  Warps 0 to 3 multiply; the others stage: what a stager reads comes by cp.async into a ring of
+// its own, RING chunks deep, is rotated, scaled and split and goes to one of two buffers while the other is multiplied.
+constexpr int STAGERS = 256, STATE_THREADS = 128 + STAGERS, V_RING = 4;
+
+template <int DK, int NTL, Mode MODE, bool ROT>
+struct StateSizes {
+    static constexpr int LK = DK + PAD, LV = 8 * NTL + PAD;
+    static constexpr int GROUPS = ROT ? DK / 16 : DK / 8;            // eight channels (and their partners of the rotation)
+    static constexpr int ITEMS = CC * GROUPS / STAGERS;              // of a stager's chunk
+    static constexpr int PIECES = ROT ? 6 : 1;                       // of 16 bytes an item: the channels, the partners, two of cosines and of sines
+    static constexpr int RING = ROT && DK == 128 ? 2 : 4;
+    static constexpr size_t planes = (size_t)2 * 3 * CC * LK * sizeof(bf);
+    static constexpr size_t raw = (size_t)RING * ITEMS * PIECES * STAGERS * 16;
+    static constexpr size_t weights = MODE == GATED ? (size_t)RING * ITEMS * STAGERS * 4 : 0;
+    static constexpr size_t values = (size_t)V_RING * CC * LV * sizeof(bf);
+    static constexpr size_t bytes = planes + raw + weights + values;
+};
+
+template <int DK, int NTL, Mode MODE, bool ROT>
+__global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
+    pdl_launch_dependents();
+    using Z = StateSizes<DK, NTL, MODE, ROT>;
+    constexpr int LK = Z::LK, LV = Z::LV, MT = DK / 64, ITEMS = Z::ITEMS, PIECES = Z::PIECES, RING = Z::RING, X = MODE == GATED ? 1 : 0;
+    extern __shared__ __align__(16) uint8_t smem[];
+    bf* planes = reinterpret_cast<bf*>(smem);             // [2][3][CC][LK]: the scaled keys of two chunks
+    uint4* raw = reinterpret_cast<uint4*>(smem + Z::planes);                              // [RING][ITEMS][PIECES][STAGERS]
+    float* raw_w = reinterpret_cast<float*>(smem + Z::planes + Z::raw);                   // [RING][ITEMS][STAGERS]
+    bf* vals = reinterpret_cast<bf*>(smem + Z::planes + Z::raw + Z::weights);             // [V_RING][CC][LV]
+    __shared__ float pw[CC + 1];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * 8 * NTL, H = a.H, dk = a.dk, dv = a.dv;
+    const bool norm_cols = MODE == GATED && blockIdx.z == 0;      // this block also carries the normaliser
+    pdl_wait();
+    const int row0 = a.cu_rows[b], row1 = a.cu_rows[b + 1], base = first_place(a.cu_rows, b);
+    const int c_lo = max(0, a.first - base), c_hi = min((row1 - row0 + CC - 1) / CC, a.first + a.places - base);
+    if (c_lo >= c_hi) return;
+    float* st = a.state + (long long)a.slots[b] * a.slot_stride + (size_t)h * (dk + X) * (dv + X);
+    const GateRecord* gates = reinterpret_cast<const GateRecord*>(a.gates) + (ptrdiff_t)(base - a.first) * H + h;     // chunk c's: gates[c * H]
+    if (dk < DK)
+        for (int j = tid; j < (int)(Z::planes / 16); j += STATE_THREADS) reinterpret_cast<uint4*>(planes)[j] = make_uint4(0, 0, 0, 0);
+    if (MODE == HEAD) decay_powers(a.decay[h], pw, tid, STATE_THREADS);
+    __syncthreads();
+
+    if (warp >= 4) {
+        const int half = dk / 2, width = ROT ? half : dk, ptid = tid - 128, ch = (ptid % Z::GROUPS) * 8, s_first = ptid / Z::GROUPS;
+        constexpr int S_STEP = STAGERS / Z::GROUPS;
+        int pos[ITEMS];                            // positions of the next chunk's tokens to be asked for
+        auto find = [&](int c) {
+            if constexpr (ROT) {
+                if (c >= c_hi) return;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) pos[i] = a.tok_pos[min(row0 + c * CC + s_first + i * S_STEP, row1 - 1)];
+            }
+        };
+        auto load = [&](int c) {
+            if (c < c_hi) {
+                const int row = row0 + c * CC, n = min(CC, row1 - row);
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) {
+                    const int s = s_first + i * S_STEP;
+                    const bool in = s < n && ch < width;
+                    const bf* p = a.rows + (size_t)(row + (in ? s : 0)) * a.stride + a.k_off + h * dk + (in ? ch : 0);
+                    uint4* dst = raw + (size_t)((c % RING) * ITEMS + i) * PIECES * STAGERS + ptid;
+                    copy16(dst, p, in);
+                    if constexpr (ROT) {
+                        copy16(dst + STAGERS, p + (in ? half : 0), in);
+                        const size_t at = in ? (size_t)pos[i] * half + ch : 0;
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            copy16(dst + (2 + e) * STAGERS, a.cos_t + at + 4 * e, in);
+                            copy16(dst + (4 + e) * STAGERS, a.sin_t + at + 4 * e, in);
+                        }
+                    }
+                    if (MODE == GATED) copy4(raw_w + ((c % RING) * ITEMS + i) * STAGERS + ptid, &gates[(size_t)c * H].last[s], true);
+                }
+            }
+            copy_commit();
+            find(c + 1);
+        };
+        // The keys, times what is left of them at their chunk's end, to buffer c & 1 as three terms.
+        auto stage = [&](int c) {
+            if (ch >= width) return;
+            const int n = min(CC, row1 - row0 - c * CC);
+            bf* dst = planes + (size_t)(c & 1) * 3 * CC * LK;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                const int s = s_first + i * S_STEP;
+                const uint4* src = raw + (size_t)((c % RING) * ITEMS + i) * PIECES * STAGERS + ptid;
+                const float f = (MODE == GATED ? raw_w[((c % RING) * ITEMS + i) * STAGERS + ptid] : (s < n ? pw[n - 1 - s] : 0.f)) * a.k_scale;
+                const uint4 lo = src[0];
+                const uint32_t* x = reinterpret_cast<const uint32_t*>(&lo);
+                uint32_t p0[4][3], p1[ROT ? 4 : 1][3];
+                uint4 hi;
+                float4 cs[2], sn[2];
+                if constexpr (ROT) {
+                    hi = src[STAGERS];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        cs[e] = *reinterpret_cast<const float4*>(src + (2 + e) * STAGERS);
+                        sn[e] = *reinterpret_cast<const float4*>(src + (4 + e) * STAGERS);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float u0 = low_f32(x[e]), u1 = high_f32(x[e]);
+                    if constexpr (ROT) {
+                        const uint32_t y = reinterpret_cast<const uint32_t*>(&hi)[e];
+                        const float c0 = reinterpret_cast<const float*>(cs)[2 * e], c1 = reinterpret_cast<const float*>(cs)[2 * e + 1];
+                        const float s0 = reinterpret_cast<const float*>(sn)[2 * e], s1 = reinterpret_cast<const float*>(sn)[2 * e + 1];
+                        const float v0 = low_f32(y), v1 = high_f32(y);
+                        split3((v0 * c0 + u0 * s0) * f, (v1 * c1 + u1 * s1) * f, p1[e]);
+                        u0 = u0 * c0 - v0 * s0;
+                        u1 = u1 * c1 - v1 * s1;
+                    }
+                    split3(u0 * f, u1 * f, p0[e]);
+                }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    bf* d = dst + ((size_t)p * CC + s) * LK + ch;
+                    *reinterpret_cast<uint4*>(d) = make_uint4(p0[0][p], p0[1][p], p0[2][p], p0[3][p]);
+                    if constexpr (ROT) *reinterpret_cast<uint4*>(d + half) = make_uint4(p1[0][p], p1[1][p], p1[2][p], p1[3][p]);
+                }
+            }
+        };
+        find(c_lo);
+#pragma unroll
+        for (int i = 0; i < RING; ++i) load(c_lo + i);
+        copy_wait<RING - 1>();
+        stage(c_lo);
+        __syncthreads();
+        for (int c = c_lo; c < c_hi; ++c) {        // chunk c is being multiplied
+            load(c + RING);                        // to the ring's place that chunk c has left
+            copy_wait<RING - 1>();
+            if (c + 1 < c_hi) stage(c + 1);
+            __syncthreads();
+        }
+        copy_wait<0>();
+        if (MODE == GATED && warp == 4) {
+            const float m = gates[(size_t)(c_hi - 1) * H].m_end;
+            for (int col = col0 + lane; col < min(col0 + 8 * NTL, dv); col += 32) st[(size_t)dk * (dv + X) + col] = m;
+            if (norm_cols && lane == 0) st[(size_t)dk * (dv + X) + dv] = m;
+        }
+        return;
+    }
+
+    // Lane (g, t) holds the columns 8 j + 2 t, + 1 of the rows g and g + 8 of its tiles.
+    float S[MT][NTL][4], N[MT][4];
+    const int r_base = warp * 16 * MT;
+    auto load_values = [&](int c) {
+        if (c < c_hi) {
+            const int row = row0 + c * CC, n = min(CC, row1 - row);
+#pragma unroll
+            for (int i = 0; i < NTL / 2; ++i) {
+                const int j = tid + i * 128, s = j / NTL, col = col0 + (j % NTL) * 8;
+                const bool in = s < n && col < dv;
+                copy16(vals + ((size_t)(c % V_RING) * CC + s) * LV + (j % NTL) * 8,
+                       a.rows + (size_t)(row + (in ? s : 0)) * a.stride + a.v_off + h * dv + (in ? col : 0), in);
+            }
+        }
+        copy_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < V_RING - 1; ++i) load_values(c_lo + i);
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = r_base + i * 16 + g + (e >> 1) * 8;
+#pragma unroll
+            for (int j = 0; j < NTL; ++j) {
+                const int col = col0 + 8 * j + 2 * t + (e & 1);
+                S[i][j][e] = r < dk && col < dv ? st[(size_t)r * (dv + X) + col] : 0.f;
+            }
+            N[i][e] = norm_cols && r < dk && t == 0 && !(e & 1) ? st[(size_t)r * (dv + X) + dv] : 0.f;
+        }
+    }
+    float keep = MODE == GATED ? gates[(size_t)c_lo * H].keep : 0.f;
+    copy_wait<V_RING - 2>();
+    __syncthreads();
+    for (int c = c_lo; c < c_hi; ++c) {
+        load_values(c + V_RING - 1);
+        const float keep_next = MODE == GATED && c + 1 < c_hi ? gates[(size_t)(c + 1) * H].keep : 0.f;
+        if (MODE == HEAD) keep = pw[min(CC, row1 - row0 - c * CC)];
+        // The state ahead of the chunk.
+        float* dst = a.s0 + ((size_t)(base + c - a.first) * H + h) * dk * a.ld + col0 / 32 * 32 + col0 % 32 / 8 + 8 * t;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = r_base + i * 16 + g + e * 8;
+                if (r < dk) {
+                    float* d = dst + (size_t)r * a.ld;
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        if constexpr (NTL == 4)
+                            *reinterpret_cast<float4*>(d + 4 * x) = make_float4(S[i][0][2 * e + x], S[i][1][2 * e + x], S[i][2][2 * e + x], S[i][3][2 * e + x]);
+                        else
+                            *reinterpret_cast<float2*>(d + 4 * x) = make_float2(S[i][0][2 * e + x], S[i][1][2 * e + x]);
+                    }
+                    if (norm_cols && t == 0) d[a.ld - 4] = N[i][2 * e];
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+#pragma unroll
+            for (int j = 0; j < NTL; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[i][j][e] *= keep;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) N[i][e] *= keep;
+        }
+        const bf* src = planes + (size_t)(c & 1) * 3 * CC * LK;
+        const bf* val = vals + (size_t)(c % V_RING) * CC * LV;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t vb[NTL / 2][4];
+#pragma unroll
+            for (int j = 0; j < NTL / 2; ++j)
+                ldsm_x4_t(val + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + j * 16 + (lane >> 4) * 8, vb[j]);
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                uint32_t af[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    ldsm_x4_t(src + ((size_t)p * CC + kk * 16 + (lane & 7) + (lane >> 4) * 8) * LK + r_base + i * 16 + ((lane >> 3) & 1) * 8, af[p]);
+                float d[NTL][4] = {};
+#pragma unroll
+                for (int p = 2; p >= 0; --p)     // the columns' products between those that wait for one another
+#pragma unroll
+                    for (int j = 0; j < NTL; ++j) mma_bf16(d[j], af[p], vb[j / 2][2 * (j & 1)], vb[j / 2][2 * (j & 1) + 1]);
+#pragma unroll
+                for (int j = 0; j < NTL; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) S[i][j][e] += d[j][e];
+                if (norm_cols) {                 // the normaliser: a value column of ones
+                    const uint32_t one = g == 0 ? 0x3f803f80u : 0u;
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int p = 2; p >= 0; --p) mma_bf16(d, af[p], one, one);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) N[i][e] += d[e];
+                }
+            }
+        }
+        if (MODE == GATED) keep = keep_next;
+        copy_wait<V_RING - 2>();
+        __syncthreads();
+    }
+    copy_wait<0>();
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = r_base + i * 16 + g + (e >> 1) * 8;
+            if (r >= dk) continue;
+#pragma unroll
+            for (int j = 0; j < NTL; ++j) {
+                const int col = col0 + 8 * j + 2 * t + (e & 1);
+                if (col < dv) st[(size_t)r * (dv + X) + col] = S[i][j][e];
+            }
+            if (norm_cols && t == 0 && !(e & 1)) st[(size_t)r * (dv + X) + dv] = N[i][e];
+        }
+}
+
+// ------------------------------------------------------------------ output
+// Four warps: first 16 rows of the chunk's triangle each, then 32 value columns and 16 MTB rows of the output each.  The state
+// goes from global memory straight into the products' fragments; shared memory holds q, v, and k and then the triangle in one
+// place, so that three blocks share a multiprocessor (two where q and k are rotated heads of 128, whose k comes in two halves).
+template <int DK, int DV, Mode MODE, bool ROT>
+struct OutSizes {
+    static constexpr int NQ = ROT ? 3 : 1;               // rotated q and k are float32: three terms
+    static constexpr int LK = DK + PAD, LP = CC + PAD, LV = DV + PAD;
+    static constexpr int HALVES = ROT && DK == 128 ? 2 : 1;
+    static constexpr size_t q = (size_t)NQ * CC * LK * sizeof(bf), k = q / HALVES, p = (size_t)3 * CC * LP * sizeof(bf);
+    static constexpr size_t v = (size_t)CC * LV * sizeof(bf), rows_out = MODE == GATED ? (size_t)CC * (DV + 4) * sizeof(float) : 0;
+    static constexpr size_t work = q + v + (HALVES == 1 ? (k > p ? k : p) : k + p), bytes = work > rows_out ? work : rows_out;
+};
+
+template <int DK, int DV, Mode MODE, bool ROT>
+__global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant__ ChunkArgs a) {
+    pdl_launch_dependents();
+    using Z = OutSizes<DK, DV, MODE, ROT>;
+    extern __shared__ __align__(16) uint8_t smem[];
+    constexpr int NQ = Z::NQ, LK = Z::LK, LP = Z::LP, LV = Z::LV, HALVES = Z::HALVES, HC = CC / HALVES;
+    constexpr int WN = DV / 32, WM = 4 / WN, MTB = 4 / WM, X = MODE == GATED ? 1 : 0;
+    bf* qp = reinterpret_cast<bf*>(smem);          // [NQ][CC][LK]
+    bf* vp = qp + Z::q / sizeof(bf);               // [CC][LV]
+    bf* kp = vp + Z::v / sizeof(bf);               // [NQ][HC][LK]
+    bf* pp = HALVES == 1 ? kp : kp + Z::k / sizeof(bf);    // [3][CC][LP]
+    __shared__ float pw[CC + 1], f_row[CC], n_row[CC], n_part[2][CC], n0[DK];
+    __shared__ double up[CC], down[CC];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int h = blockIdx.y, H = a.H, dk = a.dk, dv = a.dv, place = a.first + blockIdx.x;
+    pdl_wait();
+    int lo = 0, hi = a.B - 1;                      // the last sequence whose chunks start at or ahead of this place
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (first_place(a.cu_rows, mid) <= place) lo = mid;
+        else hi = mid - 1;
+    }
+    const int row = a.cu_rows[lo] + (place - first_place(a.cu_rows, lo)) * CC, n = min(CC, a.cu_rows[lo + 1] - row);
+    if (n <= 0) return;
+    const float* s0 = a.s0 + ((size_t)blockIdx.x * H + h) * dk * a.ld;
+
+    // ---- q (which 0) or k (1) of the tokens s_lo .. s_lo + count - 1, split where they are rotated
+    auto stage = [&](int which, int s_lo, int count) {
+        constexpr int GROUPS = ROT ? DK / 16 : DK / 8;
+        const int half = dk / 2, width = ROT ? half : dk, rows = which ? HC : CC;
+        bf* dst = which ? kp : qp;
+#pragma unroll 4
+        for (int j = tid; j < count * GROUPS; j += 128) {
+            const int sl = j / GROUPS, s = s_lo + sl, ch = (j % GROUPS) * 8;
+            const bool in = s < n && ch < width;
+            const bf* src = a.rows + (size_t)(row + (in ? s : 0)) * a.stride + (which ? a.k_off : a.q_off) + h * dk + (in ? ch : 0);
+            if constexpr (!ROT) {
+                copy16(dst + sl * LK + ch, src, in);
+            } else if (ch < width) {
+                const size_t at = in ? (size_t)a.tok_pos[row + s] * half + ch : 0;
+                float cs[8], sn[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 4) {
+                    *reinterpret_cast<float4*>(cs + e) = *reinterpret_cast<const float4*>(a.cos_t + at + e);
+                    *reinterpret_cast<float4*>(sn + e) = *reinterpret_cast<const float4*>(a.sin_t + at + e);
+                }
+                const uint4 x4 = in ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
+                const uint4 y4 = in ? *reinterpret_cast<const uint4*>(src + half) : make_uint4(0, 0, 0, 0);
+                const uint32_t* x = reinterpret_cast<const uint32_t*>(&x4);
+                const uint32_t* y = reinterpret_cast<const uint32_t*>(&y4);
+                uint32_t p0[4][3], p1[4][3];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float u0 = low_f32(x[e]), u1 = high_f32(x[e]), v0 = low_f32(y[e]), v1 = high_f32(y[e]);
+                    split3(u0 * cs[2 * e] - v0 * sn[2 * e], u1 * cs[2 * e + 1] - v1 * sn[2 * e + 1], p0[e]);
+                    split3(v0 * cs[2 * e] + u0 * sn[2 * e], v1 * cs[2 * e + 1] + u1 * sn[2 * e + 1], p1[e]);
+                }
+#pragma unroll
+                for (int i = 0; i < NQ; ++i) {
+                    bf* d = dst + ((size_t)i * rows + sl) * LK + ch;
+                    *reinterpret_cast<uint4*>(d) = make_uint4(p0[0][i], p0[1][i], p0[2][i], p0[3][i]);
+                    *reinterpret_cast<uint4*>(d + half) = make_uint4(p1[0][i], p1[1][i], p1[2][i], p1[3][i]);
+                }
+            }
+        }
+    };
+    if (ROT && dk < DK) {                          // the staging leaves the channels behind dk alone
+        for (int j = tid; j < (int)(Z::work / 16); j += 128) reinterpret_cast<uint4*>(smem)[j] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+    }
+    stage(0, 0, CC);
+    stage(1, 0, HC);
+    copy_commit();
+#pragma unroll
+    for (int j = tid; j < CC * (DV / 8); j += 128) {
+        const int s = j / (DV / 8), col = (j % (DV / 8)) * 8;
+        const bool in = s < n && col < dv;
+        copy16(vp + s * LV + col, a.rows + (size_t)(row + (in ? s : 0)) * a.stride + a.v_off + h * dv + (in ? col : 0), in);
+    }
+    copy_commit();
+    if (MODE == HEAD) {
+        decay_powers(a.decay[h], pw, tid, 128);
+    } else if (tid < CC) {
+        const GateRecord& r = reinterpret_cast<const GateRecord*>(a.gates)[(size_t)blockIdx.x * H + h];
+        up[tid] = r.up[tid];
+        down[tid] = r.down[tid];
+        f_row[tid] = r.first[tid] * a.q_scale;
+    }
+    if (MODE == GATED && tid < dk) n0[tid] = s0[(size_t)tid * a.ld + a.ld - 4];
+    copy_wait<1>();
+    __syncthreads();
+    if (MODE == HEAD && tid < CC) f_row[tid] = pw[tid + 1] * a.q_scale;
+    if (MODE == GATED) {                           // q_t . n_0 on the CUDA cores: half of a row's channels a thread
+        const int s = tid & (CC - 1), part = tid / CC, r_hi = min(dk, (part + 1) * (DK / 2));
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int r = part * (DK / 2); r < r_hi; r += 8) {
+            float x[8] = {};
+#pragma unroll
+            for (int i = NQ - 1; i >= 0; --i) {
+                const uint4 q4 = *reinterpret_cast<const uint4*>(qp + ((size_t)i * CC + s) * LK + r);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    x[2 * e] += low_f32(reinterpret_cast<const uint32_t*>(&q4)[e]);
+                    x[2 * e + 1] += high_f32(reinterpret_cast<const uint32_t*>(&q4)[e]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[e & 3] = fmaf(x[e], n0[r + e], sum[e & 3]);
+        }
+        n_part[part][s] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    }
+
+    // ---- the triangle D(t, s) (q_t . k_s): this warp's 16 rows, the 16-column steps up to the diagonal
+    {
+        float s_acc[8][4] = {};
+#pragma unroll
+        for (int half = 0; half < HALVES; ++half) {
+            constexpr int STEPS = HC / 16;
+            if (half) {
+                __syncthreads();
+                stage(1, half * HC, HC);
+                __syncthreads();
+            }
+            if (half * STEPS > warp) continue;
+#pragma unroll 2
+            for (int kk = 0; kk < DK / 16; ++kk) {
+                uint32_t qf[NQ][4];
+#pragma unroll
+                for (int i = 0; i < NQ; ++i)
+                    ldsm_x4(qp + ((size_t)i * CC + warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LK + kk * 16 + (lane >> 4) * 8, qf[i]);
+#pragma unroll
+                for (int js = 0; js < STEPS; ++js) {
+                    const int jp = half * STEPS + js;
+                    if (jp > warp) break;
+                    uint32_t kf[NQ][4];
+#pragma unroll
+                    for (int i = 0; i < NQ; ++i)
+                        ldsm_x4(kp + ((size_t)i * HC + js * 16 + (lane & 7) + (lane >> 4) * 8) * LK + kk * 16 + ((lane >> 3) & 1) * 8, kf[i]);
+                    float d[NQ][2][4] = {};        // by order of magnitude: no product waits for more than two others
+#pragma unroll
+                    for (int i = 0; i < NQ; ++i)
+#pragma unroll
+                        for (int sum = NQ - 1; sum >= i; --sum)
+#pragma unroll
+                            for (int x = 0; x < 2; ++x) mma_bf16(d[sum][x], qf[i], kf[sum - i][2 * x], kf[sum - i][2 * x + 1]);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            float v = d[NQ - 1][x][e];
+#pragma unroll
+                            for (int sum = NQ - 2; sum >= 0; --sum) v += d[sum][x][e];
+                            s_acc[2 * jp + x][e] += v;
+                        }
+                }
+            }
+        }
+        if (HALVES == 1) __syncthreads();          // k has been read: the triangle takes its place
+        const float scale = a.q_scale * a.k_scale;
+        float sums[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j > 2 * warp + 1) break;
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int tt = warp * 16 + g + (e >> 1) * 8, s = j * 8 + 2 * t + (e & 1);
+                v[e] = 0.f;
+                if (s <= tt && s < n) v[e] = s_acc[j][e] * ((MODE == HEAD ? pw[tt - s] : expf((float)(up[tt] + down[s]))) * scale);
+                sums[e >> 1] += v[e];
+            }
+            uint32_t p0[3], p1[3];
+            split3(v[0], v[1], p0);
+            split3(v[2], v[3], p1);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                *reinterpret_cast<uint32_t*>(pp + ((size_t)i * CC + warp * 16 + g) * LP + j * 8 + 2 * t) = p0[i];
+                *reinterpret_cast<uint32_t*>(pp + ((size_t)i * CC + warp * 16 + g + 8) * LP + j * 8 + 2 * t) = p1[i];
+            }
+        }
+        if (MODE == GATED) {                       // the normaliser's share of the chunk: the triangle's rows added up
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                sums[e] += __shfl_xor_sync(0xffffffffu, sums[e], 1);
+                sums[e] += __shfl_xor_sync(0xffffffffu, sums[e], 2);
+                if (t == 0) n_row[warp * 16 + g + e * 8] = sums[e];
+            }
+        }
+    }
+
+    // ---- S_0^T q, then the rows' decays, then the triangle times v
+    const int wn = warp % WN, wm = warp / WN, col = wn * 32 + 4 * g;
+    float acc[MTB][4][4] = {};
+    float4 sx[2][4];
+    auto fetch_s = [&](int kk, float4 (&x)[4]) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = kk * 16 + 2 * t + (e & 1) + (e >> 1) * 8;
+            x[e] = r < dk && wn * 32 < dv ? *reinterpret_cast<const float4*>(s0 + (size_t)r * a.ld + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    fetch_s(0, sx[0]);
+    fetch_s(1, sx[1]);
+    copy_wait<0>();
+    __syncthreads();
+#pragma unroll 2
+    for (int kk = 0; kk < DK / 16; ++kk) {
+        uint32_t sb[3][4][2];
+        float4 (&x)[4] = sx[kk & 1];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t p[3];
+                split3(reinterpret_cast<const float*>(&x[2 * e])[j], reinterpret_cast<const float*>(&x[2 * e + 1])[j], p);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) sb[i][j][e] = p[i];
+            }
+        if (kk + 2 < DK / 16) fetch_s(kk + 2, x);
+#pragma unroll
+        for (int i = 0; i < MTB; ++i) {
+            uint32_t qf[NQ][4];
+#pragma unroll
+            for (int p = 0; p < NQ; ++p)
+                ldsm_x4(qp + ((size_t)p * CC + (i * WM + wm) * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LK + kk * 16 + (lane >> 4) * 8, qf[p]);
+            float d[4][4] = {};
+#pragma unroll
+            for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+                for (int p = 0; p <= sum && p < NQ; ++p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) mma_bf16(d[j], qf[p], sb[sum - p][j][0], sb[sum - p][j][1]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < MTB; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float f = f_row[(i * WM + wm) * 16 + g + (e >> 1) * 8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j][e] *= f;
+        }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        uint32_t vb[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            ldsm_x4_t(vp + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + wn * 32 + j * 16 + (lane >> 4) * 8, vb[j]);
+#pragma unroll
+        for (int i = 0; i < MTB; ++i) {
+            const int mi = i * WM + wm;
+            if (kk > mi) continue;                 // above the diagonal
+            uint32_t pf[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                ldsm_x4(pp + ((size_t)p * CC + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LP + kk * 16 + (lane >> 4) * 8, pf[p]);
+            float d[4][4] = {};
+#pragma unroll
+            for (int p = 2; p >= 0; --p)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mma_bf16(d[j], pf[p], vb[j / 2][2 * (j & 1)], vb[j / 2][2 * (j & 1) + 1]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
+        }
+    }
+    // ---- out
+    if (MODE == HEAD) {
+#pragma unroll
+        for (int i = 0; i < MTB; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int tt = (i * WM + wm) * 16 + g + e * 8;
+                if (tt >= n) continue;
+                float* o = a.out + ((size_t)(row + tt) * H + h) * dv;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c = wn * 32 + 8 * j + 2 * t;
+                    if (c < dv) *reinterpret_cast<float2*>(o + c) = make_float2(acc[i][j][2 * e], acc[i][j][2 * e + 1]);
+                }
+            }
+    } else {
+        // Rows of dv + 1 numbers start anywhere: through shared memory, so that a warp stores them in order.
+        constexpr int LO = DV + 4;
+        float* tile = reinterpret_cast<float*>(smem);      // [CC][LO]: over what the products have read
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < MTB; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float* o = tile + ((i * WM + wm) * 16 + g + e * 8) * LO + wn * 32 + 2 * t;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(o + 8 * j) = make_float2(acc[i][j][2 * e], acc[i][j][2 * e + 1]);
+            }
+        if (tid < CC) tile[tid * LO + DV] = fmaf(n_part[0][tid] + n_part[1][tid], f_row[tid], n_row[tid]);
+        __syncthreads();
+        for (int tt = warp; tt < n; tt += 4) {
+            float* o = a.out + ((size_t)(row + tt) * H + h) * (dv + X);
+            for (int c = lane; c <= dv; c += 32) o[c] = tile[tt * LO + (c < dv ? c : DV)];
+        }
+    }
+}
+
+template <typename Kernel>
+int set_smem(Kernel kernel, size_t bytes) {
+    if (bytes <= 48 * 1024) return LQ_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return e == cudaSuccess ? LQ_OK : (int)e;
+}
+
+template <int DK, Mode MODE, bool ROT>
+int launch_state(const ChunkArgs& a, cudaStream_t stream) {
+    auto go = [&](auto kernel, int cols, size_t smem) {
+        if (int e = set_smem(kernel, smem)) return e;
+        return launch_pdl(kernel, dim3(a.B, a.H, (a.dv + cols - 1) / cols), dim3(STATE_THREADS), smem, stream, a);
+    };
+    // 32 columns a block read the keys' terms least often; 16 where that leaves more than half of the multiprocessors idle.
+    if ((long long)a.B * a.H * ((a.dv + 31) / 32) > 74) return go(chunk_state_kernel<DK, 4, MODE, ROT>, 32, StateSizes<DK, 4, MODE, ROT>::bytes);
+    return go(chunk_state_kernel<DK, 2, MODE, ROT>, 16, StateSizes<DK, 2, MODE, ROT>::bytes);
+}
+
+template <int DK, int DV, Mode MODE, bool ROT>
+int launch_out(const ChunkArgs& a, cudaStream_t stream) {
+    constexpr size_t smem = OutSizes<DK, DV, MODE, ROT>::bytes;
+    auto kernel = chunk_out_kernel<DK, DV, MODE, ROT>;
+    if (int e = set_smem(kernel, smem)) return e;
+    return launch_pdl(kernel, dim3(a.places, a.H), dim3(128), smem, stream, a);
+}
+
+template <int DK, Mode MODE, bool ROT>
+int launch_both(const ChunkArgs& a, cudaStream_t stream) {
+    if (int e = launch_state<DK, MODE, ROT>(a, stream)) return e;
+    return a.dv <= 64 ? launch_out<DK, 64, MODE, ROT>(a, stream) : launch_out<DK, 128, MODE, ROT>(a, stream);
+}
+
+template <int DK>
+int launch_mode(const ChunkArgs& a, bool gated, cudaStream_t stream) {
+    if (gated) {
+        if (int e = launch_pdl(chunk_gates_kernel, dim3(a.B, a.H), dim3(256), 0, stream, a)) return e;
+        return launch_both<DK, GATED, false>(a, stream);
+    }
+    return a.cos_t ? launch_both<DK, HEAD, true>(a, stream) : launch_both<DK, HEAD, false>(a, stream);
+}
+
+}  // namespace
+
+// Chunk places of a step with these rows and sequences, and floats of scratch for one of them.
+LQ_EXPORT long long lq_chunk_place_floats(int H, int dk, int dv, int gated) {
+    return (long long)H * dk * ((dv + 31) / 32 * 32 + (gated ? 4 : 0)) + (gated ? (long long)H * GATE_FLOATS : 0);
+}
+
+// As lq_linear_scan for steps with prompts in bfloat16: dk and dv multiples of 8 up to 128, offsets and stride in whole eights;
+// with a fixed decay, rotation over whole heads (dk a multiple of 16) or none.  `places` chunks of scratch are worked on at a time.
+LQ_EXPORT int lq_chunk_scan(const void* qkv, int stride, int q_off, int k_off, int v_off, const float* cos_t, const float* sin_t,
+                            const int* tok_pos, const float* gate_pre, const float* gate_bias, float gate_cap, const float* decay,
+                            float q_scale, float k_scale, float* state, long long slot_stride, const int* cu_rows, const int* slots,
+                            float* out, float* exp_neg_m, float* scratch, int places, int rows, int B, int H, int dk, int dv,
+                            cudaStream_t stream) {
+    if (B <= 0 || rows <= 0) return LQ_OK;
+    const bool gated = gate_pre != nullptr;
+    if (dk < 8 || dv < 8 || dk > 128 || dv > 128 || dk % 8 || dv % 8 || places < 1) return LQ_BAD_SIZE;
+    if (cos_t && (gated || dk % 16 || !sin_t || !tok_pos)) return LQ_BAD_SIZE;
+    if (stride % 8 || q_off % 8 || k_off % 8 || v_off % 8 || (uintptr_t)qkv % 16 || (uintptr_t)cos_t % 16 || (uintptr_t)sin_t % 16 ||
+        (uintptr_t)scratch % 16) return LQ_BAD_SIZE;
+    if (gated ? (!gate_bias || !exp_neg_m) : !decay) return LQ_BAD_SIZE;
+    ChunkArgs a{(const bf*)qkv, stride, q_off, k_off, v_off, cos_t, sin_t, tok_pos, gate_pre, gate_bias, gate_cap, decay, q_scale, k_scale,
+                state, slot_stride, cu_rows, slots, out, exp_neg_m, scratch, nullptr, H, dk, dv, (dv + 31) / 32 * 32 + (gated ? 4 : 0), B, 0, 0};
+    a.gates = scratch + (size_t)places * H * dk * a.ld;      // 16-byte aligned: dk and ld are whole eights and fours
+    const int all = rows / CC + B;
+    for (a.first = 0; a.first < all; a.first += places) {
+        a.places = all - a.first < places ? all - a.first : places;
+        if (int e = dk <= 64 ? launch_mode<64>(a, gated, stream) : launch_mode<128>(a, gated, stream)) return e;
+    }
+    return LQ_OK;
+}

@@ -1,0 +1,132 @@
+"""The recurrences by chunks (csrc/chunk_scan.cu) against the recurrence in float64: chunk edges, short sequences beside long ones,
+every head size class, scratch that holds only a part of the step, and which calls take this route."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+# As for the kernels that walk token by token (float32 state and sums): 2e-5 of the largest value.
+TOL = 2e-5
+
+
+def _ops():
+    from longbow_quarrel_b200.kernels import ops
+    return ops
+
+
+def _i32(x):
+    return torch.tensor(np.asarray(x), dtype=torch.int32, device=DEV)
+
+
+def _scan64(q, k, v, a, b, S):
+    """All [T, H, ...] float64; a [T, H, 1 or dk], b [T, H, 1]; returns outputs and the last state."""
+    out = []
+    for t in range(q.shape[0]):
+        S = a[t][..., None] * S + (b[t] * k[t])[..., None] * v[t][:, None]
+        out.append((S * q[t][..., None]).sum(1))
+    return torch.stack(out), S
+
+
+def _case(kind, lens, H, dk, dv, pad=0, seed=0):
+    """A step's rows, the call's options and the float64 result."""
+    gen = torch.Generator().manual_seed(seed + dk * dv)
+    T, X = sum(lens), int(kind == "mlstm")
+    x = torch.randn(T, 2 * H * dk + H * dv + pad, generator=gen).to(torch.bfloat16)
+    slots = [2 * i + 1 for i in range(len(lens))][::-1]
+    state = torch.randn(2 * len(lens) + 1, H, dk + X, dv + X, generator=gen)
+    pos = np.concatenate([np.arange(n) + 3 * i for i, n in enumerate(lens)])
+    opts, a, b, last_m = {}, None, torch.ones(T, H, 1, dtype=torch.float64), None
+    z = x.double()
+    q, k, v = z[:, :H * dk].view(T, H, dk), z[:, H * dk:2 * H * dk].view(T, H, dk), z[:, 2 * H * dk:2 * H * dk + H * dv].view(T, H, dv)
+    if kind == "rotated":
+        f = 1000.0 ** (-2.0 * torch.arange(dk // 2, dtype=torch.float64) / dk)
+        ang = torch.arange(int(pos.max()) + 1, dtype=torch.float64)[:, None] * f[None]
+        cos, sin = torch.cos(ang).float(), torch.sin(ang).float()
+        opts["rot"] = (cos.to(DEV), sin.to(DEV), dk)
+        c, s = cos.double()[pos][:, None], sin.double()[pos][:, None]
+        turn = lambda y: torch.cat([y[..., :dk // 2] * c - y[..., dk // 2:] * s, y[..., dk // 2:] * c + y[..., :dk // 2] * s], -1)
+        q, k = turn(q), turn(k)
+    opts["q_scale"], opts["k_scale"] = dk ** -0.5, 0.5
+    q, k = q * opts["q_scale"], k * opts["k_scale"]
+    if kind == "mlstm":
+        state[:, :, dk] = state[:, :, dk, :1]
+        cap = 8.0
+        pre, bias = torch.randn(T, 2 * H, generator=gen) * 2 * cap, torch.randn(2 * H, generator=gen)
+        pre[T // 2:T // 2 + 5, H:] = -4 * cap                 # forget nearly everything
+        opts["gates"] = (pre.to(DEV), bias.to(DEV), cap)
+        g = pre.double() + bias.double()
+        li, lf = cap * torch.tanh(g[:, :H] / cap), torch.nn.functional.logsigmoid(cap * torch.tanh(g[:, H:] / cap))
+        v = torch.cat([v, torch.ones_like(v[..., :1])], dim=2)
+    else:
+        decay = torch.linspace(0.5, 1.0, H)
+        opts["decay"] = decay.to(DEV)
+        a = decay.double()[None, :, None].expand(T, H, 1)
+    outs, finals, row = [], [], 0
+    for n, slot in zip(lens, slots):
+        S, rows = state[slot].double(), slice(row, row + n)
+        if kind == "mlstm":
+            m, aa, bb = S[:, dk, 0], [], []
+            for t in range(row, row + n):
+                m, old = torch.maximum(lf[t] + m, li[t]), m
+                aa.append(torch.exp(lf[t] + old - m)[:, None])
+                bb.append(torch.exp(li[t] - m)[:, None])
+            o, S = _scan64(q[rows], k[rows], v[rows], torch.stack(aa), torch.stack(bb), S[:, :dk])
+            S = torch.cat([S, m[:, None, None].expand(-1, 1, dv + 1)], dim=1)
+        else:
+            o, S = _scan64(q[rows], k[rows], v[rows], a[rows], b[rows], S)
+        outs.append(o)
+        finals.append(S)
+        row += n
+    return x, state, slots, pos, opts, torch.cat(outs), finals
+
+
+def _run(ops, x, state, slots, lens, pos, opts, H, dk, dv):
+    before = ops.launches_by_name().get("linear_scan:chunks", 0)
+    st = state.to(DEV).contiguous()
+    out, enm = ops.linear_scan(x.to(DEV), 0, H * dk, 2 * H * dk, st, _i32(np.concatenate([[0], np.cumsum(lens)])), _i32(slots), _i32(pos),
+                               len(lens), H, dk, dv, **opts)
+    return out.cpu().double(), st.cpu(), ops.launches_by_name().get("linear_scan:chunks", 0) - before
+
+
+def _check(got, st, want, finals, state, slots):
+    assert float((got - want).abs().max()) < TOL * float(want.abs().max())
+    for slot, S in zip(slots, finals):
+        assert float((st[slot].double() - S).abs().max()) < TOL * float(S.abs().max())
+    others = [i for i in range(state.shape[0]) if i not in slots]
+    assert torch.equal(st[others], state[others])
+
+
+SIZES = [([64], 2, 64, 64), ([65, 1, 200], 3, 128, 128), ([191], 1, 16, 8), ([127, 130], 2, 64, 128), ([300, 2, 64], 2, 128, 40), ([129], 2, 80, 96)]
+
+
+@pytest.mark.parametrize("lens,H,dk,dv", SIZES)
+@pytest.mark.parametrize("kind", ["plain", "rotated", "mlstm"])
+def test_chunks_follow_the_recurrence(kind, lens, H, dk, dv):
+    ops = _ops()
+    x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv, pad=8)
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    assert chunks == 1
+    _check(got, st, want, finals, state, slots)
+
+
+@pytest.mark.parametrize("kind", ["plain", "mlstm"])
+def test_scratch_for_a_part_of_the_chunks(kind, monkeypatch):
+    """The chunks in turns of two places: the state goes on from turn to turn through its slot."""
+    ops = _ops()
+    lens, H, dk, dv = [200, 70, 130], 2, 64, 32
+    x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_FLOATS", 2 * ops.build.load("chunk_scan").lq_chunk_place_floats(H, dk, dv, int(kind == "mlstm")))
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    assert chunks == 1
+    _check(got, st, want, finals, state, slots)
+
+
+@pytest.mark.parametrize("why,lens,H,dk,dv,pad", [("few rows", [63], 2, 64, 64, 0), ("odd head", [100], 2, 24, 20, 0), ("odd stride", [100], 2, 16, 16, 3),
+                                                  ("a head of 136", [100], 1, 136, 16, 0)])
+def test_other_sizes_keep_the_walk_by_tokens(why, lens, H, dk, dv, pad):
+    ops = _ops()
+    x, state, slots, pos, opts, want, finals = _case("plain", lens, H, dk, dv, pad=pad)
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    assert chunks == 0
+    _check(got, st, want, finals, state, slots)
