@@ -2,26 +2,29 @@
 //
 //   S_t = a_t S_(t-1) + b_t k_t v_t^T          o_t = S_t^T q_t
 //
-// with the head's fixed decay (retention) or the gates of an mlstm.  With S_0 the state ahead of a chunk and
+// with the head's fixed decay (retention), the gates of an mlstm, or a decay a_t per key channel.  With S_0 the state ahead of a chunk and
 // D(t, s) = a_(s+1) ... a_t b_s,
 //   o_t = D(t, 0) S_0^T q_t + sum_(s<=t) D(t, s) (q_t . k_s) v_s          S_n = D(n, 0) S_0 + sum_s D(n, s) k_s v_s^T
 // Token by token the recurrence is a chain over all tokens whose steps leave most of the chip idle; by chunks only the state
 // is a chain, one short step per 64 tokens:
 //   gates   (mlstm) a block per (sequence, head): every token's logarithms and running maximum
+//   prepare (channel decays) a block per (chunk, head): q and k with their decays, and the triangle of the sum over s
 //   state   a block per (sequence, head, some value columns) walks the chunks in order: four warps hold their share of S in
 //           registers and multiply, eight others stage the next chunk's scaled keys; S_0 of every chunk goes to scratch
 //   output  a block per (chunk, head), all at once
 // The state kernel is bound by what a block does per chunk (its products where heads are of 128, its stagers' copies of cosines
 // and sines where they are rotated), the output kernel by the latencies of eight to twelve warps a multiprocessor (tensor cores
 // busy a quarter of the time).  2,048 tokens of 32 heads, both kernels (and gates), us: heads of 64 rotated 491 token by token
-// (recurrent.cu), 75 here; with gates 731 and 87; heads of 128 rotated 1,165 and 236; with gates 1,264 and 160.
+// (recurrent.cu), 75 here; with gates 731 and 87; with decays per key channel 397 and 157; heads of
+// 128: 1,165 and 236, 1,264 and 160, 1,915 and 333 (of which prepare 147: exponentials and logarithms, then the halves' sums).
 //
 // Precision: what the recurrence holds in 32 bits stays so.  A float32 operand enters the products as three bfloat16 terms
 // (its 24 bits), a pair of such operands as the six products that reach 2^-24; bfloat16 operands enter as they are.  The
 // tensor cores cut their sums off where float32 rounds, so no sum of theirs is longer than one step of 16 terms: each
 // starts from zero, least terms first, and joins the float32 accumulator by an ordinary addition.  The decays' logarithms add up
 // in float64, so that their differences keep their digits.  Distance from the recurrence in float64, 2,048 tokens, outputs / state:
-// 1.3e-7 / 1.0e-7 with a fixed decay (token by token 2.2e-7 / 2.2e-7), 2.0e-7 / 1.7e-7 with gates (3.9e-7 / 3.0e-7).
+// 1.3e-7 / 1.0e-7 with a fixed decay (token by token 2.2e-7 / 2.2e-7), 2.0e-7 / 1.7e-7 with gates (3.9e-7 / 3.0e-7), 2.0e-6 / 2.3e-6 with decays per
+// channel (the same: what the float32 decays themselves leave).
 #include "common.cuh"
 #include <math_constants.h>
 
@@ -29,7 +32,7 @@ namespace {
 
 constexpr int CC = 64;          // tokens of a chunk
 constexpr int PAD = 8;          // bfloat16 behind a row of shared memory: rows of ldmatrix start in different banks
-enum Mode { HEAD, GATED };      // a fixed decay per head; gates per head and token
+enum Mode { HEAD, GATED, VEC };  // a fixed decay per head; gates per head and token; a decay per key channel and token
 
 typedef __nv_bfloat16 bf;
 
@@ -53,6 +56,11 @@ struct ChunkArgs {
     float* s0;                   // scratch [places][H][dk][ld]: the state ahead of every chunk, column c of 32 at 4 (c % 8) + c / 8,
                                  // the normaliser behind the columns
     float* gates;                // GATED, scratch [places][H][GATE_FLOATS]: see GateRecord
+    const float* decay_pre;      // VEC: [rows, decay_stride], head h's dk pre-activations at column h * dk
+    int decay_stride;
+    const float* decay_bias;     // VEC: [H * dk] or null
+    float inv_tau;               // VEC: a = exp(logsigmoid(pre + bias) * inv_tau)
+    float* prep;                 // VEC, scratch [places][H][vec_floats(dk)]: see prepare
     int H, dk, dv, ld, B;
     int first, places;           // the chunk places that this set of launches works on
 };
@@ -192,6 +200,222 @@ __global__ void __launch_bounds__(256) chunk_gates_kernel(const __grid_constant_
     }
 }
 
+// ------------------------------------------------------------------ prepare
+// With a decay per key channel, D(t, s) is a vector and stands inside the sum over the channels, so a block per (chunk, head)
+// makes, all chunks at once, what the two kernels behind it multiply (float32, products of the decays themselves, so that no
+// difference of logarithms loses digits and a decay of zero is harmless):
+//   k_s D(n, s), q_t D(t, 0), D(n, 0), and the triangle (q_t * D(t, s)) . k_s
+// The triangle's two halves of 32 tokens are walked with the products of the decays in registers (a warp per four columns, a
+// lane per DK / 32 channels); the square between them is one product on the tensor cores, q_t D(t, 32) against k_s D(32, s).
+__host__ __device__ __forceinline__ int vec_floats(int dk) { return 2 * CC * dk + CC * CC + dk; }
+constexpr int PREP_THREADS = 512, PREP_COLS = 4, HALF = CC / 2;
+
+template <int DK>
+struct PrepSizes {
+    static constexpr int LK = DK + PAD;
+    static constexpr size_t decays = (size_t)CC * DK * sizeof(float), q = (size_t)CC * DK * sizeof(bf);
+    static constexpr size_t planes = (size_t)3 * HALF * LK * sizeof(bf), bytes = decays + q + 2 * planes;
+};
+
+template <int DK>
+__global__ void __launch_bounds__(PREP_THREADS, 2) chunk_prepare_kernel(const __grid_constant__ ChunkArgs a) {
+    pdl_launch_dependents();
+    using Z = PrepSizes<DK>;
+    constexpr int LK = Z::LK, PARTS = PREP_THREADS / DK, L = CC / PARTS, PER = DK / 32;
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* dec = reinterpret_cast<float*>(smem);                       // [CC][DK]
+    bf* qs = reinterpret_cast<bf*>(smem + Z::decays);                  // [CC][DK], as stored
+    bf* qt = qs + Z::q / sizeof(bf);                                   // [3][HALF][LK]: the second half's q_t D(t, 32)
+    bf* kt = qt + Z::planes / sizeof(bf);                              // [3][HALF][LK]: the first half's k_s D(32, s)
+    __shared__ float total[PARTS][DK];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.y, H = a.H, dk = a.dk, place = a.first + blockIdx.x;
+    pdl_wait();
+    int lo = 0, hi = a.B - 1;                      // the last sequence whose chunks start at or ahead of this place
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (first_place(a.cu_rows, mid) <= place) lo = mid;
+        else hi = mid - 1;
+    }
+    const int row = a.cu_rows[lo] + (place - first_place(a.cu_rows, lo)) * CC, n = min(CC, a.cu_rows[lo + 1] - row);
+    if (n <= 0) return;
+    float* kw = a.prep + ((size_t)blockIdx.x * H + h) * vec_floats(dk);
+    float* qw = kw + CC * dk;
+    float* tri = qw + CC * dk;
+    float* keep = tri + CC * CC;
+
+    const int r = tid % DK, part = tid / DK, t_lo = part * L;
+    const bool live = r < dk;
+    {
+        float d[L];
+        float all = 1.f;
+        const float bias = live && a.decay_bias ? a.decay_bias[h * dk + r] : 0.f;
+#pragma unroll
+        for (int i = 0; i < L; ++i) d[i] = live && t_lo + i < n ? a.decay_pre[(size_t)(row + t_lo + i) * a.decay_stride + h * dk + r] : 0.f;
+#pragma unroll
+        for (int i = 0; i < L; ++i) {
+            d[i] = live && t_lo + i < n ? expf(log_sigmoid(d[i] + bias) * a.inv_tau) : 1.f;
+            dec[(t_lo + i) * DK + r] = d[i];
+            all *= d[i];
+        }
+        total[part][r] = all;
+        __syncthreads();
+        // What the parts ahead and behind multiply: within this half, and within the chunk.
+        float ahead = 1.f, behind = 1.f, ahead_half = 1.f, behind_half = 1.f;
+        constexpr int HP = PARTS / 2;              // parts of a half
+#pragma unroll
+        for (int p = 0; p < PARTS; ++p) {
+            const float f = total[p][r];
+            if (p < part) ahead *= f;
+            if (p > part) behind *= f;
+            if (p < part && p / HP == part / HP) ahead_half *= f;
+            if (p > part && p / HP == part / HP) behind_half *= f;
+        }
+        if (part == 0 && live) keep[r] = all * behind;
+        const bf* src = a.rows + (size_t)row * a.stride + h * dk + (live ? r : 0);
+        const bool late = part >= HP;
+        float run = 1.f;
+#pragma unroll
+        for (int i = 0; i < L; ++i) {
+            const int t = t_lo + i;
+            const bool in = live && t < n;
+            const bf raw = in ? src[(size_t)t * a.stride + a.q_off] : __float2bfloat16_rn(0.f);
+            const float q = __bfloat162float(raw);
+            run *= d[i];
+            qs[t * DK + r] = raw;
+            if (live) qw[t * dk + r] = q * a.q_scale * (run * ahead);
+            if (late) {
+                float x = q * (run * ahead_half);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const bf y = __float2bfloat16_rn(x);
+                    qt[(p * HALF + t - HALF) * LK + r] = y;
+                    x -= __bfloat162float(y);
+                }
+            }
+        }
+        run = 1.f;
+#pragma unroll
+        for (int i = L - 1; i >= 0; --i) {
+            const int t = t_lo + i;
+            const float k = live && t < n ? to_f32(src[(size_t)t * a.stride + a.k_off]) : 0.f;
+            if (live) kw[t * dk + r] = k * a.k_scale * (run * behind);
+            if (!late) {
+                float x = k * (run * behind_half);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const bf y = __float2bfloat16_rn(x);
+                    kt[(p * HALF + t) * LK + r] = y;
+                    x -= __bfloat162float(y);
+                }
+            }
+            run *= d[i];
+        }
+    }
+    __syncthreads();
+    const float scale = a.q_scale * a.k_scale;
+    if (warp < 8) {   // ---- the square between the halves: 16 rows and 8 columns a warp
+        const int mi = warp >> 2, nj = warp & 3, g = lane >> 2, t = lane & 3;
+        float acc[4] = {};
+#pragma unroll
+        for (int kk = 0; kk < DK / 32; ++kk) {
+            uint32_t kf[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldsm_x4(kt + (size_t)(p * HALF + nj * 8 + (lane & 7)) * LK + kk * 32 + (lane >> 3) * 8, kf[p]);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                uint32_t qf[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    ldsm_x4(qt + (size_t)(p * HALF + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LK + kk * 32 + x * 16 + (lane >> 4) * 8, qf[p]);
+                float d[3][4] = {};
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int sum = 2; sum >= i; --sum) mma_bf16(d[sum], qf[i], kf[sum - i][2 * x], kf[sum - i][2 * x + 1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] += (d[2][e] + d[1][e]) + d[0][e];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<float2*>(tri + (HALF + mi * 16 + g + e * 8) * CC + nj * 8 + 2 * t) = make_float2(acc[2 * e] * scale, acc[2 * e + 1] * scale);
+    }
+    {   // ---- the halves: four columns from s0 on a warp, every row of the half from their 16-row block on
+        constexpr int N = PREP_COLS;
+        const int s0 = (warp >> 3) * HALF + (warp & 7) * N, end = (warp >> 3) * HALF + HALF, ch = lane * PER;
+        float p[N][PER] = {};
+        auto decay_row = [&](int t, float (&d)[PER]) {
+            if constexpr (PER == 4) *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(dec + t * DK + ch);
+            else *reinterpret_cast<float2*>(d) = *reinterpret_cast<const float2*>(dec + t * DK + ch);
+        };
+        auto unpack = [&](const uint32_t (&w)[PER / 2], float (&x)[PER]) {
+#pragma unroll
+            for (int c = 0; c < PER; c += 2) { x[c] = low_f32(w[c / 2]); x[c + 1] = high_f32(w[c / 2]); }
+        };
+        auto row_sums = [&](int t) {               // q_t . p_i for the four columns, to row t of the triangle
+            uint32_t w[PER / 2];
+            if constexpr (PER == 4) *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(qs + t * DK + ch);
+            else w[0] = *reinterpret_cast<const uint32_t*>(qs + t * DK + ch);
+            float q[PER], v[N];
+            unpack(w, q);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                v[i] = 0.f;
+#pragma unroll
+                for (int c = 0; c < PER; ++c) v[i] = fmaf(q[c], p[i][c], v[i]);
+            }
+            // Four sums over the lanes at once: halves of the values change sides until lane l is left with column l & 3.
+#pragma unroll
+            for (int x = N / 2; x >= 1; x >>= 1) {
+                const bool upper = lane & x;
+#pragma unroll
+                for (int i = 0; i < x; ++i) {
+                    const float give = upper ? v[i] : v[i + x], mine = upper ? v[i + x] : v[i];
+                    v[i] = mine + __shfl_xor_sync(0xffffffffu, give, x);
+                }
+            }
+#pragma unroll
+            for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            if (lane < N) tri[t * CC + s0 + lane] = v[0] * scale;
+        };
+        for (int t = s0 / 16 * 16 + lane / N; t < s0; t += 32 / N) tri[t * CC + s0 + lane % N] = 0.f;
+        float k[N][PER];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            uint32_t w[PER / 2] = {};
+            if (s0 + i < n && ch < dk) {
+                const bf* src = a.rows + (size_t)(row + s0 + i) * a.stride + a.k_off + h * dk + ch;
+                if constexpr (PER == 4) *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(src);
+                else w[0] = *reinterpret_cast<const uint32_t*>(src);
+            }
+            unpack(w, k[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {              // the four tokens themselves: column i starts at its own row
+            float d[PER];
+            decay_row(s0 + i, d);
+#pragma unroll
+            for (int c = 0; c < PER; ++c) {
+#pragma unroll
+                for (int j = 0; j < i; ++j) p[j][c] *= d[c];
+                p[i][c] = k[i][c];
+            }
+            row_sums(s0 + i);
+        }
+#pragma unroll 4
+        for (int t = s0 + N; t < end; ++t) {
+            float d[PER];
+            decay_row(t, d);
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int c = 0; c < PER; ++c) p[j][c] *= d[c];
+            row_sums(t);
+        }
+    }
+}
+
 // ------------------------------------------------------------------ state
 // 8 NTL value columns a block.  Warps 0 to 3 multiply; the others stage: what a stager reads comes by cp.async into a ring of
 // its own, RING chunks deep, is rotated, scaled and split and goes to one of two buffers while the other is multiplied.
@@ -202,8 +426,9 @@ struct StateSizes {
     static constexpr int LK = DK + PAD, LV = 8 * NTL + PAD;
     static constexpr int GROUPS = ROT ? DK / 16 : DK / 8;            // eight channels (and their partners of the rotation)
     static constexpr int ITEMS = CC * GROUPS / STAGERS;              // of a stager's chunk
-    static constexpr int PIECES = ROT ? 6 : 1;                       // of 16 bytes an item: the channels, the partners, two of cosines and of sines
-    static constexpr int RING = ROT && DK == 128 ? 2 : 4;
+    // Pieces of 16 bytes an item: the channels, the partners, two of cosines and of sines; or eight prepared float32 channels.
+    static constexpr int PIECES = ROT ? 6 : (MODE == VEC ? 2 : 1);
+    static constexpr int RING = DK < 128 || PIECES == 1 ? 4 : (MODE == VEC ? 3 : 2);
     static constexpr size_t planes = (size_t)2 * 3 * CC * LK * sizeof(bf);
     static constexpr size_t raw = (size_t)RING * ITEMS * PIECES * STAGERS * 16;
     static constexpr size_t weights = MODE == GATED ? (size_t)RING * ITEMS * STAGERS * 4 : 0;
@@ -231,6 +456,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
     if (c_lo >= c_hi) return;
     float* st = a.state + (long long)a.slots[b] * a.slot_stride + (size_t)h * (dk + X) * (dv + X);
     const GateRecord* gates = reinterpret_cast<const GateRecord*>(a.gates) + (ptrdiff_t)(base - a.first) * H + h;     // chunk c's: gates[c * H]
+    const float* prep = a.prep + ((ptrdiff_t)(base - a.first) * H + h) * vec_floats(dk);       // chunk c's: prep + c * H * vec_floats
     if (dk < DK)
         for (int j = tid; j < (int)(Z::planes / 16); j += STATE_THREADS) reinterpret_cast<uint4*>(planes)[j] = make_uint4(0, 0, 0, 0);
     if (MODE == HEAD) decay_powers(a.decay[h], pw, tid, STATE_THREADS);
@@ -256,6 +482,12 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
                     const bool in = s < n && ch < width;
                     const bf* p = a.rows + (size_t)(row + (in ? s : 0)) * a.stride + a.k_off + h * dk + (in ? ch : 0);
                     uint4* dst = raw + (size_t)((c % RING) * ITEMS + i) * PIECES * STAGERS + ptid;
+                    if constexpr (MODE == VEC) {
+                        const float* w = prep + (ptrdiff_t)c * H * vec_floats(dk) + (ch < width ? s * dk + ch : 0);
+                        copy16(dst, w, ch < width);
+                        copy16(dst + STAGERS, w + 4, ch < width);
+                        continue;
+                    }
                     copy16(dst, p, in);
                     if constexpr (ROT) {
                         copy16(dst + STAGERS, p + (in ? half : 0), in);
@@ -281,10 +513,17 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
             for (int i = 0; i < ITEMS; ++i) {
                 const int s = s_first + i * S_STEP;
                 const uint4* src = raw + (size_t)((c % RING) * ITEMS + i) * PIECES * STAGERS + ptid;
-                const float f = (MODE == GATED ? raw_w[((c % RING) * ITEMS + i) * STAGERS + ptid] : (s < n ? pw[n - 1 - s] : 0.f)) * a.k_scale;
+                const float f = MODE == VEC ? 1.f : (MODE == GATED ? raw_w[((c % RING) * ITEMS + i) * STAGERS + ptid] : (s < n ? pw[n - 1 - s] : 0.f)) * a.k_scale;
                 const uint4 lo = src[0];
                 const uint32_t* x = reinterpret_cast<const uint32_t*>(&lo);
                 uint32_t p0[4][3], p1[ROT ? 4 : 1][3];
+                if constexpr (MODE == VEC) {
+                    const uint4 more = src[STAGERS];
+                    split3(__uint_as_float(lo.x), __uint_as_float(lo.y), p0[0]);
+                    split3(__uint_as_float(lo.z), __uint_as_float(lo.w), p0[1]);
+                    split3(__uint_as_float(more.x), __uint_as_float(more.y), p0[2]);
+                    split3(__uint_as_float(more.z), __uint_as_float(more.w), p0[3]);
+                } else {
                 uint4 hi;
                 float4 cs[2], sn[2];
                 if constexpr (ROT) {
@@ -308,6 +547,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
                         u1 = u1 * c1 - v1 * s1;
                     }
                     split3(u0 * f, u1 * f, p0[e]);
+                }
                 }
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
@@ -370,6 +610,20 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
         }
     }
     float keep = MODE == GATED ? gates[(size_t)c_lo * H].keep : 0.f;
+    float keep_row[MT][2];                         // VEC: D(n, 0) of this lane's rows
+    auto fetch_keep = [&](int c) {
+        if constexpr (MODE == VEC) {
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = r_base + i * 16 + g + e * 8;
+                    keep_row[i][e] = r < dk && c < c_hi ? prep[(ptrdiff_t)c * H * vec_floats(dk) + 2 * CC * dk + CC * CC + r] : 0.f;
+                }
+            }
+        }
+    };
+    fetch_keep(c_lo);
     copy_wait<V_RING - 2>();
     __syncthreads();
     for (int c = c_lo; c < c_hi; ++c) {
@@ -400,10 +654,11 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
 #pragma unroll
             for (int j = 0; j < NTL; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) S[i][j][e] *= keep;
+                for (int e = 0; e < 4; ++e) S[i][j][e] *= MODE == VEC ? keep_row[i][e >> 1] : keep;
 #pragma unroll
             for (int e = 0; e < 4; ++e) N[i][e] *= keep;
         }
+        fetch_keep(c + 1);
         const bf* src = planes + (size_t)(c & 1) * 3 * CC * LK;
         const bf* val = vals + (size_t)(c % V_RING) * CC * LV;
 #pragma unroll
@@ -463,10 +718,10 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
 // place, so that three blocks share a multiprocessor (two where q and k are rotated heads of 128, whose k comes in two halves).
 template <int DK, int DV, Mode MODE, bool ROT>
 struct OutSizes {
-    static constexpr int NQ = ROT ? 3 : 1;               // rotated q and k are float32: three terms
+    static constexpr int NQ = ROT || MODE == VEC ? 3 : 1;     // rotated q and k, and q with its decays, are float32: three terms
     static constexpr int LK = DK + PAD, LP = CC + PAD, LV = DV + PAD;
     static constexpr int HALVES = ROT && DK == 128 ? 2 : 1;
-    static constexpr size_t q = (size_t)NQ * CC * LK * sizeof(bf), k = q / HALVES, p = (size_t)3 * CC * LP * sizeof(bf);
+    static constexpr size_t q = (size_t)NQ * CC * LK * sizeof(bf), k = MODE == VEC ? 0 : q / HALVES, p = (size_t)3 * CC * LP * sizeof(bf);
     static constexpr size_t v = (size_t)CC * LV * sizeof(bf), rows_out = MODE == GATED ? (size_t)CC * (DV + 4) * sizeof(float) : 0;
     static constexpr size_t work = q + v + (HALVES == 1 ? (k > p ? k : p) : k + p), bytes = work > rows_out ? work : rows_out;
 };
@@ -541,8 +796,37 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
         for (int j = tid; j < (int)(Z::work / 16); j += 128) reinterpret_cast<uint4*>(smem)[j] = make_uint4(0, 0, 0, 0);
         __syncthreads();
     }
-    stage(0, 0, CC);
-    stage(1, 0, HC);
+    if constexpr (MODE == VEC) {
+        const float* prep = a.prep + ((size_t)blockIdx.x * H + h) * vec_floats(dk) + CC * dk;
+#pragma unroll 4
+        for (int j = tid; j < CC * (DK / 8); j += 128) {
+            const int s = j / (DK / 8), ch = (j % (DK / 8)) * 8;
+            uint32_t p[4][3] = {};
+            if (ch < dk) {
+                const float4 x = *reinterpret_cast<const float4*>(prep + s * dk + ch), y = *reinterpret_cast<const float4*>(prep + s * dk + ch + 4);
+                split3(x.x, x.y, p[0]);
+                split3(x.z, x.w, p[1]);
+                split3(y.x, y.y, p[2]);
+                split3(y.z, y.w, p[3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(qp + ((size_t)i * CC + s) * LK + ch) = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
+        }
+#pragma unroll 4
+        for (int j = tid; j < CC * (CC / 4); j += 128) {
+            const int tt = j / (CC / 4), s = (j % (CC / 4)) * 4;
+            if (s / 16 > tt / 16) continue;        // never read
+            const float4 x = *reinterpret_cast<const float4*>(prep + CC * dk + tt * CC + s);
+            uint32_t p[2][3];
+            split3(x.x, x.y, p[0]);
+            split3(x.z, x.w, p[1]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(pp + ((size_t)i * CC + tt) * LP + s) = make_uint2(p[0][i], p[1][i]);
+        }
+    } else {
+        stage(0, 0, CC);
+        stage(1, 0, HC);
+    }
     copy_commit();
 #pragma unroll
     for (int j = tid; j < CC * (DV / 8); j += 128) {
@@ -553,7 +837,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     copy_commit();
     if (MODE == HEAD) {
         decay_powers(a.decay[h], pw, tid, 128);
-    } else if (tid < CC) {
+    } else if (MODE == GATED && tid < CC) {
         const GateRecord& r = reinterpret_cast<const GateRecord*>(a.gates)[(size_t)blockIdx.x * H + h];
         up[tid] = r.up[tid];
         down[tid] = r.down[tid];
@@ -584,7 +868,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     }
 
     // ---- the triangle D(t, s) (q_t . k_s): this warp's 16 rows, the 16-column steps up to the diagonal
-    {
+    if constexpr (MODE != VEC) {
         float s_acc[8][4] = {};
 #pragma unroll
         for (int half = 0; half < HALVES; ++half) {
@@ -713,7 +997,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     for (int i = 0; i < MTB; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const float f = f_row[(i * WM + wm) * 16 + g + (e >> 1) * 8];
+            const float f = MODE == VEC ? 1.f : f_row[(i * WM + wm) * 16 + g + (e >> 1) * 8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j][e] *= f;
         }
@@ -743,7 +1027,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
         }
     }
     // ---- out
-    if (MODE == HEAD) {
+    if (MODE != GATED) {
 #pragma unroll
         for (int i = 0; i < MTB; ++i)
 #pragma unroll
@@ -817,33 +1101,40 @@ int launch_mode(const ChunkArgs& a, bool gated, cudaStream_t stream) {
         if (int e = launch_pdl(chunk_gates_kernel, dim3(a.B, a.H), dim3(256), 0, stream, a)) return e;
         return launch_both<DK, GATED, false>(a, stream);
     }
+    if (a.decay_pre) {
+        constexpr size_t smem = PrepSizes<DK>::bytes;
+        if (int e = set_smem(chunk_prepare_kernel<DK>, smem)) return e;
+        if (int e = launch_pdl(chunk_prepare_kernel<DK>, dim3(a.places, a.H), dim3(PREP_THREADS), smem, stream, a)) return e;
+        return launch_both<DK, VEC, false>(a, stream);
+    }
     return a.cos_t ? launch_both<DK, HEAD, true>(a, stream) : launch_both<DK, HEAD, false>(a, stream);
 }
 
 }  // namespace
 
-// Chunk places of a step with these rows and sequences, and floats of scratch for one of them.
-LQ_EXPORT long long lq_chunk_place_floats(int H, int dk, int dv, int gated) {
-    return (long long)H * dk * ((dv + 31) / 32 * 32 + (gated ? 4 : 0)) + (gated ? (long long)H * GATE_FLOATS : 0);
+// Floats of scratch for one chunk place.  kind: 0 a fixed decay, 1 gates, 2 decays per key channel.
+LQ_EXPORT long long lq_chunk_place_floats(int H, int dk, int dv, int kind) {
+    return (long long)H * dk * ((dv + 31) / 32 * 32 + (kind == 1 ? 4 : 0)) + (long long)H * (kind == 1 ? GATE_FLOATS : kind == 2 ? vec_floats(dk) : 0);
 }
 
 // As lq_linear_scan for steps with prompts in bfloat16: dk and dv multiples of 8 up to 128, offsets and stride in whole eights;
 // with a fixed decay, rotation over whole heads (dk a multiple of 16) or none.  `places` chunks of scratch are worked on at a time.
 LQ_EXPORT int lq_chunk_scan(const void* qkv, int stride, int q_off, int k_off, int v_off, const float* cos_t, const float* sin_t,
                             const int* tok_pos, const float* gate_pre, const float* gate_bias, float gate_cap, const float* decay,
-                            float q_scale, float k_scale, float* state, long long slot_stride, const int* cu_rows, const int* slots,
-                            float* out, float* exp_neg_m, float* scratch, int places, int rows, int B, int H, int dk, int dv,
-                            cudaStream_t stream) {
+                            const float* decay_pre, int decay_stride, const float* decay_bias, float inv_tau, float q_scale,
+                            float k_scale, float* state, long long slot_stride, const int* cu_rows, const int* slots, float* out,
+                            float* exp_neg_m, float* scratch, int places, int rows, int B, int H, int dk, int dv, cudaStream_t stream) {
     if (B <= 0 || rows <= 0) return LQ_OK;
     const bool gated = gate_pre != nullptr;
     if (dk < 8 || dv < 8 || dk > 128 || dv > 128 || dk % 8 || dv % 8 || places < 1) return LQ_BAD_SIZE;
-    if (cos_t && (gated || dk % 16 || !sin_t || !tok_pos)) return LQ_BAD_SIZE;
+    if (cos_t && (gated || decay_pre || dk % 16 || !sin_t || !tok_pos)) return LQ_BAD_SIZE;
     if (stride % 8 || q_off % 8 || k_off % 8 || v_off % 8 || (uintptr_t)qkv % 16 || (uintptr_t)cos_t % 16 || (uintptr_t)sin_t % 16 ||
         (uintptr_t)scratch % 16) return LQ_BAD_SIZE;
-    if (gated ? (!gate_bias || !exp_neg_m) : !decay) return LQ_BAD_SIZE;
+    if (gated ? (!gate_bias || !exp_neg_m || decay_pre) : (!decay && !decay_pre)) return LQ_BAD_SIZE;
     ChunkArgs a{(const bf*)qkv, stride, q_off, k_off, v_off, cos_t, sin_t, tok_pos, gate_pre, gate_bias, gate_cap, decay, q_scale, k_scale,
-                state, slot_stride, cu_rows, slots, out, exp_neg_m, scratch, nullptr, H, dk, dv, (dv + 31) / 32 * 32 + (gated ? 4 : 0), B, 0, 0};
-    a.gates = scratch + (size_t)places * H * dk * a.ld;      // 16-byte aligned: dk and ld are whole eights and fours
+                state, slot_stride, cu_rows, slots, out, exp_neg_m, scratch, nullptr, decay_pre, decay_stride, decay_bias, inv_tau, nullptr,
+                H, dk, dv, (dv + 31) / 32 * 32 + (gated ? 4 : 0), B, 0, 0};
+    a.gates = a.prep = scratch + (size_t)places * H * dk * a.ld;      // 16-byte aligned: dk and ld are whole eights and fours
     const int all = rows / CC + B;
     for (a.first = 0; a.first < all; a.first += places) {
         a.places = all - a.first < places ? all - a.first : places;

@@ -119,6 +119,11 @@ def load(name: str, extra_flags: list[str] | None = None) -> ctypes.CDLL:
         return _loaded[name]
 
 
+def loaded(name: str) -> bool:
+    """Whether load(name) has been called with the usual flags."""
+    return name in _loaded
+
+
 def all_sources() -> list[str]:
     return sorted(p.stem for p in CSRC.glob("*.cu"))
 

@@ -142,7 +142,9 @@ def prepare(dtype: torch.dtype, verbose: bool = True, extra: tuple = ()) -> None
     that parts of the model name beyond the common ones (`Part.kernel_libraries`)."""
     from concurrent.futures import ThreadPoolExecutor
     names = ["plain_kernels", *extra] + (["gemm_skinny", "gemm_tc", "gemm_pair"] if dtype == torch.bfloat16 else [])
-    names = list(dict.fromkeys(names))
+    names = [n for n in dict.fromkeys(names) if not build.loaded(n)]
+    if not names:
+        return
     with ThreadPoolExecutor(max_workers=len(names)) as pool:
         list(pool.map(build.build, names))
     for name in names:
@@ -927,16 +929,18 @@ def moe_down(u: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, weights: 
 # ------------------------------------------------------------------ mixers with a matrix state per head
 # Rows a sequence, on average, from which the scan runs by chunks: its two or three launches pay from one whole chunk on (32 heads
 # of 64 / of 128, one sequence, us by tokens and by chunks: 32 rows 11.5 / 22 and 16 / 24, 64 rows 19 / 39 and 18 / 26, 256 rows
-# 67 / 136 and 23 / 37).
+# 67 / 136 and 23 / 37).  With decays per key channel a third launch prepares every chunk: 128 rows (26 / 88 and 27 / 52).
 CHUNK_SCAN_ROWS = 64
+CHUNK_SCAN_ROWS_CHANNELS = 128
 CHUNK_SCRATCH_FLOATS = 1 << 27        # the most scratch that the scan by chunks takes at a time (512 MB); longer steps run in turns
 
 
-def _scan_takes_chunks(qkv: torch.Tensor, offsets: tuple, B: int, dk: int, dv: int, mlstm: bool, cos, sin, dims: int) -> bool:
-    """Whether lq_chunk_scan takes a step's rows (sizes, types and alignment) and is the faster kernel for them."""
-    return (qkv.dtype == torch.bfloat16 and qkv.shape[0] >= CHUNK_SCAN_ROWS * B and dk % 8 == 0 and dv % 8 == 0 and dk <= 128 and dv <= 128
+def _scan_takes_chunks(qkv: torch.Tensor, offsets: tuple, fewest: int, dk: int, dv: int, turns: bool, cos, sin, dims: int) -> bool:
+    """Whether lq_chunk_scan takes a step's rows (sizes, types and alignment; turns: a form that it also takes rotated) and is the
+    faster kernel for them."""
+    return (qkv.dtype == torch.bfloat16 and qkv.shape[0] >= fewest and dk % 8 == 0 and dv % 8 == 0 and dk <= 128 and dv <= 128
             and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and all(o % 8 == 0 for o in offsets)
-            and (not dims or (not mlstm and dims == dk and dk % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (cos, sin)))))
+            and (not dims or (turns and dims == dk and dk % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (cos, sin)))))
 
 
 def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_rows, slots, tok_pos,
@@ -979,19 +983,22 @@ def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: to
     if decay is not None and (decay.dtype != torch.float32 or decay.numel() != H):
         raise KernelError("linear_scan: decay must be float32 [H]")
     cos, sin, dims = rot if rot is not None else (None, None, 0)
-    if channel_decay is None and in_act is None and not (single and rows == B) and \
-            _scan_takes_chunks(qkv, (q_off, k_off, v_off), B, dk, dv, mlstm, cos, sin, dims):
+    if in_act is None and not (single and rows == B) and \
+            _scan_takes_chunks(qkv, (q_off, k_off, v_off), B * (CHUNK_SCAN_ROWS if d_pre is None else CHUNK_SCAN_ROWS_CHANNELS),
+                               dk, dv, decay is not None, cos, sin, dims):
         count = build.load("chunk_scan").lq_chunk_place_floats
         count.argtypes, count.restype = [c_int] * 4, c_longlong
-        each = count(H, dk, dv, int(mlstm))
+        kind = 1 if mlstm else 2 if d_pre is not None else 0
+        each = count(H, dk, dv, kind)
         places = max(1, min(rows // 64 + B, CHUNK_SCRATCH_FLOATS // each))
         scratch = torch.empty(places * each, dtype=torch.float32, device=qkv.device)
         fn = _fn("chunk_scan", "lq_chunk_scan", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                                 c_float, c_void_p, c_float, c_float, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
-                                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+                                                 c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_float, c_void_p, c_longlong,
+                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
         _check(fn(_p(qkv), qkv.stride(0), q_off, k_off, v_off, _p(cos), _p(sin), _p(tok_pos), _p(pre), _p(bias), float(cap), _p(decay),
-                  float(q_scale), float(k_scale), _p(state), state.stride(0), _p(cu_rows), _p(slots), _p(out), _p(enm), _p(scratch), places,
-                  rows, B, H, dk, dv, _stream()), "linear_scan", (3 if mlstm else 2) * -(-(rows // 64 + B) // places), "linear_scan:chunks")
+                  _p(d_pre), d_pre.stride(0) if d_pre is not None else 0, _p(d_bias), 1.0 / float(tau), float(q_scale), float(k_scale), _p(state),
+                  state.stride(0), _p(cu_rows), _p(slots), _p(out), _p(enm), _p(scratch), places, rows, B, H, dk, dv, _stream()),
+               "linear_scan", (3 if kind else 2) * -(-(rows // 64 + B) // places), "linear_scan:chunks")
         return out, enm
     fn = _fn("recurrent", "lq_linear_scan", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                                              c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_float, c_float, c_void_p,

@@ -30,9 +30,9 @@ Gates, decays, the state and the per-head norms are 32-bit in both precisions; t
 gates' pre-activations come from a 32-bit product of their own.  A sequence's tokens
 are walked in order from the state in its slot (`csrc/recurrent.cu`: one kernel for
 prompts and portions, one for steps of a single token per sequence), so a position's
-result does not depend on how its prompt was cut, beyond rounding.  (In bfloat16, prompts of "retention" and "mlstm" run by
-chunks of 64 tokens on the tensor cores, `csrc/chunk_scan.cu`; "lightning" walks prompts by records of four tokens,
-`csrc/delta.cu`.)
+result does not depend on how its prompt was cut, beyond rounding.  (In bfloat16, prompts of "retention", "mlstm" and
+"channel_decay" run by chunks of 64 tokens on the tensor cores, `csrc/chunk_scan.cu`; "lightning" walks prompts by records of
+four tokens, `csrc/delta.cu`.)
 """
 from __future__ import annotations
 

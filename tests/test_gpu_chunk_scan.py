@@ -58,6 +58,16 @@ def _case(kind, lens, H, dk, dv, pad=0, seed=0):
         g = pre.double() + bias.double()
         li, lf = cap * torch.tanh(g[:, :H] / cap), torch.nn.functional.logsigmoid(cap * torch.tanh(g[:, H:] / cap))
         v = torch.cat([v, torch.ones_like(v[..., :1])], dim=2)
+    elif kind == "channels":
+        # Decays from almost nothing kept to exactly one, in every mixture; a stretch that forgets all in the middle.
+        pre = torch.randn(T, H * dk + 3, generator=gen)[:, 1:1 + H * dk] * 6
+        pre[T // 3:T // 3 + 3] = -60.0
+        bias, tau = torch.randn(H * dk, generator=gen) * 2, 2.0
+        bias[::5], bias[1::7] = 60.0, -12.0
+        dev = torch.zeros(T, H * dk + 3, device=DEV)
+        dev[:, 1:1 + H * dk] = pre.to(DEV)
+        opts["channel_decay"] = (dev[:, 1:1 + H * dk], bias.to(DEV), tau)
+        a = torch.exp(torch.nn.functional.logsigmoid(pre.double() + bias.double()) / tau).view(T, H, dk)
     else:
         decay = torch.linspace(0.5, 1.0, H)
         opts["decay"] = decay.to(DEV)
@@ -101,22 +111,23 @@ SIZES = [([64], 2, 64, 64), ([65, 1, 200], 3, 128, 128), ([191], 1, 16, 8), ([12
 
 
 @pytest.mark.parametrize("lens,H,dk,dv", SIZES)
-@pytest.mark.parametrize("kind", ["plain", "rotated", "mlstm"])
-def test_chunks_follow_the_recurrence(kind, lens, H, dk, dv):
+@pytest.mark.parametrize("kind", ["plain", "rotated", "mlstm", "channels"])
+def test_chunks_follow_the_recurrence(kind, lens, H, dk, dv, monkeypatch):
     ops = _ops()
+    monkeypatch.setattr(ops, "CHUNK_SCAN_ROWS_CHANNELS", ops.CHUNK_SCAN_ROWS)      # short sequences as well
     x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv, pad=8)
     got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
     assert chunks == 1
     _check(got, st, want, finals, state, slots)
 
 
-@pytest.mark.parametrize("kind", ["plain", "mlstm"])
+@pytest.mark.parametrize("kind", ["plain", "mlstm", "channels"])
 def test_scratch_for_a_part_of_the_chunks(kind, monkeypatch):
     """The chunks in turns of two places: the state goes on from turn to turn through its slot."""
     ops = _ops()
-    lens, H, dk, dv = [200, 70, 130], 2, 64, 32
+    lens, H, dk, dv = [200, 70, 130], 2, 64, 32         # 133 rows a sequence
     x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv)
-    monkeypatch.setattr(ops, "CHUNK_SCRATCH_FLOATS", 2 * ops.build.load("chunk_scan").lq_chunk_place_floats(H, dk, dv, int(kind == "mlstm")))
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH_FLOATS", 2 * ops.build.load("chunk_scan").lq_chunk_place_floats(H, dk, dv, {"plain": 0, "mlstm": 1, "channels": 2}[kind]))
     got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
     assert chunks == 1
     _check(got, st, want, finals, state, slots)
