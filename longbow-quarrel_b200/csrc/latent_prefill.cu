@@ -1,0 +1,409 @@
+// Latent attention (latent_attn.cu) of prompts on the fifth-generation tensor cores, with keys and values expanded once per token.
+//
+// Moving the per-head maps to the query's side (latent_attn_tc.cu) spares single tokens the expansion, but costs a prompt
+// 2 (R + dr) + 2 R operations per pair of tokens and head (2,176 at R = 512, dr = 64) where expanded keys and values of 128 + 64
+// and 128 numbers cost 640, and R x 512 operations per key and head to expand.  From a dozen query tokens per key on the expansion
+// is the smaller part, and what is left is an ordinary attention whose heads have keys of their own but for the 64 rotated
+// dimensions that all share.
+//   gather   the latent rows that the step sees, out of the cache's pages, side by side (the product behind it expands them)
+//   turn     the rotated part of every head's query, rounded to bfloat16 as the attention reads it
+//   attend   two chains of 128 query rows of one head per block, as attn_prefill_two_kernel of attn_prefill_tc.cu, here two blocks
+//            of tokens that share the head's tiles of 128 keys: S = Q K^T over three panels of 64 dimensions (two of the head's
+//            keys, one shared), P in the place of S, O += P V; keys in two stages, values in one whose halves are freed and
+//            filled by themselves
+// Measured, 2,048 tokens of 16 heads, R = 512, us: attention, expansion and the maps of the absorbed form 686 + 102 + 78, this kernel
+// 64 (340 TFLOP/s; 128 blocks of equal work), the expansion 8, gather and turn 3 each; the whole layer 910 and 184 (heads 32, width
+// 4,096: 1,818 and 321; 4,096 tokens: 5,559 and 657).  Distance of the layer from 64 bits 3.67e-3 absorbed, 3.64e-3 here.
+// Every wait on a barrier is bounded (status word).
+#include "tcgen05.cuh"
+#include <math_constants.h>
+
+using namespace tc;
+
+namespace {
+
+constexpr int BM = 128;                 // query rows of a chain
+constexpr int BN = 128;                 // keys of a tile
+constexpr int DN = 128, DR = 64, DV = 128;      // a head's own key dimensions, the shared ones, its values
+constexpr int PANEL = 128 * 128;        // bytes of a [128 rows, 64 elements] panel
+constexpr int N_THREADS = 384;
+constexpr float RESCALE_STEP = 8.0f;    // log2 units the maximum may run ahead of the reference
+
+struct Smem {
+    alignas(1024) uint8_t q[2][3][PANEL];             // [chain][panel][128 rows x 128 B]
+    alignas(1024) uint8_t k[2][3][PANEL];             // [stage][panel][128 keys x 128 B]
+    alignas(1024) uint8_t v[2][2][PANEL / 2];         // [half of the keys][panel][64 keys x 128 B]
+    alignas(8) uint64_t q_full;
+    uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
+    uint64_t s_full[2], p_full[2], pv_done[2];        // per chain
+    uint32_t tmem_base;
+};
+
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+// x rounded to bfloat16 on the multiply-add pipe, and 2^x by the special-function unit: see attn_prefill_tc.cu.
+__device__ __forceinline__ float bf16_round(float x) {
+    const float p = __fmul_rn(x, 65537.0f);
+    return __fadd_rn(__fsub_rn(x, p), p);
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+#define LQ_WAIT(bar, parity, code) \
+    if (!mbar_wait(smem_u32(&(bar)), (parity))) { give_up(code); ok = false; }
+
+// What the host lists for a step (one int32 array): blocks [7][n] = sequence, then first packed row, rows (0: none) and first
+// position of either chain; first_row [B + 1]: where each sequence's expanded rows start; lo [B]: the position of its first one.
+__global__ void __launch_bounds__(N_THREADS, 1)
+latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr,
+                      const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_kr,
+                      const __grid_constant__ CUtensorMap map_v, const int* __restrict__ blocks, int n_blocks,
+                      const int* __restrict__ first_row, const int* __restrict__ lo, const int* __restrict__ kv_len,
+                      __nv_bfloat16* __restrict__ out, int H, float scale_log2, int window, const float* __restrict__ sink) {
+    extern __shared__ uint8_t smem_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr uint32_t TMEM_COLS = 512;          // S (then P) of the chains in columns 0..127 and 128..255, O from 256 on
+
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&sm.q_full), 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(smem_u32(&sm.k_full[s]), 1);
+            mbar_init(smem_u32(&sm.k_empty[s]), 1);
+            mbar_init(smem_u32(&sm.v_full[s]), 1);
+            mbar_init(smem_u32(&sm.v_empty[s]), 1);
+            mbar_init(smem_u32(&sm.s_full[s]), 1);
+            mbar_init(smem_u32(&sm.p_full[s]), BM);
+            mbar_init(smem_u32(&sm.pv_done[s]), 1);
+        }
+        mbar_fence_init();
+        prefetch_map(&map_q);
+        prefetch_map(&map_qr);
+        prefetch_map(&map_kv);
+        prefetch_map(&map_kr);
+        prefetch_map(&map_v);
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&sm.tmem_base), TMEM_COLS);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem_base = sm.tmem_base;
+    pdl_wait();
+
+    // Heads vary fastest: the blocks with the most keys come first over all heads.
+    const int blk = blockIdx.x / H, h = blockIdx.x % H;
+    const int seq = blocks[blk], len = kv_len[seq];
+    // Chain c's tiles of keys: from[c] .. to[c] - 1 (none without rows); the block walks their union, which has no gap.
+    int row0[2], n_rows[2], pos0[2], from[2], to[2];
+    int t_lo = 0x7fffffff, t_hi = 0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        row0[c] = blocks[(1 + 3 * c) * n_blocks + blk];
+        n_rows[c] = blocks[(2 + 3 * c) * n_blocks + blk];
+        pos0[c] = blocks[(3 + 3 * c) * n_blocks + blk];
+        from[c] = lq_first_key(pos0[c], window) / BN;
+        to[c] = n_rows[c] > 0 ? (pos0[c] + n_rows[c] - 1) / BN + 1 : from[c];
+        if (n_rows[c] > 0) {
+            t_lo = min(t_lo, from[c]);
+            t_hi = max(t_hi, to[c]);
+        }
+    }
+    const int key_row = first_row[seq] - lo[seq];          // the expanded row of position 0
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0 && lane == 0) {
+            // ------------------------------------------------------------ TMA producer
+            bool ok = true;
+            mbar_expect_tx(smem_u32(&sm.q_full), 2 * 3 * PANEL);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                for (int i = 0; i < 2; ++i) tma_load_2d(smem_u32(sm.q[c][i]), &map_q, h * (DN + DR) + i * 64, row0[c], smem_u32(&sm.q_full));
+                tma_load_2d(smem_u32(sm.q[c][2]), &map_qr, h * DR, row0[c], smem_u32(&sm.q_full));
+            }
+            auto load_k = [&](int t) {
+                const int j = t - t_lo, s = j & 1;
+                LQ_WAIT(sm.k_empty[s], ((j >> 1) & 1) ^ 1, 1);
+                if (!ok) return;
+                mbar_expect_tx(smem_u32(&sm.k_full[s]), 3 * PANEL);
+                for (int i = 0; i < 2; ++i) tma_load_2d(smem_u32(sm.k[s][i]), &map_kv, h * DN + i * 64, key_row + t * BN, smem_u32(&sm.k_full[s]));
+                tma_load_2d(smem_u32(sm.k[s][2]), &map_kr, 0, key_row + t * BN, smem_u32(&sm.k_full[s]));
+            };
+            load_k(t_lo);
+            if (ok && t_lo + 1 < t_hi) load_k(t_lo + 1);
+            for (int t = t_lo; t < t_hi && ok; ++t) {
+                for (int x = 0; x < 2 && ok; ++x) {
+                    LQ_WAIT(sm.v_empty[x], ((t - t_lo) & 1) ^ 1, 2);
+                    if (!ok) break;
+                    mbar_expect_tx(smem_u32(&sm.v_full[x]), PANEL);
+                    for (int i = 0; i < 2; ++i)
+                        tma_load_2d(smem_u32(sm.v[x][i]), &map_v, (H + h) * DV + i * 64, key_row + t * BN + x * 64, smem_u32(&sm.v_full[x]));
+                }
+                if (ok && t + 2 < t_hi) load_k(t + 2);
+            }
+        } else if (warp == 1 && lane == 0) {
+            // ------------------------------------------------------------ MMA issuer
+            constexpr uint32_t idesc_s = idesc_bf16(BM, BN, false);
+            constexpr uint32_t idesc_pv = idesc_bf16(BM, DV, true);
+            bool ok = true;
+            auto active = [&](int c, int t) { return t >= from[c] && t < to[c]; };
+            auto issue_s = [&](int c, int s) {          // S of chain c from the keys in stage s
+#pragma unroll
+                for (int kk = 0; kk < (DN + DR) / 16; ++kk) {
+                    const uint64_t a = desc_k_major(smem_u32(sm.q[c][kk >> 2]) + (kk & 3) * 32);
+                    const uint64_t b = desc_k_major(smem_u32(sm.k[s][kk >> 2]) + (kk & 3) * 32);
+                    mma_f16(tmem_base + c * BN, a, b, idesc_s, kk > 0 ? 1u : 0u);
+                }
+                commit(smem_u32(&sm.s_full[c]));
+            };
+            LQ_WAIT(sm.q_full, 0, 3);
+            if (ok) LQ_WAIT(sm.k_full[0], 0, 4);
+            if (ok) {
+                fence_after();
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    if (active(c, t_lo)) issue_s(c, 0);
+                commit(smem_u32(&sm.k_empty[0]));
+            }
+            int done[2] = {0, 0};                  // tiles of a chain whose P has been waited for
+            for (int t = t_lo; t < t_hi && ok; ++t) {
+                const int j = t - t_lo, s1 = (j + 1) & 1;
+                const int last = active(1, t) ? 1 : 0;     // the chain whose product frees the values
+#pragma unroll
+                for (int c = 0; c < 2 && ok; ++c) {
+                    if (active(c, t)) {
+                        LQ_WAIT(sm.p_full[c], done[c] & 1, 5);
+                        for (int x = 0; x < 2 && ok; ++x) {
+                            LQ_WAIT(sm.v_full[x], j & 1, 6);
+                            if (!ok) break;
+                            fence_after();
+#pragma unroll
+                            for (int kk = 0; kk < BN / 32; ++kk)
+                                mma_f16_ts(tmem_base + 2 * BN + c * DV, tmem_base + c * BN + (x * 4 + kk) * 8,
+                                           desc_mn_major(smem_u32(sm.v[x][0]) + kk * 2048, PANEL / 2), idesc_pv,
+                                           (done[c] > 0 || x > 0 || kk > 0) ? 1u : 0u);
+                            if (c == last) commit(smem_u32(&sm.v_empty[x]));
+                        }
+                        if (!ok) break;
+                        commit(smem_u32(&sm.pv_done[c]));
+                        ++done[c];
+                    }
+                    if (t + 1 < t_hi && active(c, t + 1)) {
+                        // The chain's next S takes the place of its P: issued after P V, it runs after it.
+                        LQ_WAIT(sm.k_full[s1], ((j + 1) >> 1) & 1, 4);
+                        if (!ok) break;
+                        fence_after();
+                        issue_s(c, s1);
+                    }
+                }
+                if (ok && t + 1 < t_hi) commit(smem_u32(&sm.k_empty[s1]));
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------------------------------------------------------- softmax: one thread per query row and chain
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+        const int chain = (warp - 4) >> 2, quarter = warp & 3;
+        const int r = quarter * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const uint32_t tmem_s = tmem_base + chain * BN + lane_base;              // S, then P in its first 64 columns
+        const uint32_t tmem_o = tmem_base + 2 * BN + chain * DV + lane_base;
+        const int rows = chain ? n_rows[1] : n_rows[0], p0 = chain ? pos0[1] : pos0[0];
+        const int t_from = chain ? from[1] : from[0], n_tiles = (chain ? to[1] : to[0]) - t_from;
+        const int pos_r = p0 + r;
+        const int first_r = lq_first_key(pos_r, window);                         // the first key this row sees
+        const int first_last = lq_first_key(p0 + rows - 1, window);              // a tile from here on is inside every row's mask
+        const bool row_ok = r < rows;
+        float m_ref = -CUDART_INF_F, l = 0.f;
+        bool ok = true;
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            LQ_WAIT(sm.s_full[chain], j & 1, 7);         // S of this tile is there, and so is the last tile's P V (issued before it)
+            if (!ok) break;
+            fence_after();
+            float t[BN];
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) ld32(tmem_s + c * 32, reinterpret_cast<uint32_t*>(t) + c * 32);
+            wait_ld();
+            const int kb = (t_from + j) * BN;
+            const bool whole = rows == BM && kb + BN - 1 <= p0 && kb + BN <= len && kb >= first_last;
+            float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+            if (whole) {
+#pragma unroll
+                for (int c = 0; c < BN; ++c) mx[c & 3] = fmaxf(mx[c & 3], t[c]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < BN; ++c) {
+                    const int key = kb + c;
+                    const bool vis = row_ok && key <= pos_r && key < len && key >= first_r;
+                    t[c] = vis ? t[c] : -CUDART_INF_F;
+                    mx[c & 3] = fmaxf(mx[c & 3], t[c]);
+                }
+            }
+            const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
+            // Move the reference only when the maximum has run ahead of it by more than the step.
+            const bool need = m_tile > m_ref + RESCALE_STEP;
+            const float corr = need ? ex2(m_ref - m_tile) : 1.0f;
+            if (need) { m_ref = m_tile; l *= corr; }
+            if (j > 0 && __any_sync(0xffffffffu, need)) {
+#pragma unroll 1
+                for (int c = 0; c < DV / 32; ++c) {
+                    uint32_t o[32];
+                    ld32(tmem_o + c * 32, o);
+                    wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                    st32(tmem_o + c * 32, o);
+                }
+            }
+            const float base = m_ref == -CUDART_INF_F ? 0.f : m_ref;
+            float sums[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t pk[32];
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    const float b0 = bf16_round(ex2(fmaf(t[half * 64 + 2 * c], scale_log2, -base)));
+                    const float b1 = bf16_round(ex2(fmaf(t[half * 64 + 2 * c + 1], scale_log2, -base)));
+                    sums[c & 3] += b0 + b1;
+                    pk[c] = __byte_perm(__float_as_uint(b0), __float_as_uint(b1), 0x7632);
+                }
+                st32(tmem_s + half * 32, pk);           // keys 64 half + 2c, + 1 in column 32 half + c
+            }
+            wait_st();
+            l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
+            fence_before();
+            mbar_arrive(smem_u32(&sm.p_full[chain]));
+        }
+        if (ok && n_tiles > 0) {
+            LQ_WAIT(sm.pv_done[chain], (n_tiles - 1) & 1, 8);
+        }
+        if (ok && n_tiles > 0) {
+            fence_after();
+            if (sink) l += ex2(fmaf(sink[h], 1.4426950408889634f, m_ref == -CUDART_INF_F ? 0.f : -m_ref));
+            const float inv = 1.0f / l;
+            __nv_bfloat16* orow = out + ((size_t)((chain ? row0[1] : row0[0]) + r) * H + h) * DV;
+#pragma unroll 1
+            for (int c = 0; c < DV / 32; ++c) {
+                uint32_t o[32];
+                ld32(tmem_o + c * 32, o);
+                wait_ld();
+                if (row_ok) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        reinterpret_cast<uint4*>(orow + c * 32)[i] =
+                            make_uint4(pack2(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv),
+                                       pack2(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv),
+                                       pack2(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv),
+                                       pack2(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv));
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        fence_after();
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// ------------------------------------------------------------------ gather and turn
+// A warp per expanded row: its latent (R numbers) to c, its shared key part (DR) to kr; positions whose page has gone back
+// (ahead of every window) are zero.
+__global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ pages, const int* __restrict__ page_table, int pt_stride,
+                                                            const int* __restrict__ slots, const int* __restrict__ first_row,
+                                                            const int* __restrict__ lo, int B, int rows, int R, int page_size,
+                                                            __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ kr) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    int b = 0, hi = B - 1;                         // the last sequence that starts at or ahead of this row
+    while (b < hi) {
+        const int mid = (b + hi + 1) / 2;
+        if (first_row[mid] <= row) b = mid;
+        else hi = mid - 1;
+    }
+    const int pos = lo[b] + row - first_row[b];
+    const int page = page_table[(size_t)slots[b] * pt_stride + pos / page_size];
+    const uint4* src = reinterpret_cast<const uint4*>(pages + ((size_t)max(page, 0) * page_size + pos % page_size) * (R + DR));
+    uint4* dc = reinterpret_cast<uint4*>(c + (size_t)row * R);
+    uint4* dr = reinterpret_cast<uint4*>(kr + (size_t)row * DR);
+    for (int i = lane; i < (R + DR) / 8; i += 32) {
+        const uint4 v = page >= 0 ? src[i] : make_uint4(0, 0, 0, 0);
+        if (i < R / 8) dc[i] = v;
+        else dr[i - R / 8] = v;
+    }
+}
+
+// Four pairs a thread: head h's rotated part (columns h (DN + DR) + DN of q) turned by the row's position, to out [T, H DR].
+__global__ void __launch_bounds__(256) latent_turn_kernel(const __nv_bfloat16* __restrict__ q, const float* __restrict__ cos_t,
+                                                          const float* __restrict__ sin_t, const int* __restrict__ tok_pos, int T, int H,
+                                                          __nv_bfloat16* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int e = blockIdx.x * 256 + threadIdx.x, i = (e % (DR / 8)) * 4, h = e / (DR / 8) % H, t = e / (DR / 8) / H;
+    if (t >= T) return;
+    const __nv_bfloat16* src = q + ((size_t)t * H + h) * (DN + DR) + DN + i;
+    __nv_bfloat16* dst = out + ((size_t)t * H + h) * DR + i;
+    uint2 u = *reinterpret_cast<const uint2*>(src), w = *reinterpret_cast<const uint2*>(src + DR / 2);
+    if (cos_t) {
+        const float4 c = *reinterpret_cast<const float4*>(cos_t + (size_t)tok_pos[t] * (DR / 2) + i);
+        const float4 s = *reinterpret_cast<const float4*>(sin_t + (size_t)tok_pos[t] * (DR / 2) + i);
+        const float a0 = __uint_as_float(u.x << 16), a1 = __uint_as_float(u.x & 0xffff0000u), a2 = __uint_as_float(u.y << 16), a3 = __uint_as_float(u.y & 0xffff0000u);
+        const float b0 = __uint_as_float(w.x << 16), b1 = __uint_as_float(w.x & 0xffff0000u), b2 = __uint_as_float(w.y << 16), b3 = __uint_as_float(w.y & 0xffff0000u);
+        u = make_uint2(pack2(a0 * c.x - b0 * s.x, a1 * c.y - b1 * s.y), pack2(a2 * c.z - b2 * s.z, a3 * c.w - b3 * s.w));
+        w = make_uint2(pack2(b0 * c.x + a0 * s.x, b1 * c.y + a1 * s.y), pack2(b2 * c.z + a2 * s.z, b3 * c.w + a3 * s.w));
+    }
+    *reinterpret_cast<uint2*>(dst) = u;
+    *reinterpret_cast<uint2*>(dst + DR / 2) = w;
+}
+
+}  // namespace
+
+LQ_EXPORT int lq_latent_gather(const void* pages, const int* page_table, int pt_stride, const int* slots, const int* first_row,
+                               const int* lo, int B, int rows, int R, int page_size, void* c, void* kr, cudaStream_t stream) {
+    if (rows <= 0) return LQ_OK;
+    if (R % 8 || ((uintptr_t)pages | (uintptr_t)c | (uintptr_t)kr) % 16) return LQ_BAD_SIZE;
+    return launch_pdl(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)pages, page_table, pt_stride,
+                      slots, first_row, lo, B, rows, R, page_size, (__nv_bfloat16*)c, (__nv_bfloat16*)kr);
+}
+
+// q [T, H (128 + 64)] -> the rotated parts [T, H 64] (cos_t null: as they are).
+LQ_EXPORT int lq_latent_turn(const void* q, const float* cos_t, const float* sin_t, const int* tok_pos, int T, int H, void* out,
+                             cudaStream_t stream) {
+    if (T <= 0) return LQ_OK;
+    if (((uintptr_t)q | (uintptr_t)out) % 8 || ((uintptr_t)cos_t | (uintptr_t)sin_t) % 16) return LQ_BAD_SIZE;
+    const long long n = (long long)T * H * (DR / 8);
+    return launch_pdl(latent_turn_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, (const __nv_bfloat16*)q, cos_t, sin_t,
+                      tok_pos, T, H, (__nv_bfloat16*)out);
+}
+
+// q [T, H 192] (its first 128 of a head), qr [T, H 64], kv [rows, H (128 + 128)] keys then values, kr [rows, 64]; out [T, H 128].
+LQ_EXPORT int lq_latent_prefill(const void* q, const void* qr, const void* kv, const void* kr, int T, int rows, const int* blocks, int n_blocks,
+                                const int* first_row, const int* lo, const int* kv_len, void* out, int H, float scale, int window,
+                                const float* sink, cudaStream_t stream) {
+    if (n_blocks <= 0) return LQ_OK;
+    if (scale <= 0.f || ((uintptr_t)q | (uintptr_t)qr | (uintptr_t)kv | (uintptr_t)kr | (uintptr_t)out) % 16) return LQ_BAD_SIZE;
+    CUtensorMap mq, mqr, mk, mkr, mv;
+    int rc = make_map_bf16(&mq, q, T, (long)H * (DN + DR), (long)H * (DN + DR), BM);
+    if (rc == LQ_OK) rc = make_map_bf16(&mqr, qr, T, (long)H * DR, (long)H * DR, BM);
+    if (rc == LQ_OK) rc = make_map_bf16(&mk, kv, rows, (long)H * (DN + DV), (long)H * (DN + DV), BN);
+    if (rc == LQ_OK) rc = make_map_bf16(&mkr, kr, rows, DR, DR, BN);
+    if (rc == LQ_OK) rc = make_map_bf16(&mv, kv, rows, (long)H * (DN + DV), (long)H * (DN + DV), BN / 2);
+    if (rc != LQ_OK) return rc;
+    constexpr size_t smem = sizeof(Smem) + 1024;
+    static_assert(smem <= 232448, "more shared memory than a block may have");
+    if (cudaFuncSetAttribute(latent_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return lq_launch_status();
+    return launch_pdl(latent_prefill_kernel, dim3(n_blocks * H), dim3(N_THREADS), smem, stream, mq, mqr, mk, mkr, mv, blocks, n_blocks,
+                      first_row, lo, kv_len, (__nv_bfloat16*)out, H, scale * 1.4426950408889634f, window, sink);
+}
+
+// The status word in host memory that the device writes through; null when it could not be set up.
+LQ_EXPORT int* lq_latent_prefill_status_word() { return tc::status_word(); }

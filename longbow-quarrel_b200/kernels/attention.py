@@ -38,6 +38,53 @@ def query_blocks(size: int):
     return build
 
 
+# ------------------------------------------------------------------ latent attention over expanded keys and values
+EXPAND_TILE = 128
+# Query rows per key, over a step's sequences, from which keys and values are expanded: measured, us absorbed and expanded, 16 heads:
+# 24 rows 260 / 251, 64 rows 263 / 262 (both the host's launches), 32 rows on 2,000 earlier ones 442 / 251, 2,048 rows 910 / 279; 32
+# heads, 16 rows on 1,000 earlier ones 274 / 218.
+EXPAND_QUERIES = 16
+EXPAND_ELEMENTS = 1 << 29          # the most expanded numbers (1 GB in bfloat16); a longer step keeps the absorbed form
+
+
+def expanded_rows(past, new, window: int) -> tuple[list[int], list[int]]:
+    """(first position, rows) of every sequence's expanded keys: from the first one that a new row sees, in whole tiles, on."""
+    lo = [(max(0, p - window + 1) if window > 0 else 0) // EXPAND_TILE * EXPAND_TILE for p in past]
+    return lo, [p + n - a for p, n, a in zip(past, new, lo)]
+
+
+def expands(past, new, window: int, H: int, per_head: int) -> bool:
+    """Whether a step's latent attention runs over expanded keys and values (per_head numbers for each head and key)."""
+    if max(new) == 1:
+        return False
+    _, rows = expanded_rows(past, new, window)
+    pairs = sum(n * r for n, r in zip(new, rows))
+    return pairs >= EXPAND_QUERIES * sum(rows) and sum(rows) * H * per_head <= EXPAND_ELEMENTS
+
+
+def expanded_work(H: int, per_head: int, window: int, sms: int):
+    """Builder of lq_latent_prefill's step array: blocks [7, n] (sequence, then first row, rows and first position of two chains of
+    at most 128 rows), where every sequence's expanded rows start [B + 1], the position of its first one [B]; empty for a step that
+    keeps the absorbed form."""
+    def build(step) -> np.ndarray:
+        if not expands(step.past, step.new, window, H, per_head):
+            return np.zeros(0, dtype=np.int32)
+        lo, rows = expanded_rows(step.past, step.new, window)
+        tiles = [[(step.cu[b] + r, min(128, n - r), p + r) for r in range(0, n, 128)] for b, (p, n) in enumerate(zip(step.past, step.new))]
+        # Chains of neighbouring rows share all their tiles of keys.  A step whose blocks all run at once is as long as its longest
+        # block: there the first rows go with the last ones, so that all blocks have the same work (not under a window, where
+        # two such chains would have no keys in common).
+        level = window <= 0 and sum((len(t) + 1) // 2 for t in tiles) * H <= sms
+        none, blocks = (0, 0, 0), []
+        for b, t in enumerate(tiles):
+            for i in range((len(t) + 1) // 2):
+                first, second = (i, len(t) - 1 - i) if level else (2 * i, 2 * i + 1)
+                blocks.append((b, *t[first], *(t[second] if first < second < len(t) else none)))
+        blocks.sort(key=lambda e: -sum((e[k + 2] + e[k + 1]) // 128 + 1 for k in (1, 4) if e[k + 1]))
+        return np.concatenate([np.asarray(blocks, dtype=np.int32).T.reshape(-1), np.cumsum([0] + rows), lo]).astype(np.int32)
+    return build
+
+
 # ------------------------------------------------------------------ work list of the decode kernel
 MIN_PART_TILES = KEYS_PER_SPLIT // 16      # the same floor in the kernel's 16-key tiles
 DECODE_TILE = 16

@@ -8,8 +8,9 @@
 Only c and the rotated k_r are cached: one row of `kv_rank + rot_dim` numbers per token for all
 heads (`KVNeed` with one kv head and no value pool).  Keys and values are never expanded per
 cached token: the per-head maps go to the query's side, (W_uk,h^T q_h) . c_j and W_uv,h (sum_j p_j c_j),
-so the attention is multi-query attention over the latent rows (`csrc/latent_attn.cu`), for
-prompts, portions and single tokens alike.
+so the attention is multi-query attention over the latent rows (`csrc/latent_attn.cu`).  A step with many query
+rows per key (prompts; heads of 128 + 64 and values of 128 in bfloat16) expands the keys and values of the positions it sees
+instead, for the length of the step: three and a half times fewer operations per pair (`csrc/latent_prefill.cu`).
 
 Norms, angles, scores and the softmax are 32-bit; in bfloat16 runs the projections' outputs that
 feed a norm or the attention stay 32-bit rows (wide queries, latent means), the cache rows are
@@ -21,6 +22,7 @@ the softmax denominator, with no key and no value).
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..kernels import attention as attention_kernels
@@ -44,7 +46,7 @@ class LatentAttention(Mixer):
 
     @property
     def kernel_libraries(self):
-        return ("latent_attn", "latent_attn_tc", "grouped_gemm") if self.runtime.dtype == torch.bfloat16 else ("latent_attn",)
+        return ("latent_attn", "latent_attn_tc", "grouped_gemm", "latent_prefill") if self.runtime.dtype == torch.bfloat16 else ("latent_attn",)
 
     def __init__(self, runtime: Runtime, hidden_size: int, n_heads: int, head_dim: int, rot_dim: int, value_dim: int,
                  q_rank: int | None, kv_rank: int, scale: float, eps: float, position: PartSpec | None = None,
@@ -66,6 +68,11 @@ class LatentAttention(Mixer):
         self.w_o: linear.LinearWeight | None = None
         self.w_uk = self.w_uv = self.w_uk_t = self.w_uv_t = self.g_q = self.g_kv = None
         self.tc_heads = False
+        # Sizes whose prompts may run over expanded keys and values (w_kv, made at load); whether a step's do is
+        # attention_kernels.expands' answer.
+        self.expandable = (runtime.dtype == torch.bfloat16 and (head_dim, rot_dim, value_dim) == ops.LATENT_EXPANDED and kv_rank % 8 == 0
+                           and self.rot in (0, rot_dim))
+        self.w_kv: linear.LinearWeight | None = None
 
     def cache_need(self):
         return KVNeed(1, self.R + self.dr, self.window, values=False)
@@ -75,7 +82,13 @@ class LatentAttention(Mixer):
         if self.runtime.dtype != torch.bfloat16 or (self.R + self.dr) % 8:
             return {}
         size = ops.latent_tc_tokens(self.H)
-        return {f"latent_blocks{size}": attention_kernels.query_blocks(size)}
+        blocks = attention_kernels.query_blocks(size)
+        if self.w_kv is None:                    # sizes or weights that keep the absorbed form throughout
+            return {f"latent_blocks{size}": blocks}
+        H, each, window = self.H, self.dn + self.dv, int(self.window or 0)
+        absorbed = lambda step: np.zeros(0, dtype=np.int32) if attention_kernels.expands(step.past, step.new, window, H, each) else blocks(step)
+        return {f"latent_blocks{size}:{H}:{window}": absorbed,
+                f"latent_expanded:{H}:{window}": attention_kernels.expanded_work(H, each, window, ops.sm_count(self.runtime.device))}
 
     def weights(self):
         n, H = self.names, self.H
@@ -126,6 +139,25 @@ class LatentAttention(Mixer):
         self.w_uv_t = tensors[n["uv"]].reshape(H, self.dv, self.R).contiguous()
         self.tc_heads = (self.runtime.dtype == torch.bfloat16 and self.w_uk.dtype == torch.bfloat16 and self.dn % 8 == 0
                          and (self.dn + self.dr) % 8 == 0 and self.R % 8 == 0)
+        if self.expandable and self.tc_heads and tensors[n["uv"]].dtype == torch.bfloat16:
+            self.w_kv = linear.LinearWeight(torch.cat([tensors[n["uk"]], tensors[n["uv"]]], dim=0))
+
+    def _expanded(self, q, pages, ctx: StepContext, cache_view, cos, sin):
+        """Attention of a prompt over the keys and values of the positions it sees, expanded here: [T, H dv], or None where the
+        step keeps the absorbed form."""
+        flat = ctx.extra.get(f"latent_expanded:{self.H}:{int(self.window or 0)}")
+        if self.w_kv is None or flat is None or flat.numel() == 0 or q.dtype != torch.bfloat16 or \
+                not ops.latent_attention_tc_takes(pages, cache_view.page_size):
+            return None
+        B = ctx.B
+        n = (flat.numel() - 2 * B - 1) // 7
+        blocks, first_row, lo = flat[:7 * n].view(7, n), flat[7 * n:7 * n + B + 1], flat[7 * n + B + 1:]
+        # Host lists: steps with prompts are never captured (the part stays graph-safe for steps of single tokens).
+        _, rows = attention_kernels.expanded_rows(ctx.h_past, ctx.h_new, int(self.window or 0))
+        c, kr = ops.latent_gather(pages, cache_view.page_table, ctx.slots, first_row, lo, B, sum(rows), self.R, cache_view.page_size)
+        kv = linear.linear(c, self.w_kv, torch.bfloat16)
+        qr = ops.latent_turn(q, cos, sin, ctx.tok_pos, self.H)
+        return ops.latent_prefill(q, qr, kv, kr, blocks, first_row, lo, ctx.kv_len, self.H, self.scale, self.window, self.sinks)
 
     def _splits(self, ctx: StepContext, blocks_per_token: int, places_per_sm: int = 1) -> int:
         """Slices per row for a step of single tokens: as many as fill the multiprocessors, none shorter than
@@ -147,7 +179,8 @@ class LatentAttention(Mixer):
                 return ops.latent_attention_tc(wide, pages, cache_view.page_table, ctx.slots, H, R, cache_view.page_size,
                                                self.scale, self.window, tok_pos=ctx.tok_pos, tok_seq=ctx.tok_seq,
                                                splits=self._splits(ctx, -(-H // 64) * chunks), **more)
-            flat = ctx.extra.get(f"latent_blocks{ops.latent_tc_tokens(H)}")
+            name = f"latent_blocks{ops.latent_tc_tokens(H)}"
+            flat = ctx.extra.get(f"{name}:{H}:{int(self.window or 0)}", ctx.extra.get(name))
             if flat is not None and flat.numel():
                 return ops.latent_attention_tc(wide, pages, cache_view.page_table, ctx.slots, H, R, cache_view.page_size,
                                                self.scale, self.window, blocks=tuple(flat.view(4, -1)), **more)
@@ -167,6 +200,20 @@ class LatentAttention(Mixer):
         ops.latent_kv_store(down, 0, R, self.g_kv, self.eps, cos, sin, self.rot, ctx.tok_pos, ctx.tok_seq, ctx.slots,
                             cache_view.page_table, pages, R, dr, cache_view.page_size)
         q = linear.linear(cq, self.w_uq, act if self.tc_heads else torch.float32)     # [T, H (dn + dr)]
+        out = None if ctx.decode else self._expanded(q, pages, ctx, cache_view, cos, sin)
+        if out is None:
+            out = self._absorbed(q, pages, ctx, cache_view, cos, sin)
+        if self.gate is not None:
+            ops.gate_mul(out, down[:, R + dr:], "sigmoid")
+        if residual is None:
+            return linear.linear(out, self.w_o, torch.float32)
+        linear.linear(out, self.w_o, self.runtime.act_dtype, residual=residual)
+        return None
+
+    def _absorbed(self, q, pages, ctx: StepContext, cache_view, cos, sin):
+        """Attention with the per-head maps on the query's side: [T, H dv]."""
+        H, dn, dr, dv, R = self.H, self.dn, self.dr, self.dv, self.R
+        T = q.shape[0]
         wide = torch.empty((T, H, R + dr), dtype=torch.float32, device=q.device)
         wide2 = wide.view(T, H * (R + dr))
         if self.tc_heads and ops.grouped_gemm_takes(q, self.w_uk_t, dn + dr):
@@ -175,15 +222,10 @@ class LatentAttention(Mixer):
             ops.head_matmul(q, dn + dr, 0, self.w_uk, wide2, R + dr, 0)
         ops.rope_tail(q, dn + dr, dn, wide2, R + dr, R, cos, sin, self.rot, ctx.tok_pos, H, dr)
         mean = self._attend(wide, pages, ctx, cache_view)
-        out = torch.empty((T, H * dv), dtype=act, device=q.device)
+        out = torch.empty((T, H * dv), dtype=self.runtime.act_dtype, device=q.device)
         mean = mean.view(T, H * R)
         if mean.dtype == torch.bfloat16 and ops.grouped_gemm_takes(mean, self.w_uv_t, R):
             ops.grouped_gemm(mean, self.w_uv_t, out, a_group_stride=R, o_group_stride=dv)                  # W_uv,h (sum_j p_j c_j)
         else:
             ops.head_matmul(mean, R, 0, self.w_uv, out, dv, 0)
-        if self.gate is not None:
-            ops.gate_mul(out, down[:, R + dr:], "sigmoid")
-        if residual is None:
-            return linear.linear(out, self.w_o, torch.float32)
-        linear.linear(out, self.w_o, self.runtime.act_dtype, residual=residual)
-        return None
+        return out

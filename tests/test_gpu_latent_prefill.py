@@ -1,0 +1,81 @@
+"""Latent attention of prompts over expanded keys and values (csrc/latent_prefill.cu) against the same part in 32-bit and against
+its absorbed form: edges of the 128-row chains and 128-key tiles, portions, windows, a sink, sequences side by side."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+D, R = 192, 64
+
+
+def _part(dtype, H, window, sink, weights=None):
+    from longbow_quarrel_b200.parts.base import Runtime
+    from longbow_quarrel_b200.parts.latent_attention import LatentAttention
+    from longbow_quarrel_b200.parts.spec import PartSpec
+    from longbow_quarrel_b200.weights import random_weights
+    part = LatentAttention(Runtime(DEV, dtype, 2048), hidden_size=D, n_heads=H, head_dim=128, rot_dim=64, value_dim=128, q_rank=None, kv_rank=R,
+                           scale=0.12, eps=1e-5, position=PartSpec("rope", {"head_dim": 64, "theta": 1e4}), window=window, sink=sink)
+    weights = weights or random_weights(part.weights(), 3, torch.bfloat16, DEV, std=0.08)
+    part.load(weights)
+    return part, weights
+
+
+def _run(part, portions, h):
+    """Steps of the sequences, portion by portion: the rows of every sequence, in order."""
+    from longbow_quarrel_b200.cache import Cache
+    from longbow_quarrel_b200.engine.step import make_context, pack_step
+    from longbow_quarrel_b200.kernels import ops
+    cache = Cache({0: part.cache_need()}, 8192, 2048, part.runtime.dtype, DEV, max_slots=4)
+    slots = [cache.alloc_slot() for _ in h]
+    past, got, routes = [0] * len(h), [[] for _ in h], []
+    for step in portions:
+        live = [i for i, n in enumerate(step) if n]
+        for i in live:
+            cache.reserve(slots[i], step[i])
+        cache.upload()
+        flat, info = pack_step([(slots[i], [0] * step[i]) for i in live], None, [past[i] for i in live], part.step_needs())
+        ctx = make_context(torch.from_numpy(flat).to(DEV), info, [slots[i] for i in live])
+        rows = torch.cat([h[i][past[i]:past[i] + step[i]] for i in live]).to(part.runtime.dtype)
+        before = ops.launches_by_name().get("latent_prefill", 0)
+        out = part.forward(rows, ctx, cache.view(0), None)
+        routes.append(ops.launches_by_name().get("latent_prefill", 0) - before)
+        at = 0
+        for i in live:
+            got[i].append(out[at:at + step[i]])
+            at += step[i]
+            past[i] += step[i]
+            cache.commit(slots[i], step[i])
+    torch.cuda.synchronize()
+    ops.check_status()
+    return [torch.cat(g).double() for g in got], routes
+
+
+@pytest.mark.parametrize("H,window,sink,portions", [
+    (2, None, False, [(128,)]), (3, None, True, [(129, 257, 40)]), (2, None, False, [(300, 0), (70, 511), (33, 100)]), (1, 100, True, [(450, 130), (200, 64)]),
+    (2, 300, False, [(700,), (129,)]), (16, None, False, [(1100,)])])
+def test_expanded_prompts_agree_with_32_bit_and_with_the_absorbed_form(H, window, sink, portions, monkeypatch):
+    from longbow_quarrel_b200.kernels import attention as kernels
+    gen = torch.Generator().manual_seed(H)
+    h = [torch.randn(sum(s[i] for s in portions), D, generator=gen).to(torch.bfloat16).to(DEV) for i in range(len(portions[0]))]
+    part, weights = _part(torch.bfloat16, H, window, sink)
+    got, routes = _run(part, portions, h)
+    assert all(routes)
+    monkeypatch.setattr(kernels, "EXPAND_QUERIES", 10 ** 9)
+    absorbed, routes = _run(part, portions, h)
+    assert not any(routes)
+    want, _ = _run(_part(torch.float32, H, window, sink, weights)[0], portions, h)
+    for g, a, w in zip(got, absorbed, want):
+        err, other = float((g - w).norm() / w.norm()), float((a - w).norm() / w.norm())
+        # Both forms round three tensors to bfloat16 on the way (2^-9 each at most, at random); neither may lose against the other.
+        assert err < 3 * 2.0 ** -8 and err < 1.25 * other + 1e-4, (err, other)
+        assert float((g - w).abs().max()) < 0.06 * float(w.abs().max())
+
+
+def test_few_queries_per_key_keep_the_absorbed_form():
+    gen = torch.Generator().manual_seed(1)
+    part, weights = _part(torch.bfloat16, 2, None, False)
+    h = [torch.randn(310, D, generator=gen).to(torch.bfloat16).to(DEV)]
+    got, routes = _run(part, [(300,), (9,), (1,)], h)
+    assert routes == [1, 0, 0]
+    want, _ = _run(_part(torch.float32, 2, None, False, weights)[0], [(310,)], h)
+    assert float((got[0] - want[0]).norm() / want[0].norm()) < 3 * 2.0 ** -8
