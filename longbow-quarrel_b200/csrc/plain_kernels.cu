@@ -725,68 +725,152 @@ LQ_EXPORT int lq_rmsnorm_add(const float* y, const float* gain, float* x, const 
 // ------------------------------------------------------------------ linear (FFMA)
 // C[M,N] = A[M,K] . W[N,K]^T (+ residual[M,N]).  Each output is one chain of fused
 // multiply-adds over k = 0..K-1 in rising order, whatever M is.
-constexpr int GT = 64;   // tile of C
-constexpr int GK = 16;   // k step
+// Tiles of BM x BN outputs, TM x TN a thread; steps of GK of K in two buffers of shared memory, the next step's numbers on their
+// way into registers while the present one is multiplied, four k of a row a load; two neighbouring outputs share a packed
+// multiply-add (each of its halves rounds as a plain one does, so an output's chain is the same in every tile).  Bound by the
+// reads of shared memory, and below a few tiles a multiprocessor by the steps' latency.  Float32, rows x outputs x K, us (one
+// buffer, one load a number, one tile size before): 600 x 768 x 512 29 (58), 300 x 512 x 1536 68 (158), 64 x 512 x 512 14 (53), 8 x 768
+// x 512 13 (53), 16 x 2048 x 2048 48 (209).
+constexpr int G_THREADS = 256;
+typedef unsigned long long f32x2;       // two float32 side by side
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpair2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
 
-template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256)
+template <typename T> __device__ __forceinline__ float4 load4(const T* p);
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+
+template <typename TA, typename TW, typename TC, int BM, int BN, int TM, int TN, int GK>
+__global__ void __launch_bounds__(G_THREADS)
 gemm_plain_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C,
-                  const float* __restrict__ residual, int M, int N, int K) {
+                  const float* __restrict__ residual, int M, int N, int K, int whole) {
     pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float As[GK][GT + 1];
-    __shared__ float Ws[GK][GT + 1];
-    int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int i = threadIdx.x; i < GT * GK; i += 256) {
-            int r = i / GK, c = i % GK;
-            int gm = m0 + r, gn = n0 + r, gk = k0 + c;
-            As[c][r] = (gm < M && gk < K) ? to_f32(A[(size_t)gm * K + gk]) : 0.f;
-            Ws[c][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * K + gk]) : 0.f;
+    static_assert((BM / TM) * (BN / TN) == G_THREADS && TN % 2 == 0, "a thread per tile of outputs, taken in pairs");
+    constexpr int LA = BM + 4, LW = BN + 4, AQ = BM * GK / 4, WQ = BN * GK / 4;      // groups of four k in a step's rows
+    constexpr int NA = (AQ + G_THREADS - 1) / G_THREADS, NW = (WQ + G_THREADS - 1) / G_THREADS;
+    __shared__ __align__(16) float As[2][GK][LA];
+    __shared__ __align__(16) float Ws[2][GK][LW];
+    const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float4 ra[NA], rw[NW];
+    // Four k of one row; `whole`: rows start on a vector's boundary and K is a multiple of four.
+    auto four = [&](const auto* base, int row, int rows, int k) {
+        if (row >= rows || k >= K) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const auto* p = base + (size_t)row * K + k;
+        if (whole) return load4(p);
+        return make_float4(to_f32(p[0]), k + 1 < K ? to_f32(p[1]) : 0.f, k + 2 < K ? to_f32(p[2]) : 0.f, k + 3 < K ? to_f32(p[3]) : 0.f);
+    };
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int j = tid + i * G_THREADS;
+            if (j < AQ) ra[i] = four(A, m0 + j / (GK / 4), M, k0 + j % (GK / 4) * 4);
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            const int j = tid + i * G_THREADS;
+            if (j < WQ) rw[i] = four(W, n0 + j / (GK / 4), N, k0 + j % (GK / 4) * 4);
+        }
+    };
+    auto stage = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int j = tid + i * G_THREADS, r = j / (GK / 4), c = j % (GK / 4) * 4;
+            if (j < AQ) { As[buf][c][r] = ra[i].x; As[buf][c + 1][r] = ra[i].y; As[buf][c + 2][r] = ra[i].z; As[buf][c + 3][r] = ra[i].w; }
+        }
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            const int j = tid + i * G_THREADS, r = j / (GK / 4), c = j % (GK / 4) * 4;
+            if (j < WQ) { Ws[buf][c][r] = rw[i].x; Ws[buf][c + 1][r] = rw[i].y; Ws[buf][c + 2][r] = rw[i].z; Ws[buf][c + 3][r] = rw[i].w; }
+        }
+    };
+    f32x2 acc[TM][TN / 2];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
+    pdl_wait();
+    fetch(0);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += GK, buf ^= 1) {
+        const bool more = k0 + GK < K;
+        if (more) fetch(k0 + GK);
 #pragma unroll
         for (int kk = 0; kk < GK; ++kk) {
-            float a[4], w[4];
+            float x[TM];
+            f32x2 w[TN / 2];
+            if constexpr (TM % 4 == 0) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+                for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(x + i) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM + i]);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tx * 4 + j];
+                for (int i = 0; i < TM; ++i) x[i] = As[buf][kk][ty * TM + i];
+            }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < TN / 2; ++j) w[j] = *reinterpret_cast<const f32x2*>(&Ws[buf][kk][tx * TN + 2 * j]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+            for (int i = 0; i < TM; ++i) {
+                const f32x2 xx = pair2(x[i], x[i]);
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(xx, w[j], acc[i][j]);
+            }
         }
+        if (more) stage(buf ^ 1);
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int gm = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + ty * TM + i;
         if (gm >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int gn = n0 + tx * 4 + j;
+        for (int j = 0; j < TN; ++j) {
+            const int gn = n0 + tx * TN + j;
             if (gn >= N) continue;
-            float v = acc[i][j];
+            const float2 both = unpair2(acc[i][j / 2]);
+            float v = j & 1 ? both.y : both.x;
             if (residual) v += residual[(size_t)gm * N + gn];
             C[(size_t)gm * N + gn] = from_f32<TC>(v);
         }
     }
 }
 
+template <typename TA, typename TW, typename TC>
+static int gemm_plain_go(const TA* A, const TW* W, TC* C, const float* residual, int M, int N, int K, cudaStream_t stream) {
+    const int whole = K % 4 == 0 && (uintptr_t)A % (4 * sizeof(TA)) == 0 && (uintptr_t)W % (4 * sizeof(TW)) == 0;
+    auto go = [&](auto kernel, int bm, int bn) {
+        return launch_pdl(kernel, dim3((N + bn - 1) / bn, (M + bm - 1) / bm), dim3(G_THREADS), 0, stream, A, W, C, residual, M, N, K, whole);
+    };
+    // Few rows: tiles of 16 rows and 32 outputs, half as many steps.  Tiles of 64 x 64 read shared memory half as often as those of
+    // 32 x 32, which win where there are so few of them that latency is all (64 x 512 x 512: 14 us against 24; 600 x 512 x 512: 43 and 25).
+    if (M <= 16) return go(gemm_plain_kernel<TA, TW, TC, 16, 32, 1, 2, 32>, 16, 32);
+    if ((long long)((N + 63) / 64) * ((M + 63) / 64) <= 32) return go(gemm_plain_kernel<TA, TW, TC, 32, 32, 2, 2, 16>, 32, 32);
+    return go(gemm_plain_kernel<TA, TW, TC, 64, 64, 4, 4, 16>, 64, 64);
+}
+
 template <typename TA, typename TW>
 static int gemm_plain_c(const void* A, const void* W, void* C, int c_dtype, const float* residual,
                         int M, int N, int K, cudaStream_t stream) {
-    dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
-    if (c_dtype == LQ_F32)
-        return launch_pdl(gemm_plain_kernel<TA, TW, float>, grid, dim3(256), 0, stream, (const TA*)A, (const TW*)W, (float*)C, residual, M, N, K);
-    else if (c_dtype == LQ_BF16)
-        return launch_pdl(gemm_plain_kernel<TA, TW, __nv_bfloat16>, grid, dim3(256), 0, stream, (const TA*)A, (const TW*)W, (__nv_bfloat16*)C, residual, M, N, K);
-    else
-        return LQ_BAD_DTYPE;
-    return lq_launch_status();
+    if (c_dtype == LQ_F32) return gemm_plain_go((const TA*)A, (const TW*)W, (float*)C, residual, M, N, K, stream);
+    if (c_dtype == LQ_BF16) return gemm_plain_go((const TA*)A, (const TW*)W, (__nv_bfloat16*)C, residual, M, N, K, stream);
+    return LQ_BAD_DTYPE;
 }
 
 LQ_EXPORT int lq_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype,
@@ -1330,6 +1414,8 @@ LQ_EXPORT int lq_softcap(float* x, long long total, float cap, cudaStream_t stre
 // same order.  cap > 0: score <- cap * tanh(score / cap) after the scale.  keep_first: with a window, the first
 // keep_first positions of the sequence stay visible (at their own positions) when the window has moved past them.
 // slope (or null): [H], score <- score - slope[h] * (position - key), after the cap.
+// Bound by the latency of the chunk's chains (every sum in order): keys four numbers a load and values sixteen loads at a time,
+// each key's place worked out once, take 600 rows of 8 heads of 64 in float32 from 238 us to 84, with the same bits.
 constexpr int ATT_CHUNK = 128;
 
 template <typename T, typename TG>
@@ -1346,7 +1432,8 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
     extern __shared__ float sm[];
     float* qs = sm;              // [hd]
     float* sc = sm + hd;         // [ATT_CHUNK]
-    int* pg = (int*)(sc + ATT_CHUNK);  // [ATT_CHUNK] page of each key of the chunk
+    int* at = (int*)(sc + ATT_CHUNK);  // [ATT_CHUNK] where each key of the chunk lies, in rows of the pages
+    const bool vec = hd % 4 == 0 && (uintptr_t)k_pages % (4 * sizeof(T)) == 0;
     int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     int pos = tok_pos[t];
     int slot = slots[tok_seq[t]];
@@ -1365,11 +1452,22 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
         float s = -CUDART_INF_F;
         if (tid < n) {
             int key = vbase + tid < head ? vbase + tid : start + (vbase + tid - head);
-            int page = pt[key / page_size];
-            pg[tid] = page;
-            const T* kr = k_pages + (((size_t)page * Hkv + kvh) * page_size + key % page_size) * hd;
+            const int row = (pt[key / page_size] * Hkv + kvh) * page_size + key % page_size;
+            at[tid] = row;
+            const T* kr = k_pages + (size_t)row * hd;
             float d = 0.f;
-            for (int i = 0; i < hd; ++i) d = fmaf(qs[i], to_f32(kr[i]), d);
+            if (vec) {
+#pragma unroll 8
+                for (int i = 0; i < hd; i += 4) {
+                    const float4 k4 = load4(kr + i);
+                    d = fmaf(qs[i], k4.x, d);
+                    d = fmaf(qs[i + 1], k4.y, d);
+                    d = fmaf(qs[i + 2], k4.z, d);
+                    d = fmaf(qs[i + 3], k4.w, d);
+                }
+            } else {
+                for (int i = 0; i < hd; ++i) d = fmaf(qs[i], to_f32(kr[i]), d);
+            }
             s = d * scale;
             if (cap > 0.f) s = cap * tanhf(s / cap);
             if (slope) s = fmaf(-slope[h], (float)(pos - key), s);
@@ -1377,23 +1475,22 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
         sc[tid] = s;
         __syncthreads();
         float cm = m;
+#pragma unroll 8
         for (int j = 0; j < n; ++j) cm = fmaxf(cm, sc[j]);
         float corr = expf(m - cm);  // m = -inf at the first chunk gives 0
         __syncthreads();
         if (tid < n) sc[tid] = expf(sc[tid] - cm);
         __syncthreads();
         float ls = 0.f;
+#pragma unroll 8
         for (int j = 0; j < n; ++j) ls += sc[j];
         l = l * corr + ls;
         for (int rep = 0; rep < 2; ++rep) {
             int d = tid + rep * ATT_CHUNK;
             if (d >= vd) break;
             float a = 0.f;
-            for (int j = 0; j < n; ++j) {
-                int key = vbase + j < head ? vbase + j : start + (vbase + j - head);
-                const T* vr = v_pages + (((size_t)pg[j] * Hkv + kvh) * page_size + key % page_size) * vd;
-                a = fmaf(sc[j], to_f32(vr[d]), a);
-            }
+#pragma unroll 16
+            for (int j = 0; j < n; ++j) a = fmaf(sc[j], to_f32(v_pages[(size_t)at[j] * vd + d]), a);
             if (rep == 0) acc0 = acc0 * corr + a; else acc1 = acc1 * corr + a;
         }
         m = cm;

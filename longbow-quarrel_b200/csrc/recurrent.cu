@@ -572,9 +572,97 @@ __global__ void __launch_bounds__(256) small_proj_kernel(const TX* __restrict__ 
     }
 }
 
+// The same for bfloat16 rows and weights: a warp takes R rows and J outputs, a lane eight neighbouring k of every 256, sixteen bytes
+// of a row or an output's weights at a time, in packed multiply-adds.  An output's four sums a lane (pairs of k by turns), their
+// total and the order across the lanes depend on K alone, so a row's result is the same whatever rows and outputs share its
+// warp.  (As products of the tensor cores, exact as they are there, the sums' error grew by a third to a half: not kept.)  Bound
+// by the multiply-adds and the unpacking.
+__device__ __forceinline__ unsigned long long sp_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long sp_pair(uint32_t v) {      // two bfloat16 as two float32
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(v << 16), "r"(v & 0xffff0000u));
+    return d;
+}
+constexpr int SPB_WARPS = 4;
+template <int R, int J>
+__global__ void __launch_bounds__(SPB_WARPS * 32) small_proj_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                          float* __restrict__ out, int rows, int N, int K) {
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, t0 = blockIdx.x * R, n0 = (blockIdx.y * SPB_WARPS + (threadIdx.x >> 5)) * J;
+    pdl_wait();
+    if (n0 >= N) return;
+    const uint4* xr[R];
+    const uint4* wr[J];
+#pragma unroll
+    for (int r = 0; r < R; ++r) xr[r] = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + r, rows - 1) * K);
+#pragma unroll
+    for (int j = 0; j < J; ++j) wr[j] = reinterpret_cast<const uint4*>(w + (size_t)min(n0 + j, N - 1) * K);
+    unsigned long long acc[R][J][2];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < J; ++j) acc[r][j][0] = acc[r][j][1] = 0;
+    uint4 wv[J], xv[R];
+    auto fetch = [&](int k) {
+        if (k >= K / 8) return;
+#pragma unroll
+        for (int j = 0; j < J; ++j) wv[j] = wr[j][k];
+#pragma unroll
+        for (int r = 0; r < R; ++r) xv[r] = xr[r][k];
+    };
+    fetch(lane);
+#pragma unroll 1
+    for (int k = lane; k < K / 8; k += 32) {
+        unsigned long long wf[J][4], xf[R][4];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            wf[j][0] = sp_pair(wv[j].x); wf[j][1] = sp_pair(wv[j].y); wf[j][2] = sp_pair(wv[j].z); wf[j][3] = sp_pair(wv[j].w);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            xf[r][0] = sp_pair(xv[r].x); xf[r][1] = sp_pair(xv[r].y); xf[r][2] = sp_pair(xv[r].z); xf[r][3] = sp_pair(xv[r].w);
+        }
+        fetch(k + 32);                           // on its way while these are multiplied
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int j = 0; j < J; ++j) acc[r][j][e & 1] = sp_fma2(xf[r][e], wf[j][e], acc[r][j][e & 1]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            float2 a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(acc[r][j][0]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(b.x), "=f"(b.y) : "l"(acc[r][j][1]));
+            const float v = warp_sum((a.x + a.y) + (b.x + b.y));
+            if (lane == 0 && t0 + r < rows && n0 + j < N) out[(size_t)(t0 + r) * N + n0 + j] = v;
+        }
+}
+
+static int small_proj_bf16(const __nv_bfloat16* x, const __nv_bfloat16* w, float* out, int rows, int N, int K, cudaStream_t stream) {
+    auto go = [&](auto kernel, int r, int j) {
+        const int per = j * SPB_WARPS;
+        return launch_pdl(kernel, dim3((rows + r - 1) / r, (N + per - 1) / per), dim3(SPB_WARPS * 32), 0, stream, x, w, out, rows, N, K);
+    };
+    // Few rows: as many warps as possible; many: as many products from every number that is read and unpacked.
+    if (rows <= 2) return go(small_proj_bf16_kernel<2, 1>, 2, 1);
+    if ((long long)((rows + 3) / 4) * ((N + 3) / 4) < 148 * 4) return go(small_proj_bf16_kernel<4, 1>, 4, 1);
+    return go(small_proj_bf16_kernel<4, 4>, 4, 4);
+}
+
 LQ_EXPORT int lq_small_proj(const void* x, int x_dtype, const void* w, int w_dtype, float* out, int rows, int N, int K,
                             cudaStream_t stream) {
     if (rows <= 0 || N <= 0) return LQ_OK;
+    // Rows on 16-byte boundaries, whatever their number: a row's result must not depend on it.
+    if (x_dtype == LQ_BF16 && w_dtype == LQ_BF16 && K % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0)
+        return small_proj_bf16((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, rows, N, K, stream);
     const size_t smem = (size_t)SP_ROWS * K * sizeof(float);
     if (smem > 200 * 1024) return LQ_BAD_SIZE;
     auto go = [&](auto kernel, auto xp, auto wp) {

@@ -1,0 +1,50 @@
+"""The 32-bit products: the tiled one (csrc/plain_kernels.cu) in its three tile sizes, and the projection of bfloat16 rows onto few
+outputs (csrc/recurrent.cu), at the edges of their tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _ops():
+    from longbow_quarrel_b200.kernels import ops
+    return ops
+
+
+def _rand(shape, seed, dtype):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(dtype)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 31, 15), (16, 33, 64), (17, 65, 17), (33, 64, 16), (130, 1100, 20), (700, 531, 7)])
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+def test_the_tiled_product_sums_in_one_order_whatever_the_tile(M, N, K, ta, tw):
+    ops = _ops()
+    a, w, r = _rand((M, K), M, ta), _rand((N, K), N, tw), _rand((M, N), K, torch.float32)
+    want = a.double() @ w.double().T
+    got = ops.gemm_plain(a.to(DEV), w.to(DEV), torch.float32)
+    # K additions of 2^-24 each at most, on sums no larger than the sum of the products' sizes
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((got.cpu().double() - want).abs() <= bound).all())
+    alone = ops.gemm_plain(a[:1].contiguous().to(DEV), w.to(DEV), torch.float32)             # a row by itself: the tiles of 16 rows
+    some = ops.gemm_plain(a[:20].contiguous().to(DEV), w[:30].contiguous().to(DEV), torch.float32)     # 32 x 32
+    assert torch.equal(alone[0], got[0]) and torch.equal(some, got[:20, :30])
+    added = ops.gemm_plain(a.to(DEV), w.to(DEV), torch.float32, residual=r.to(DEV).clone())
+    assert torch.equal(added.cpu(), got.cpu() + r)
+    shifted = torch.zeros(M * K + 1, dtype=ta, device=DEV)[1:].view(M, K)                    # rows off a vector's boundary
+    shifted.copy_(a.to(DEV))
+    assert torch.equal(ops.gemm_plain(shifted, w.to(DEV), torch.float32), got)
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 1, 8), (2, 65, 2048), (17, 9, 104), (300, 64, 4096), (2500, 65, 520), (40, 130, 288)])
+def test_a_projection_of_bfloat16_onto_few_outputs(rows, N, K):
+    ops = _ops()
+    x, w = _rand((rows, K), rows, torch.bfloat16), _rand((N, K), N, torch.bfloat16)
+    got = ops.small_proj(x.to(DEV), w.to(DEV))
+    want = x.double() @ w.double().T
+    # Exact products in chains of K / 128 + 2 multiply-adds at most, then seven additions, each rounding by 2^-24.
+    bound = (K / 128 + 9) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.cpu().double() - want).abs() <= bound).all())
+    # A row's result does not depend on the rows beside it, nor on how many outputs a warp makes.
+    assert torch.equal(ops.small_proj(x[-1:].contiguous().to(DEV), w.to(DEV))[0], got[-1])
+    assert torch.equal(ops.small_proj(x.to(DEV), w[:1].contiguous().to(DEV))[:, 0], got[:, 0])
