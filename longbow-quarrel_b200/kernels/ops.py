@@ -848,14 +848,15 @@ def group_rows_padded(ids: torch.Tensor, G: int) -> tuple:
     return src, dst, tile_group
 
 
-def gather_rows(a: torch.Tensor, src: torch.Tensor, div: int = 1) -> torch.Tensor:
-    """out[p] = a[src[p] // div] (zeros where src[p] < 0); rows of a multiple of 16 bytes."""
+def gather_rows(a: torch.Tensor, src: torch.Tensor, div: int = 1, tile_group: torch.Tensor | None = None) -> torch.Tensor:
+    """out[p] = a[src[p] // div] (zeros where src[p] < 0); rows of a multiple of 16 bytes.  tile_group (of group_rows_padded): the
+    rows of tiles without a group are not written."""
     row_bytes = a.shape[1] * a.element_size()
     if not a.is_contiguous() or row_bytes % 16:
         raise KernelError("gather_rows: contiguous rows of a multiple of 16 bytes")
     out = torch.empty((src.numel(), a.shape[1]), dtype=a.dtype, device=a.device)
-    fn = _fn("grouped_gemm", "lq_gather_rows", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
-    _check(fn(_p(a), _p(src), div, _p(out), src.numel(), row_bytes, _stream()), "gather_rows")
+    fn = _fn("grouped_gemm", "lq_gather_rows", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p])
+    _check(fn(_p(a), _p(src), div, _p(out), src.numel(), row_bytes, _p(tile_group), GROUP_TILE, _stream()), "gather_rows")
     return out
 
 

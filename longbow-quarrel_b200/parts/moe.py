@@ -139,7 +139,7 @@ class RoutedExperts(FeedForward):
             # tile of the tcgen05 product reads one expert's weight; the second product reads the first one's rows as
             # they lie, and the combination finds each pair's row through the order's inverse.
             src, dst, tile_group = ops.group_rows_padded(ids.view(-1), self.E)
-            u = ops.gemm_tc_grouped(ops.gather_rows(h, src, self.top), self.w_up, tile_group, h.dtype,
+            u = ops.gemm_tc_grouped(ops.gather_rows(h, src, self.top, tile_group), self.w_up, tile_group, h.dtype,
                                     swiglu=self.gated and self.up_block > 0)     # silu(gate) * up in the product's epilogue
             if self.gated and not self.up_block:
                 u = ops.gated_act(u, None, self.activation, h.dtype)     # [rows, 2F] -> act(gate columns) * up columns

@@ -1,0 +1,60 @@
+"""What surrounds the experts' products of a prompt: the pairs' order by groups, the rows' gather, their combination."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _ops():
+    from longbow_quarrel_b200.kernels import ops
+
+    return ops
+
+
+@pytest.mark.parametrize("n,G", [(1, 1), (128, 1), (129, 2), (1023, 31), (1025, 33), (6000, 64), (4096, 1000)])
+def test_every_index_has_one_place_in_a_tile_of_its_group(n, G):
+    """Around one warp's sum of the groups' tiles (32 at a time) and the 1024 threads; empty groups first, between and last; ids at
+    G and above have no place."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(n + G)
+    used = torch.randperm(G, generator=g)[:max(1, G * 2 // 3)]
+    ids = used[torch.randint(0, len(used), (n,), generator=g)].to(torch.int32)
+    if n > 1000:
+        ids[::7] = G + 3
+    src, dst, tile_group = (t.cpu().long() for t in ops.group_rows_padded(ids.to(DEV), G))
+    flat = ids.long()
+    placed = flat < G
+    assert (dst[~placed] == -1).all() and (src[dst[placed]] == torch.arange(n)[placed]).all()
+    assert int((src >= 0).sum()) == int(placed.sum())
+    tiles = (torch.bincount(flat[placed], minlength=G) + 127) // 128
+    want = torch.cat([torch.repeat_interleave(torch.arange(G), tiles), torch.full((len(tile_group) - int(tiles.sum()),), -1)])
+    assert (tile_group == want).all() and (tile_group[dst[placed] // 128] == flat[placed]).all()
+    h = torch.randn(n, 8, generator=g).to(torch.bfloat16)
+    rows = ops.gather_rows(h.to(DEV), src.to(torch.int32).to(DEV), 1, tile_group.to(torch.int32).to(DEV)).cpu()
+    inside = torch.repeat_interleave(tile_group >= 0, 128)
+    assert torch.equal(rows[inside], torch.where((src >= 0)[:, None], h[src.clamp(min=0)], 0.0)[inside])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("T,top,D,identity", [(3, 1, 4, False), (17, 6, 104, True), (5, 8, 1028, False), (2, 64, 256, True), (2, 65, 256, False)])
+def test_the_combination_of_four_columns_at_a_time_is_that_of_one(T, top, D, identity, accumulate):
+    """The same products in the same order: rows that do not start on 16 bytes take the other kernel, with the same bits."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(T + D)
+    y = torch.randn(T * top, D, generator=g).to(DEV)
+    h = torch.randn(T, D, generator=g).to(torch.bfloat16).to(DEV)
+    weights = torch.rand(T, top, generator=g).to(DEV)
+    shared, z = torch.randn(T, D, generator=g).to(DEV), torch.randn(T, 3, generator=g).to(DEV)
+    place = torch.randperm(T * top, generator=g).to(torch.int32).to(DEV)
+    ids = torch.randint(0, 9, (T, top), generator=g).to(torch.int32).to(DEV)
+    more = dict(ids=ids, E=7, h=h) if identity else {}
+    x = torch.randn(T, D, generator=g).to(DEV)
+    off = torch.empty(T * D + 1, device=DEV)[1:].view(T, D).copy_(x)
+    for into in (x, off):
+        ops.moe_combine(y, weights, into, accumulate, shared=shared, shared_gate=z[:, 2], place=place, shared_scale=0.5, **more)
+    assert torch.equal(x, off)
+    ops.check_status()
