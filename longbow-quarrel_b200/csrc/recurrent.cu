@@ -463,6 +463,105 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(const float* __rest
     }
 }
 
+// The same with everything a head needs asked for at once and held in registers.  VEC 4: LPH lanes a head, NV times four
+// neighbouring values each (whole fours on 16-byte boundaries, no denominator); VEC 1: a warp a head, values lane, lane + 32, ...
+// (with a denominator a row of raw starts anywhere), the sums in the order of the kernel above.  Bound by the bytes: 2,048
+// rows of 32 heads of 64, bfloat16: 22 us one value a load in two passes, 12 here; 3,075 rows of 32 heads of 128 with a denominator
+// 31 and 27.
+template <typename T, int LPH, int NV, int VEC>
+__global__ void __launch_bounds__(128) head_norm_gate_held_kernel(const float* __restrict__ raw, int dvx, const float* __restrict__ exp_neg_m,
+                                                                  const float* __restrict__ weight, const T* __restrict__ gate,
+                                                                  int gate_stride, int act, T* __restrict__ out, int n_pairs,
+                                                                  int H, int dv, float eps) {
+    pdl_launch_dependents();
+    const int own = blockIdx.x * (128 / LPH) + threadIdx.x / LPH, l = threadIdx.x % LPH, pair = min(own, n_pairs - 1);
+    const int row = pair / H, h = pair % H;
+    pdl_wait();
+    const float* r = raw + (size_t)pair * dvx;
+    const T* gr = gate ? gate + (size_t)row * gate_stride + h * dv : nullptr;
+    alignas(16) float v[NV][VEC], g[NV][VEC], w[NV][VEC];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (l + i * LPH) * VEC;
+        const bool in = d < dv;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) { v[i][e] = 0.f; g[i][e] = 0.f; w[i][e] = 1.f; }
+        if (!in) continue;
+        if constexpr (VEC == 4) {
+            *reinterpret_cast<float4*>(v[i]) = *reinterpret_cast<const float4*>(r + d);
+            if (weight) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(weight + h * dv + d);
+            if (act) {
+                if constexpr (sizeof(T) == 4) {
+                    *reinterpret_cast<float4*>(g[i]) = *reinterpret_cast<const float4*>(gr + d);
+                } else {
+                    const uint2 b = *reinterpret_cast<const uint2*>(gr + d);
+                    g[i][0] = __uint_as_float(b.x << 16); g[i][1] = __uint_as_float(b.x & 0xffff0000u);
+                    g[i][2] = __uint_as_float(b.y << 16); g[i][3] = __uint_as_float(b.y & 0xffff0000u);
+                }
+            }
+        } else {
+            v[i][0] = r[d];
+            if (weight) w[i][0] = weight[h * dv + d];
+            if (act) g[i][0] = to_f32(gr[d]);
+        }
+    }
+    float inv = 1.f;
+    if (exp_neg_m) inv = 1.f / (fmaxf(fabsf(r[dv]), exp_neg_m[pair]) + 1e-6f);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            const float x = v[i][e] * inv;
+            s = fmaf(x, x, s);
+        }
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (own >= n_pairs) return;
+    const float scale = inv / sqrtf(s / (float)dv + eps);
+    T* o = out + (size_t)pair * dv;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (l + i * LPH) * VEC;
+        if (d >= dv) continue;
+        alignas(16) T y[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            float x = v[i][e] * scale;
+            if (weight) x *= w[i][e];
+            if (act) {
+                const float sg = 1.f / (1.f + expf(-g[i][e]));
+                x *= act == 1 ? sg : g[i][e] * sg;
+            }
+            y[e] = from_f32<T>(x);
+        }
+        if constexpr (VEC == 4 && sizeof(T) == 4) *reinterpret_cast<uint4*>(o + d) = *reinterpret_cast<const uint4*>(y);
+        else if constexpr (VEC == 4) *reinterpret_cast<uint2*>(o + d) = *reinterpret_cast<const uint2*>(y);
+        else o[d] = y[0];
+    }
+}
+
+template <typename T>
+static int head_norm_gate_held(const float* raw, int dvx, const float* exp_neg_m, const float* weight, const void* gate, int gate_stride,
+                               int act, void* out, int n, int H, int dv, float eps, cudaStream_t stream) {
+    auto go = [&](auto kernel, int lanes) {
+        const int per = 128 / lanes;
+        return launch_pdl(kernel, dim3((n + per - 1) / per), dim3(128), 0, stream, raw, dvx, exp_neg_m, weight, (const T*)gate, gate_stride, act,
+                          (T*)out, n, H, dv, eps);
+    };
+    const bool fours = !exp_neg_m && dv % 4 == 0 && dvx == dv && (uintptr_t)raw % 16 == 0 && (uintptr_t)weight % 16 == 0 &&
+                       (uintptr_t)out % (4 * sizeof(T)) == 0 && (!act || (gate_stride % 4 == 0 && (uintptr_t)gate % (4 * sizeof(T)) == 0));
+    if (fours && dv <= 32) return go(head_norm_gate_held_kernel<T, 8, 1, 4>, 8);
+    if (fours && dv <= 64) return go(head_norm_gate_held_kernel<T, 16, 1, 4>, 16);
+    if (fours && dv <= 128) return go(head_norm_gate_held_kernel<T, 32, 1, 4>, 32);
+    if (fours && dv <= 256) return go(head_norm_gate_held_kernel<T, 32, 2, 4>, 32);
+    if (dv <= 64) return go(head_norm_gate_held_kernel<T, 32, 2, 1>, 32);
+    if (dv <= 128) return go(head_norm_gate_held_kernel<T, 32, 4, 1>, 32);
+    if (dv <= 256) return go(head_norm_gate_held_kernel<T, 32, 8, 1>, 32);
+    return launch_pdl(head_norm_gate_kernel<T>, dim3((n + 3) / 4), dim3(128), 0, stream, raw, dvx, exp_neg_m, weight, (const T*)gate, gate_stride,
+                      act, (T*)out, n, H, dv, eps);
+}
+
 // The same for heads of many values (all heads normed together count as one head): a block per (row, head).
 template <typename T>
 __global__ void __launch_bounds__(256) head_norm_gate_wide_kernel(const float* __restrict__ raw, int dvx,
@@ -517,13 +616,8 @@ LQ_EXPORT int lq_head_norm_gate(const float* raw, int dvx, const float* exp_neg_
                               (const __nv_bfloat16*)gate, gate_stride, act, (__nv_bfloat16*)out, H, dv, eps);
         return LQ_BAD_DTYPE;
     }
-    dim3 grid((n + 3) / 4);
-    if (dtype == LQ_F32)
-        return launch_pdl(head_norm_gate_kernel<float>, grid, dim3(128), 0, stream, raw, dvx, exp_neg_m, weight,
-                          (const float*)gate, gate_stride, act, (float*)out, n, H, dv, eps);
-    if (dtype == LQ_BF16)
-        return launch_pdl(head_norm_gate_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, raw, dvx, exp_neg_m, weight,
-                          (const __nv_bfloat16*)gate, gate_stride, act, (__nv_bfloat16*)out, n, H, dv, eps);
+    if (dtype == LQ_F32) return head_norm_gate_held<float>(raw, dvx, exp_neg_m, weight, gate, gate_stride, act, out, n, H, dv, eps, stream);
+    if (dtype == LQ_BF16) return head_norm_gate_held<__nv_bfloat16>(raw, dvx, exp_neg_m, weight, gate, gate_stride, act, out, n, H, dv, eps, stream);
     return LQ_BAD_DTYPE;
 }
 
