@@ -48,7 +48,7 @@ from .spec import PartSpec
 class _MatrixStateMixer(Mixer):
     graph_safe = True
     returns_branch = True
-    kernel_libraries = ("recurrent", "chunk_scan")
+    kernel_libraries = ("recurrent",)
 
     def __init__(self, runtime: Runtime, hidden_size: int, n_heads: int, key_dim: int, value_dim: int, eps: float,
                  names: dict | None = None):
