@@ -58,6 +58,18 @@ struct Glu {
     }
 };
 
+// What an expert's first product passes through (ungated).  act: 0 none, 1 gelu (erf), 2 gelu (tanh form), 3 silu, 4 relu, 5 the square of relu
+__device__ __forceinline__ float lq_expert_act(float v, int act) {
+    switch (act) {
+        case 1: return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
+        case 2: return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+        case 3: return v / (1.f + expf(-v));
+        case 4: return fmaxf(v, 0.f);
+        case 5: { const float r = fmaxf(v, 0.f); return r * r; }
+        default: return v;
+    }
+}
+
 // ------------------------------------------------------------------ programmatic dependent launch
 // Kernels of a step follow one another on one stream.  Launched with launch_pdl, a kernel's
 // blocks may be scheduled while the kernel before it is still draining; they run up to

@@ -12,6 +12,7 @@
 #define EPI_RESID 2
 #define EPI_SWIGLU 3
 #define EPI_QKV 4       // q, k, v rows: rotate q and k, store k and v into the cache pages
+#define EPI_ACT 5       // bfloat16 behind an activation of the float32 sums (staged stores only)
 
 namespace tc {
 
@@ -30,7 +31,7 @@ __device__ __forceinline__ uint4* staged_at(uint8_t* buf, int row, int piece) {
 // Accumulator columns that fill a buffer's 128 bytes per row: 32 floats, 64 bfloat16, or 128 columns of
 // interleaved gate and up rows (64 outputs).
 template <int EPI> struct StagedCols {
-    static constexpr int value = (EPI == EPI_F32 || EPI == EPI_RESID) ? 32 : (EPI == EPI_BF16 ? 64 : 128);
+    static constexpr int value = (EPI == EPI_F32 || EPI == EPI_RESID) ? 32 : (EPI == EPI_BF16 || EPI == EPI_ACT ? 64 : 128);
 };
 
 // Columns [0, bn) of this warp's 32 lanes of the accumulator at `taddr` go to rows y .. y + 31 of the output
@@ -39,7 +40,7 @@ template <int EPI> struct StagedCols {
 // next and is kept across calls, as are the stores in flight (wait for them with bulk_wait<0> at the end).
 template <int EPI>
 __device__ __forceinline__ void staged_epilogue(uint32_t taddr, int bn, uint8_t* bufs, int& which, const CUtensorMap* map_c,
-                                                int y, int n0, int N, int lane, float glu_limit) {
+                                                int y, int n0, int N, int lane, float glu_limit, int act = 0) {
     const Glu glu(glu_limit);
     constexpr int COLS = StagedCols<EPI>::value;
 #pragma unroll 1
@@ -56,7 +57,20 @@ __device__ __forceinline__ void staged_epilogue(uint32_t taddr, int bn, uint8_t*
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     *staged_at(buf, lane, i) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-            } else if (EPI == EPI_BF16) {
+            } else if (EPI == EPI_BF16 || EPI == EPI_ACT) {
+                if constexpr (EPI == EPI_ACT) {
+                    auto all = [&](auto f) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(f(__uint_as_float(r[i])));
+                    };
+                    switch (act) {
+                        case 1: all([](float v) { return lq_expert_act(v, 1); }); break;
+                        case 2: all([](float v) { return lq_expert_act(v, 2); }); break;
+                        case 3: all([](float v) { return lq_expert_act(v, 3); }); break;
+                        case 4: all([](float v) { return lq_expert_act(v, 4); }); break;
+                        default: all([](float v) { return lq_expert_act(v, 5); }); break;
+                    }
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     *staged_at(buf, lane, sub * 4 + i) =
@@ -104,6 +118,7 @@ struct QkvArgs {
     __nv_bfloat16* v_pages;
     int pt_stride, H, Hkv, hd, page_size;
     float glu_limit;          // EPI_SWIGLU: see Glu
+    int act;                  // EPI_ACT: see lq_expert_act
 };
 
 // Where elements j .. of head `head` of row m go: q_out, or the row's place in a cache page.

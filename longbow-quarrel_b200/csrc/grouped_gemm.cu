@@ -44,18 +44,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// act: 0 none, 1 gelu (erf), 2 gelu (tanh form), 3 silu, 4 relu, 5 the square of relu
-__device__ __forceinline__ float gg_act(float v, int act) {
-    switch (act) {
-        case 1: return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-        case 2: return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-        case 3: return v / (1.f + expf(-v));
-        case 4: return fmaxf(v, 0.f);
-        case 5: { const float r = fmaxf(v, 0.f); return r * r; }
-        default: return v;
-    }
-}
-
 struct GroupedArgs {
     const __nv_bfloat16* A;
     long long lda, a_group_stride;
@@ -170,8 +158,8 @@ __global__ void __launch_bounds__(BN) grouped_gemm_kernel(GroupedArgs a) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int n = n0 + wn * 64 + j * 8 + 2 * t;
-                if (n < N) o[n] = from_f32<TO>(gg_act(acc[i][j][2 * half], a.act));
-                if (n + 1 < N) o[n + 1] = from_f32<TO>(gg_act(acc[i][j][2 * half + 1], a.act));
+                if (n < N) o[n] = from_f32<TO>(lq_expert_act(acc[i][j][2 * half], a.act));
+                if (n + 1 < N) o[n + 1] = from_f32<TO>(lq_expert_act(acc[i][j][2 * half + 1], a.act));
             }
         }
 }

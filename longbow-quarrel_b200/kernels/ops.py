@@ -867,21 +867,24 @@ def gather_rows(a: torch.Tensor, src: torch.Tensor, div: int = 1, tile_group: to
 
 
 def gemm_tc_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, out_dtype: torch.dtype,
-                    swiglu: bool = False) -> torch.Tensor:
+                    swiglu: bool = False, act: str | None = None) -> torch.Tensor:
     """a [M, K] (M a multiple of 128, its row tiles each of one group) times w [G, N, K]: row tile i is multiplied with
     w[tile_group[i]] on the tcgen05 tensor cores (tiles with group -1 are left out and their rows of the result are not
     written).  Returns [M, N] in out_dtype (bfloat16 or float32).  swiglu: every group's rows are 8 gate rows and 8 up
-    rows by turns (`linear.interleave_gate_up`), and what comes back is silu(gate) * up, [M, N / 2] bfloat16."""
+    rows by turns (`linear.interleave_gate_up`), and what comes back is silu(gate) * up, [M, N / 2] bfloat16.  act: the float32
+    sums pass through one of MOE_ACTS ahead of their rounding to bfloat16 (N a multiple of 8)."""
     M, K = a.shape
     G, N, K2 = w.shape
     if swiglu and (N % 16 or out_dtype != torch.bfloat16):
         raise KernelError("gemm_tc_grouped: the gated form takes 16 rows of weight at a time and hands on bfloat16")
+    if act is not None and (swiglu or N % 8 or out_dtype != torch.bfloat16):
+        raise KernelError("gemm_tc_grouped: an activation comes with a plain bfloat16 output of whole eights")
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K2 != K or K % 8 or M % GROUP_TILE or not a.is_contiguous() \
             or not w.is_contiguous() or tile_group.numel() != M // GROUP_TILE:
         raise KernelError("gemm_tc_grouped: contiguous bfloat16 operands, K a multiple of 8, whole row tiles with a group each")
     out = torch.empty((M, N // 2 if swiglu else N), dtype=out_dtype, device=a.device)
     fn = _fn("gemm_tc", "lq_gemm_tc_grouped", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
-    _check(fn(_p(a), _p(w), _p(out), 2 if swiglu else int(out_dtype == torch.float32), M, N, K, G, _p(tile_group), _stream()),
+    _check(fn(_p(a), _p(w), _p(out), 2 if swiglu else 2 + MOE_ACTS[act] if act is not None else int(out_dtype == torch.float32), M, N, K, G, _p(tile_group), _stream()),
            "gemm_tc_grouped")
     return out
 

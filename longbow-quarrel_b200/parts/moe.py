@@ -140,11 +140,10 @@ class RoutedExperts(FeedForward):
             # they lie, and the combination finds each pair's row through the order's inverse.
             src, dst, tile_group = ops.group_rows_padded(ids.view(-1), self.E)
             u = ops.gemm_tc_grouped(ops.gather_rows(h, src, self.top, tile_group), self.w_up, tile_group, h.dtype,
-                                    swiglu=self.gated and self.up_block > 0)     # silu(gate) * up in the product's epilogue
+                                    swiglu=self.gated and self.up_block > 0,     # silu(gate) * up in the product's epilogue
+                                    act=None if self.gated else self.activation)
             if self.gated and not self.up_block:
                 u = ops.gated_act(u, None, self.activation, h.dtype)     # [rows, 2F] -> act(gate columns) * up columns
-            elif not self.gated and self.activation is not None:
-                ops.activation(u, self.activation, out=u)
             y = ops.gemm_tc_grouped(u, self.w_down, tile_group, torch.float32)
             out = residual if residual is not None else torch.empty((T, self.D), dtype=torch.float32, device=h.device)
             ops.moe_combine(y, weights, out, accumulate=residual is not None, shared=shared, shared_gate=gate, place=dst,

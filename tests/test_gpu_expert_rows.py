@@ -58,3 +58,24 @@ def test_the_combination_of_four_columns_at_a_time_is_that_of_one(T, top, D, ide
         ops.moe_combine(y, weights, into, accumulate, shared=shared, shared_gate=z[:, 2], place=place, shared_scale=0.5, **more)
     assert torch.equal(x, off)
     ops.check_status()
+
+
+@pytest.mark.parametrize("T,E,D,F", [(130, 3, 64, 8), (300, 5, 128, 264), (140, 2, 520, 136)])
+@pytest.mark.parametrize("act", ["gelu", "gelu_tanh", "silu", "relu", "relu2"])
+def test_a_grouped_product_behind_an_activation(act, T, E, D, F):
+    """The activation of the float32 sums ahead of their one rounding: the product's own float32 output, activated in 64 bits, at
+    widths of one vector, of a tile and one vector more, and of half a tile."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(T + F)
+    h = torch.randn(T, D, generator=g).to(torch.bfloat16).to(DEV)
+    w = (2 * torch.randn(E, F, D, generator=g) / D ** 0.5).to(torch.bfloat16).to(DEV)
+    ids = torch.randint(0, E, (T,), generator=g).to(torch.int32).to(DEV)
+    src, dst, tile_group = ops.group_rows_padded(ids, E)
+    rows = ops.gather_rows(h, src, 1, tile_group)
+    sums = ops.gemm_tc_grouped(rows, w, tile_group, torch.float32)[dst.long()].double()
+    got = ops.gemm_tc_grouped(rows, w, tile_group, torch.bfloat16, act=act)[dst.long()].double()
+    want = {"gelu": lambda v: 0.5 * v * (1 + torch.erf(v / 2 ** 0.5)), "silu": lambda v: v * torch.sigmoid(v), "relu": torch.relu,
+            "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh"), "relu2": lambda v: torch.relu(v) ** 2}[act](sums)
+    # half a unit of bfloat16, and a few float32 roundings of the factor (1 + erf or tanh), which cancels for negative sums
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 16 * 2.0 ** -24 * sums.abs()).all())
+    ops.check_status()
