@@ -29,16 +29,19 @@ def dtype_code(t: torch.Tensor | torch.dtype) -> int:
         raise KernelError(f"kernels take float32 or bfloat16, not {dt}") from None
 
 
-def _p(t: torch.Tensor | None):
+def _p(t: torch.Tensor | None) -> int | None:
+    """A tensor's address, as a c_void_p argument takes it."""
     if t is None:
-        return c_void_p(0)
+        return None
     if not t.is_cuda:
         raise KernelError("the kernels run on the GPU only: got a tensor on " + str(t.device))
-    return c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """The current stream of the current device (the handle itself: making torch's stream object took a fifth of a launch's
+    time on the host)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _launches = 0
@@ -124,7 +127,13 @@ def check_status() -> None:
             raise KernelError(f"{lib}: {why} for two seconds and gave up (code {code}); the step's results are not valid")
 
 
+_functions: dict[tuple[str, str], object] = {}       # functions whose library needs no more set-up
+
+
 def _fn(lib: str, name: str, argtypes):
+    fn = _functions.get((lib, name))
+    if fn is not None:
+        return fn
     handle = build.load(lib)
     if lib in _WATCHED:
         _watch(lib, handle)
@@ -133,6 +142,8 @@ def _fn(lib: str, name: str, argtypes):
         fn.argtypes = argtypes
         fn.restype = c_int
         _declared.add((lib, name))
+    if lib not in _WATCHED or lib in _status_words:
+        _functions[(lib, name)] = fn
     return fn
 
 
