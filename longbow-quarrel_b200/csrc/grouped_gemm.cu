@@ -207,7 +207,6 @@ __global__ void __launch_bounds__(1024) group_rows_padded_kernel(const int* __re
     extern __shared__ int sm[];
     int* count = sm;                             // [G]
     int* start = sm + G;                         // [G], in tiles
-    __shared__ int all;                          // tiles of all groups
     const int tid = threadIdx.x;
     pdl_wait();
     for (int g = tid; g < G; g += blockDim.x) count[g] = 0;
@@ -231,9 +230,9 @@ __global__ void __launch_bounds__(1024) group_rows_padded_kernel(const int* __re
             if (g < G) start[g] = at + run - own;
             at += __shfl_sync(0xffffffffu, run, 31);
         }
-        if (tid == 0) all = at;
     }
     __syncthreads();
+    const int all = start[G - 1] + (count[G - 1] + tile - 1) / tile;      // tiles of all groups
     for (int k = tid; k < cap / tile; k += blockDim.x) {
         int g = -1;
         if (k < all) {                           // the last group that starts at or ahead of this tile (empty ones start where the next does)

@@ -14,7 +14,7 @@ def _ops():
     return ops
 
 
-@pytest.mark.parametrize("n,G", [(1, 1), (128, 1), (129, 2), (1023, 31), (1025, 33), (6000, 64), (4096, 1000)])
+@pytest.mark.parametrize("n,G", [(1, 1), (128, 1), (129, 2), (1023, 31), (1025, 33), (6000, 64), (4096, 1000), (5, 6144)])
 def test_every_index_has_one_place_in_a_tile_of_its_group(n, G):
     """Around one warp's sum of the groups' tiles (32 at a time) and the 1024 threads; empty groups first, between and last; ids at
     G and above have no place."""
