@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(MX_WARPS * 32) moe_down_kernel(const T* __rest
 // it multiplies any (one row's two before: a chain of loads), and reads the input once for all R rows, from two planes of four
 // values so that neighbouring lanes read neighbouring 16 bytes.  Bound by the weights' bytes.  Each output is the same sum in the
 // same order as above (even and odd steps of K apart).  8 tokens of
-// 6 of 64 experts, 1,408 x 2,048: first product 54 -> 41 us, second 70 -> 64 (the bytes of the 35 experts chosen: 30 each).
+// 6 of 64 experts, 1,408 x 2,048: first product 54 -> 36 us, second 70 -> 41 (the bytes of the 35 experts chosen: 30 each).  Four
+// blocks an SM: with eight rows' vectors a lane and three blocks both were slower.
 template <int R, int U>
 __device__ __forceinline__ void rows_part(const float4* lo, const float4* hi, const uint4* const (&w)[R], int n8, int lane, float (&out)[R]) {
     float s[R][2];
@@ -263,30 +264,25 @@ __device__ __forceinline__ void rows_part(const float4* lo, const float4* hi, co
             s[r][odd] = t;
         }
     };
-    int k = lane;
-    for (; k + 32 * (U - 1) < n8; k += 32 * U) {
+    static_assert(U % 2 == 0, "even and odd steps are told apart by their place in a round");
+    for (int k = lane; k < n8; k += 32 * U) {
         uint4 v[U][R];
 #pragma unroll
         for (int u = 0; u < U; ++u)
+            if (k + 32 * u < n8) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[u][r] = __ldg(w[r] + k + 32 * u);
+                for (int r = 0; r < R; ++r) v[u][r] = __ldg(w[r] + k + 32 * u);
+            }
 #pragma unroll
-        for (int u = 0; u < U; ++u) multiply(k + 32 * u, v[u], u & 1);
+        for (int u = 0; u < U; ++u)
+            if (k + 32 * u < n8) multiply(k + 32 * u, v[u], u & 1);
     }
-    uint4 v[U - 1][R];
-#pragma unroll
-    for (int u = 0; u < U - 1; ++u)
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (k + 32 * u < n8) v[u][r] = __ldg(w[r] + k + 32 * u);
-#pragma unroll
-    for (int u = 0; u < U - 1; ++u)
-        if (k + 32 * u < n8) multiply(k + 32 * u, v[u], u & 1);
 #pragma unroll
     for (int r = 0; r < R; ++r) out[r] = s[r][0] + s[r][1];
 }
 
 __device__ __forceinline__ void unpack_planes(const uint4* from, float4* lo, float4* hi, int n8) {
+#pragma unroll 4
     for (int i = threadIdx.x; i < n8; i += MX_WARPS * 32) {
         const uint4 v = from[i];
         lo[i] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
@@ -296,7 +292,7 @@ __device__ __forceinline__ void unpack_planes(const uint4* from, float4* lo, flo
 
 // grid (T * top, ceil(F / (MX_WARPS * outputs a warp))): R rows of weight a warp, R / 2 outputs where they are gated.
 template <int R, int U, bool GATED>
-__global__ void __launch_bounds__(MX_WARPS * 32) moe_up_rows_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ w_up,
+__global__ void __launch_bounds__(MX_WARPS * 32, 4) moe_up_rows_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ w_up,
                                                                     const int* __restrict__ ids, __nv_bfloat16* __restrict__ u, int top, int D,
                                                                     int F, int act, int n_real, int block) {
     constexpr int OUT = GATED ? R / 2 : R;
@@ -331,7 +327,7 @@ __global__ void __launch_bounds__(MX_WARPS * 32) moe_up_rows_kernel(const __nv_b
 constexpr int MX_TOP = 64;
 // grid (T, ceil(D / (MX_WARPS * R))); at most MX_TOP choices.
 template <int R, int U>
-__global__ void __launch_bounds__(MX_WARPS * 32) moe_down_rows_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ w_down,
+__global__ void __launch_bounds__(MX_WARPS * 32, 4) moe_down_rows_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ w_down,
                                                                       const int* __restrict__ ids, const float* __restrict__ weights,
                                                                       const float* __restrict__ shared, const float* __restrict__ zs,
                                                                       int zs_stride, float* __restrict__ x, int accumulate, int top,
@@ -426,12 +422,13 @@ LQ_EXPORT int lq_moe_down(const void* u, const void* w_down, const int* ids, con
     typedef __nv_bfloat16 bf;
     if (dtype == LQ_BF16 && F % 8 == 0 && top <= MX_TOP && ((uintptr_t)u | (uintptr_t)w_down) % 16 == 0) {
         auto go = [&](auto kernel, int rows) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            constexpr size_t fixed = MX_TOP * (sizeof(int) + sizeof(float));      // the kernel's other shared memory
+            if (smem + fixed > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             return launch_pdl(kernel, dim3(T, (D + MX_WARPS * rows - 1) / (MX_WARPS * rows)), dim3(MX_WARPS * 32), smem, stream, (const bf*)u,
                               (const bf*)w_down, ids, weights, shared, zs, zs_stride, x, accumulate, top, D, F, (const bf*)h, n_real, shared_scale);
         };
-        // Too few blocks of four rows a warp for two on every SM: two rows a warp.
-        return (long long)T * ((D + 31) / 32) < 296 ? go(moe_down_rows_kernel<2, 4>, 2) : go(moe_down_rows_kernel<4, 2>, 4);
+        // Rows are short here (F) and change with every choice: two rows four steps ahead, so that 1,024 numbers are one round.
+        return go(moe_down_rows_kernel<2, 4>, 2);
     }
 #define LQ_GO(TT) do { if (smem > 48 * 1024) cudaFuncSetAttribute(moe_down_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         return launch_pdl(moe_down_kernel<TT>, grid, dim3(MX_WARPS * 32), smem, stream, (const TT*)u, (const TT*)w_down, ids, weights, \

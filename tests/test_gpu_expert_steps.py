@@ -9,11 +9,11 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("gated,block", [(False, 0), (True, 0), (True, 8)])
-@pytest.mark.parametrize("T,top,E,D,F", [(1, 2, 3, 8, 8), (1, 6, 7, 256, 264), (3, 6, 9, 264, 1000), (9, 3, 4, 1288, 40), (40, 2, 8, 520, 776),
+@pytest.mark.parametrize("T,top,E,D,F", [(1, 2, 3, 8, 8), (1, 6, 7, 256, 264), (3, 6, 9, 264, 1000), (9, 3, 4, 1288, 40), (40, 2, 8, 520, 776), (2, 6, 7, 64, 2048),
                                          (2, 64, 70, 72, 136), (2, 65, 70, 64, 64)])
 def test_several_rows_at_a_time_give_the_bits_of_one(T, top, E, D, F, gated, block):
     """Inputs that do not start on 16 bytes take the kernel of one row at a time: remainders of every unrolled step, outputs that
-    the last warps do not have, two and four rows a warp, identity experts, one choice more than the kernel holds."""
+    the last warps do not have, 48 KB of inputs, identity experts, one choice more than the kernel holds."""
     from longbow_quarrel_b200.kernels import ops
     g = torch.Generator().manual_seed(T + D + F)
     draw = lambda *n: torch.randn(n, generator=g)
