@@ -148,6 +148,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // is the float32-store one and Cout the scratch [splits, plane_rows, N] (plane_rows: M rounded up to 32, so
     // that a warp's box of 32 rows stays inside its range's plane).
     const int total = m_tiles * n_tiles * splits;
+    // Row tiles of one column of tiles by turns: neighbours read the same weights.  Grouped: the columns of one row tile by turns, so that
+    // the blocks at work share few groups' rows and weights, each read from memory once, and the tiles without a group lie behind
+    // all others (12,288 rows in 64 groups, 2,048 x 1,408 with gelu and 1,408 x 2,048: 119 and 94 us, 137 and 127 a column at a time).
+    const auto m_of = [&](int tile) { return tile_group ? tile / n_tiles : tile % m_tiles; };
+    const auto n_of = [&](int tile) { return tile_group ? tile % n_tiles : tile / m_tiles; };
     const int n_kb = (K + BK - 1) / BK;
     constexpr uint32_t STAGE_BYTES = (AROWS + BN) * BK * 2;
     constexpr uint32_t ACC_COLS = BN <= 128 ? 128 : 256;   // columns of tensor memory per accumulator (BN of them used)
@@ -178,10 +183,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x) {
                 const int tile = piece / splits, range = piece % splits;
-                const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
+                const int m0 = m_of(tile) * BM, n0 = n_of(tile) * BN;
                 // Grouped products: the rows of a tile all belong to one group, whose weight is rows
                 // group * N .. of W; a tile without a group (padding behind the last one) is left out by all roles.
-                const int group = tile_group ? tile_group[tile % m_tiles] : 0;
+                const int group = tile_group ? tile_group[m_of(tile)] : 0;
                 if (group < 0) continue;
                 const int kb_lo = (int)((long)n_kb * range / splits), kb_hi = (int)((long)n_kb * (range + 1) / splits);
                 for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
@@ -209,7 +214,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x, ++t) {
-                if (tile_group && tile_group[(piece / splits) % m_tiles] < 0) { --t; continue; }
+                if (tile_group && tile_group[m_of(piece / splits)] < 0) { --t; continue; }
                 const int range = piece % splits;
                 const int kb_lo = (int)((long)n_kb * range / splits), kb_hi = (int)((long)n_kb * (range + 1) / splits);
                 const uint32_t acc = t & 1;
@@ -238,8 +243,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         bool ok = true;
         for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x, ++t) {
             const int tile = piece / splits, range = piece % splits;
-            if (tile_group && tile_group[tile % m_tiles] < 0) { --t; continue; }
-            const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
+            if (tile_group && tile_group[m_of(tile)] < 0) { --t; continue; }
+            const int m0 = m_of(tile) * BM, n0 = n_of(tile) * BN;
             void* dst = splits > 1 ? (void*)((float*)Cout + (size_t)range * plane_rows * N) : Cout;
             const uint32_t acc = t & 1;
             const int m = m0 + quarter * 32 + lane;
@@ -560,7 +565,7 @@ LQ_EXPORT int lq_gemm_tc_qkv(const void* X, const void* W, void* q_out, int M, i
 // g * N .. (g + 1) * N of W [G * N, K].  C [M, N] bfloat16 (out_f32 0) or float32 (1); out_f32 2: every group's rows are
 // 8 gate rows and 8 up rows by turns (N a multiple of 16) and C is [M, N / 2] bfloat16, silu(gate) * up; out_f32 2 + a: bfloat16
 // behind activation a (lq_expert_act) of the float32 sums (N a multiple of 8, C 16-byte aligned; 12,288 rows in
-// 64 groups, 2,048 x 1,408, gelu: 137 us, 130 without and 35 for a kernel of its own).  M a multiple of 128.
+// 64 groups, 2,048 x 1,408, gelu: 7 us more than without, and 35 for a kernel of its own).  M a multiple of 128.
 LQ_EXPORT int lq_gemm_tc_grouped(const void* A, const void* W, void* C, int out_f32, int M, int N, int K, int G,
                                  const int* tile_group, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || G <= 0) return LQ_OK;
