@@ -464,11 +464,11 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(const float* __rest
 }
 
 // The same with everything a head needs asked for at once and held in registers.  VEC 4: LPH lanes a head, NV times four
-// neighbouring values each (whole fours on 16-byte boundaries, no denominator); VEC 1: a warp a head, values lane, lane + 32, ...
-// (with a denominator a row of raw starts anywhere), the sums in the order of the kernel above.  Bound by the bytes: 2,048
-// rows of 32 heads of 64, bfloat16: 22 us one value a load in two passes, 12 here; 3,075 rows of 32 heads of 128 with a denominator
-// 31 and 27.
-template <typename T, int LPH, int NV, int VEC>
+// neighbouring values each (weight, gate and output in whole fours on their boundaries; RAW4: raw too, which with a denominator
+// behind each head starts anywhere); VEC 1: a warp a head, values lane, lane + 32, ..., the sums in the order of the kernel above.
+// Bound by the bytes: 2,048 rows of 32 heads of 64, bfloat16: 22 us one value a load in two passes, 12 here; 3,075 rows of 32
+// heads of 128 with a denominator 31 and 23 (27 one value a load).
+template <typename T, int LPH, int NV, int VEC, bool RAW4>
 __global__ void __launch_bounds__(128) head_norm_gate_held_kernel(const float* __restrict__ raw, int dvx, const float* __restrict__ exp_neg_m,
                                                                   const float* __restrict__ weight, const T* __restrict__ gate,
                                                                   int gate_stride, int act, T* __restrict__ out, int n_pairs,
@@ -488,7 +488,12 @@ __global__ void __launch_bounds__(128) head_norm_gate_held_kernel(const float* _
         for (int e = 0; e < VEC; ++e) { v[i][e] = 0.f; g[i][e] = 0.f; w[i][e] = 1.f; }
         if (!in) continue;
         if constexpr (VEC == 4) {
-            *reinterpret_cast<float4*>(v[i]) = *reinterpret_cast<const float4*>(r + d);
+            if constexpr (RAW4) {
+                *reinterpret_cast<float4*>(v[i]) = *reinterpret_cast<const float4*>(r + d);
+            } else {
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) v[i][e] = r[d + e];
+            }
             if (weight) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(weight + h * dv + d);
             if (act) {
                 if constexpr (sizeof(T) == 4) {
@@ -549,15 +554,17 @@ static int head_norm_gate_held(const float* raw, int dvx, const float* exp_neg_m
         return launch_pdl(kernel, dim3((n + per - 1) / per), dim3(128), 0, stream, raw, dvx, exp_neg_m, weight, (const T*)gate, gate_stride, act,
                           (T*)out, n, H, dv, eps);
     };
-    const bool fours = !exp_neg_m && dv % 4 == 0 && dvx == dv && (uintptr_t)raw % 16 == 0 && (uintptr_t)weight % 16 == 0 &&
-                       (uintptr_t)out % (4 * sizeof(T)) == 0 && (!act || (gate_stride % 4 == 0 && (uintptr_t)gate % (4 * sizeof(T)) == 0));
-    if (fours && dv <= 32) return go(head_norm_gate_held_kernel<T, 8, 1, 4>, 8);
-    if (fours && dv <= 64) return go(head_norm_gate_held_kernel<T, 16, 1, 4>, 16);
-    if (fours && dv <= 128) return go(head_norm_gate_held_kernel<T, 32, 1, 4>, 32);
-    if (fours && dv <= 256) return go(head_norm_gate_held_kernel<T, 32, 2, 4>, 32);
-    if (dv <= 64) return go(head_norm_gate_held_kernel<T, 32, 2, 1>, 32);
-    if (dv <= 128) return go(head_norm_gate_held_kernel<T, 32, 4, 1>, 32);
-    if (dv <= 256) return go(head_norm_gate_held_kernel<T, 32, 8, 1>, 32);
+    const bool fours = dv % 4 == 0 && (uintptr_t)weight % 16 == 0 && (uintptr_t)out % (4 * sizeof(T)) == 0 &&
+                       (!act || (gate_stride % 4 == 0 && (uintptr_t)gate % (4 * sizeof(T)) == 0));
+    const bool raw4 = dvx % 4 == 0 && (uintptr_t)raw % 16 == 0;
+    auto four = [&](auto with, auto without, int lanes) { return raw4 ? go(with, lanes) : go(without, lanes); };
+    if (fours && dv <= 32) return four(head_norm_gate_held_kernel<T, 8, 1, 4, true>, head_norm_gate_held_kernel<T, 8, 1, 4, false>, 8);
+    if (fours && dv <= 64) return four(head_norm_gate_held_kernel<T, 16, 1, 4, true>, head_norm_gate_held_kernel<T, 16, 1, 4, false>, 16);
+    if (fours && dv <= 128) return four(head_norm_gate_held_kernel<T, 32, 1, 4, true>, head_norm_gate_held_kernel<T, 32, 1, 4, false>, 32);
+    if (fours && dv <= 256) return four(head_norm_gate_held_kernel<T, 32, 2, 4, true>, head_norm_gate_held_kernel<T, 32, 2, 4, false>, 32);
+    if (dv <= 64) return go(head_norm_gate_held_kernel<T, 32, 2, 1, false>, 32);
+    if (dv <= 128) return go(head_norm_gate_held_kernel<T, 32, 4, 1, false>, 32);
+    if (dv <= 256) return go(head_norm_gate_held_kernel<T, 32, 8, 1, false>, 32);
     return launch_pdl(head_norm_gate_kernel<T>, dim3((n + 3) / 4), dim3(128), 0, stream, raw, dvx, exp_neg_m, weight, (const T*)gate, gate_stride,
                       act, (T*)out, n, H, dv, eps);
 }
