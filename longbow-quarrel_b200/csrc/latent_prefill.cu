@@ -14,6 +14,10 @@
 // Measured, 2,048 tokens of 16 heads, R = 512, us: attention, expansion and the maps of the absorbed form 686 + 102 + 78, this kernel
 // 64 (340 TFLOP/s; 128 blocks of equal work), the expansion 8, gather and turn 3 each; the whole layer 910 and 184 (heads 32, width
 // 4,096: 1,818 and 321; 4,096 tokens: 5,559 and 657).  Distance of the layer from 64 bits 3.67e-3 absorbed, 3.64e-3 here.
+// A cached row with an infinity or a NaN belongs to the rows that see it alone, but a tile's product meets all 128 of its keys, and 0 x NaN is
+// NaN: rows ahead of it in its sequence, and in the next sequence's first tile, would be lost.  The gather writes zeros in the
+// place of such a latent and marks it, and the rows that see a marked key come out as NaN (two warps without other work look the marks
+// over meanwhile; the whole layer 178.5 us before, 181 with the marks).
 // Every wait on a barrier is bounded (status word).
 #include "tcgen05.cuh"
 #include <math_constants.h>
@@ -35,7 +39,8 @@ struct Smem {
     alignas(1024) uint8_t v[2][2][PANEL / 2];         // [half of the keys][panel][64 keys x 128 B]
     alignas(8) uint64_t q_full;
     uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
-    uint64_t s_full[2], p_full[2], pv_done[2];        // per chain
+    uint64_t s_full[2], p_full[2], pv_done[2], marks_read[2];      // per chain
+    uint32_t marked[2];                               // whether any key of the chain's tiles is marked
     uint32_t tmem_base;
 };
 
@@ -64,7 +69,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                       const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_kr,
                       const __grid_constant__ CUtensorMap map_v, const int* __restrict__ blocks, int n_blocks,
                       const int* __restrict__ first_row, const int* __restrict__ lo, const int* __restrict__ kv_len,
-                      __nv_bfloat16* __restrict__ out, int H, float scale_log2, int window, const float* __restrict__ sink) {
+                      const uint8_t* __restrict__ marks, __nv_bfloat16* __restrict__ out, int H, float scale_log2, int window, const float* __restrict__ sink) {
     extern __shared__ uint8_t smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,6 +85,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             mbar_init(smem_u32(&sm.s_full[s]), 1);
             mbar_init(smem_u32(&sm.p_full[s]), BM);
             mbar_init(smem_u32(&sm.pv_done[s]), 1);
+            mbar_init(smem_u32(&sm.marks_read[s]), 1);
         }
         mbar_fence_init();
         prefetch_map(&map_q);
@@ -203,6 +209,17 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
                 if (ok && t + 1 < t_hi) commit(smem_u32(&sm.k_empty[s1]));
             }
+        } else if (warp >= 2) {
+            // ------------------------------------------------------------ marks of chain warp - 2, a key a lane
+            const int c = warp - 2, end = key_row + (c ? to[1] : to[0]) * BN;      // rows + BN at most: marks reach that far
+            uint32_t any = 0;
+#pragma unroll 8
+            for (int i = key_row + (c ? from[1] : from[0]) * BN + lane; i < end; i += 32) any |= marks[i];
+            any = __any_sync(0xffffffffu, any);
+            if (lane == 0) {
+                sm.marked[c] = any;
+                mbar_arrive(smem_u32(&sm.marks_read[c]));
+            }
         }
         __syncwarp();
     } else {
@@ -281,11 +298,15 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         if (ok && n_tiles > 0) {
             LQ_WAIT(sm.pv_done[chain], (n_tiles - 1) & 1, 8);
+            if (ok) LQ_WAIT(sm.marks_read[chain], 0, 9);
         }
         if (ok && n_tiles > 0) {
             fence_after();
+            bool lost = false;                           // this row sees a marked key
+            if (sm.marked[chain])
+                for (int key = first_r; key <= pos_r && key < len; ++key) lost |= marks[key_row + key] != 0;
             if (sink) l += ex2(fmaf(sink[h], 1.4426950408889634f, m_ref == -CUDART_INF_F ? 0.f : -m_ref));
-            const float inv = 1.0f / l;
+            const float inv = lost ? CUDART_NAN_F : 1.0f / l;
             __nv_bfloat16* orow = out + ((size_t)((chain ? row0[1] : row0[0]) + r) * H + h) * DV;
 #pragma unroll 1
             for (int c = 0; c < DV / 32; ++c) {
@@ -313,16 +334,23 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 }
 
 // ------------------------------------------------------------------ gather and turn
+// Whether one of two bfloat16 is an infinity or a NaN.
+__device__ __forceinline__ bool not_finite(uint32_t v) { return (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u; }
+
 // A warp per expanded row: its latent (R numbers) to c, its shared key part (DR) to kr; positions whose page has gone back
-// (ahead of every window) are zero.
+// (ahead of every window) are zero.  marks [rows + BN]: 1 where the latent holds an infinity or a NaN (c is then zero); 0 behind the last row.
 __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ pages, const int* __restrict__ page_table, int pt_stride,
                                                             const int* __restrict__ slots, const int* __restrict__ first_row,
                                                             const int* __restrict__ lo, int B, int rows, int R, int page_size,
-                                                            __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ kr) {
+                                                            __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ kr,
+                                                            uint8_t* __restrict__ marks) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= rows) return;
+    if (row >= rows) {
+        if (row < rows + BN && lane == 0) marks[row] = 0;
+        return;
+    }
     int b = 0, hi = B - 1;                         // the last sequence that starts at or ahead of this row
     while (b < hi) {
         const int mid = (b + hi + 1) / 2;
@@ -334,11 +362,20 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16*
     const uint4* src = reinterpret_cast<const uint4*>(pages + ((size_t)max(page, 0) * page_size + pos % page_size) * (R + DR));
     uint4* dc = reinterpret_cast<uint4*>(c + (size_t)row * R);
     uint4* dr = reinterpret_cast<uint4*>(kr + (size_t)row * DR);
+    bool odd = false;
     for (int i = lane; i < (R + DR) / 8; i += 32) {
         const uint4 v = page >= 0 ? src[i] : make_uint4(0, 0, 0, 0);
-        if (i < R / 8) dc[i] = v;
-        else dr[i - R / 8] = v;
+        if (i < R / 8) {
+            dc[i] = v;
+            odd = odd || not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w);
+        } else {
+            dr[i - R / 8] = v;
+        }
     }
+    odd = __any_sync(0xffffffffu, odd);
+    if (odd)
+        for (int i = lane; i < R / 8; i += 32) dc[i] = make_uint4(0, 0, 0, 0);
+    if (lane == 0) marks[row] = odd;
 }
 
 // Four pairs a thread: head h's rotated part (columns h (DN + DR) + DN of q) turned by the row's position, to out [T, H DR].
@@ -366,12 +403,13 @@ __global__ void __launch_bounds__(256) latent_turn_kernel(const __nv_bfloat16* _
 
 }  // namespace
 
+// The marks lie behind kr's rows: rows + 128 bytes.
 LQ_EXPORT int lq_latent_gather(const void* pages, const int* page_table, int pt_stride, const int* slots, const int* first_row,
                                const int* lo, int B, int rows, int R, int page_size, void* c, void* kr, cudaStream_t stream) {
     if (rows <= 0) return LQ_OK;
     if (R % 8 || ((uintptr_t)pages | (uintptr_t)c | (uintptr_t)kr) % 16) return LQ_BAD_SIZE;
-    return launch_pdl(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)pages, page_table, pt_stride,
-                      slots, first_row, lo, B, rows, R, page_size, (__nv_bfloat16*)c, (__nv_bfloat16*)kr);
+    return launch_pdl(latent_gather_kernel, dim3((rows + BN + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)pages, page_table, pt_stride,
+                      slots, first_row, lo, B, rows, R, page_size, (__nv_bfloat16*)c, (__nv_bfloat16*)kr, (uint8_t*)kr + (size_t)rows * DR * 2);
 }
 
 // q [T, H (128 + 64)] -> the rotated parts [T, H 64] (cos_t null: as they are).
@@ -384,7 +422,8 @@ LQ_EXPORT int lq_latent_turn(const void* q, const float* cos_t, const float* sin
                       tok_pos, T, H, (__nv_bfloat16*)out);
 }
 
-// q [T, H 192] (its first 128 of a head), qr [T, H 64], kv [rows, H (128 + 128)] keys then values, kr [rows, 64]; out [T, H 128].
+// q [T, H 192] (its first 128 of a head), qr [T, H 64], kv [rows, H (128 + 128)] keys then values, kr [rows, 64] and its marks as
+// lq_latent_gather wrote them; out [T, H 128].
 LQ_EXPORT int lq_latent_prefill(const void* q, const void* qr, const void* kv, const void* kr, int T, int rows, const int* blocks, int n_blocks,
                                 const int* first_row, const int* lo, const int* kv_len, void* out, int H, float scale, int window,
                                 const float* sink, cudaStream_t stream) {
@@ -402,7 +441,7 @@ LQ_EXPORT int lq_latent_prefill(const void* q, const void* qr, const void* kv, c
     if (cudaFuncSetAttribute(latent_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return lq_launch_status();
     return launch_pdl(latent_prefill_kernel, dim3(n_blocks * H), dim3(N_THREADS), smem, stream, mq, mqr, mk, mkr, mv, blocks, n_blocks,
-                      first_row, lo, kv_len, (__nv_bfloat16*)out, H, scale * 1.4426950408889634f, window, sink);
+                      first_row, lo, kv_len, (const uint8_t*)kr + (size_t)rows * DR * 2, (__nv_bfloat16*)out, H, scale * 1.4426950408889634f, window, sink);
 }
 
 // The status word in host memory that the device writes through; null when it could not be set up.

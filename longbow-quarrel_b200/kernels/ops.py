@@ -97,7 +97,8 @@ _WATCHED = {"gemm_tc": {1: "the TMA producer waited for a free stage", 2: "the p
             "latent_prefill": {1: "the TMA producer waited for a free stage of keys", 2: "the TMA producer waited for free values",
                                3: "the product issuer waited for the queries", 4: "the product issuer waited for keys",
                                5: "the product issuer waited for probabilities", 6: "the product issuer waited for values",
-                               7: "a softmax warp waited for scores", 8: "a softmax warp waited for the last product"},
+                               7: "a softmax warp waited for scores", 8: "a softmax warp waited for the last product",
+                               9: "a softmax warp waited for the marks"},
             "delta": {1: "the copying warp waited for a free stage", 2: "a warp waited for a record"},
             "head_delta": {1: "the copying warp waited for a free stage", 2: "a warp waited for a chunk"}}
 _status_words: dict[str, object] = {}
@@ -766,13 +767,19 @@ def latent_attention_tc(q: torch.Tensor, pages: torch.Tensor, page_table, slots,
 LATENT_EXPANDED = (128, 64, 128)      # a head's unrotated, rotated and value sizes that lq_latent_prefill is built for
 
 
+def _mark_rows(rows: int) -> int:
+    """Rows of 128 bytes that the marks of `rows` expanded rows take."""
+    return rows // 128 + 2
+
+
 def latent_gather(pages: torch.Tensor, page_table, slots, first_row, lo, B: int, rows: int, R: int, page_size: int) -> tuple:
-    """The cached rows [.., R + 64] of a step's sequences side by side: (latents [rows, R], shared key parts [rows, 64]).  Sequence
-    b's rows stand at first_row[b] .. and begin at its position lo[b]."""
+    """The cached rows [.., R + 64] of a step's sequences side by side: (latents [rows, R], shared key parts [rows, 64] with
+    rows + 128 bytes of marks behind them, as more of its rows).  Sequence b's rows stand at first_row[b] .. and begin at its position
+    lo[b].  A latent that holds an infinity or a NaN is marked and comes as zeros."""
     if pages.dtype != torch.bfloat16 or pages.shape[-1] != R + 64 or pages.stride(-2) != R + 64 or pages.stride(0) != page_size * (R + 64):
         raise KernelError("latent_gather: contiguous bfloat16 pages of rows [R + 64]")
     c = torch.empty((rows, R), dtype=torch.bfloat16, device=pages.device)
-    kr = torch.empty((rows, 64), dtype=torch.bfloat16, device=pages.device)
+    kr = torch.empty((rows + _mark_rows(rows), 64), dtype=torch.bfloat16, device=pages.device)
     fn = _fn("latent_prefill", "lq_latent_gather", [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                                     c_void_p, c_void_p])
     _check(fn(_p(pages), _p(page_table), page_table.stride(0), _p(slots), _p(first_row), _p(lo), B, rows, R, page_size, _p(c), _p(kr), _stream()),
@@ -792,15 +799,17 @@ def latent_turn(q: torch.Tensor, cos, sin, tok_pos, H: int) -> torch.Tensor:
 def latent_prefill(q: torch.Tensor, qr: torch.Tensor, kv: torch.Tensor, kr: torch.Tensor, blocks: torch.Tensor, first_row, lo, kv_len, H: int,
                    scale: float, window: int | None, sink: torch.Tensor | None = None) -> torch.Tensor:
     """Attention of a prompt over expanded keys and values (csrc/latent_prefill.cu): q bfloat16 [T, H 192] (a head's first 128 are
-    read), qr [T, H 64] its rotated parts, kv [rows, H 256] the heads' keys, then their values, kr [rows, 64] the shared key
-    part.  blocks int32 [7, n]; sequence b's keys stand at rows first_row[b] .. and begin at position lo[b].  Returns
-    bfloat16 [T, H 128]."""
+    read), qr [T, H 64] its rotated parts, kv [rows, H 256] the heads' keys, then their values, kr of
+    latent_gather the shared key part: a row that sees a marked key comes out as NaN.  blocks int32 [7, n]; sequence b's keys stand
+    at rows first_row[b] .. and begin at position lo[b].  Returns bfloat16 [T, H 128]."""
     T, rows = q.shape[0], kv.shape[0]
     for t, width in ((q, H * 192), (qr, H * 64), (kv, H * 256), (kr, 64)):
         if t.dtype != torch.bfloat16 or t.shape[1] != width or not t.is_contiguous():
-            raise KernelError("latent_prefill: contiguous bfloat16 q [T, H 192], qr [T, H 64], kv [rows, H 256], kr [rows, 64]")
+            raise KernelError("latent_prefill: contiguous bfloat16 q [T, H 192], qr [T, H 64], kv [rows, H 256], kr [.., 64]")
     if blocks.dtype != torch.int32 or blocks.dim() != 2 or blocks.shape[0] != 7 or not blocks.is_contiguous():
         raise KernelError("latent_prefill: the work list must be contiguous int32 [7, n]")
+    if kr.shape[0] != rows + _mark_rows(rows):
+        raise KernelError("latent_prefill: kr as latent_gather made it for kv's rows")
     _check_sink(sink, H)
     out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
     fn = _fn("latent_prefill", "lq_latent_prefill", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,

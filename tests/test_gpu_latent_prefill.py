@@ -79,3 +79,22 @@ def test_few_queries_per_key_keep_the_absorbed_form():
     assert routes == [1, 0, 0]
     want, _ = _run(_part(torch.float32, 2, None, False, weights)[0], [(310,)], h)
     assert float((got[0] - want[0]).norm() / want[0].norm()) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("H,window,portions,spoiled", [
+    (2, None, [(100, 70)], (0, 60)), (2, None, [(100, 70)], (1, 0)), (1, None, [(300, 40), (20, 200)], (0, 130)), (2, 90, [(400, 200)], (0, 137)),
+    (16, None, [(700, 31)], (0, 699))])
+def test_a_row_that_is_not_finite_spoils_only_the_rows_that_see_it(H, window, portions, spoiled):
+    """A token of NaN: every row that sees it is NaN, and no other, ahead of it in its sequence or in its neighbour, whose expanded rows
+    share a tile of keys with it."""
+    gen = torch.Generator().manual_seed(5)
+    h = [torch.randn(sum(s[i] for s in portions), D, generator=gen).to(torch.bfloat16).to(DEV) for i in range(len(portions[0]))]
+    part, _ = _part(torch.bfloat16, H, window, False)
+    clean, _ = _run(part, portions, h)
+    h[spoiled[0]][spoiled[1]] = float("nan")
+    got, routes = _run(part, portions, h)
+    assert all(routes)
+    for i, (g, c) in enumerate(zip(got, clean)):
+        at = torch.arange(g.shape[0], device=DEV)
+        sees = (at >= spoiled[1]) & ((at < spoiled[1] + window) if window else True) & (i == spoiled[0])
+        assert torch.isnan(g[sees]).all() and torch.equal(g[~sees], c[~sees])
