@@ -69,9 +69,9 @@ class LatentAttention(Mixer):
         self.w_uk = self.w_uv = self.w_uk_t = self.w_uv_t = self.g_q = self.g_kv = None
         self.tc_heads = False
         # Sizes whose prompts may run over expanded keys and values (w_kv, made at load); whether a step's do is
-        # attention_kernels.expands' answer.
+        # attention_kernels.expands' answer.  (That kernel takes the maximum ahead of the scale, which must be positive for it.)
         self.expandable = (runtime.dtype == torch.bfloat16 and (head_dim, rot_dim, value_dim) == ops.LATENT_EXPANDED and kv_rank % 8 == 0
-                           and self.rot in (0, rot_dim))
+                           and self.rot in (0, rot_dim) and self.scale > 0)
         self.w_kv: linear.LinearWeight | None = None
 
     def cache_need(self):

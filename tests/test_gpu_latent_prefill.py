@@ -8,13 +8,13 @@ DEV = torch.device("cuda:0")
 D, R = 192, 64
 
 
-def _part(dtype, H, window, sink, weights=None):
+def _part(dtype, H, window, sink, weights=None, scale=0.12):
     from longbow_quarrel_b200.parts.base import Runtime
     from longbow_quarrel_b200.parts.latent_attention import LatentAttention
     from longbow_quarrel_b200.parts.spec import PartSpec
     from longbow_quarrel_b200.weights import random_weights
     part = LatentAttention(Runtime(DEV, dtype, 2048), hidden_size=D, n_heads=H, head_dim=128, rot_dim=64, value_dim=128, q_rank=None, kv_rank=R,
-                           scale=0.12, eps=1e-5, position=PartSpec("rope", {"head_dim": 64, "theta": 1e4}), window=window, sink=sink)
+                           scale=scale, eps=1e-5, position=PartSpec("rope", {"head_dim": 64, "theta": 1e4}), window=window, sink=sink)
     weights = weights or random_weights(part.weights(), 3, torch.bfloat16, DEV, std=0.08)
     part.load(weights)
     return part, weights
@@ -98,3 +98,14 @@ def test_a_row_that_is_not_finite_spoils_only_the_rows_that_see_it(H, window, po
         at = torch.arange(g.shape[0], device=DEV)
         sees = (at >= spoiled[1]) & ((at < spoiled[1] + window) if window else True) & (i == spoiled[0])
         assert torch.isnan(g[sees]).all() and torch.equal(g[~sees], c[~sees])
+
+
+@pytest.mark.parametrize("scale", [-0.12, 0.0])
+def test_scales_that_are_not_positive_keep_the_absorbed_form(scale):
+    gen = torch.Generator().manual_seed(2)
+    h = [torch.randn(150, D, generator=gen).to(torch.bfloat16).to(DEV)]
+    part, weights = _part(torch.bfloat16, 2, None, False, scale=scale)
+    got, routes = _run(part, [(150,)], h)
+    assert routes == [0]
+    want, _ = _run(_part(torch.float32, 2, None, False, weights, scale=scale)[0], [(150,)], h)
+    assert float((got[0] - want[0]).norm() / want[0].norm()) < 3 * 2.0 ** -8
