@@ -40,11 +40,12 @@ def query_blocks(size: int):
 
 # ------------------------------------------------------------------ latent attention over expanded keys and values
 EXPAND_TILE = 128
-# Query rows per key, over a step's sequences, from which keys and values are expanded: measured, us absorbed and expanded, 16 heads:
-# 24 rows 260 / 251, 64 rows 263 / 262 (both the host's launches), 32 rows on 2,000 earlier ones 442 / 251, 2,048 rows 910 / 279; 32
-# heads, 16 rows on 1,000 earlier ones 274 / 218.
+# New rows from which a sequence's keys and values are expanded (every key is expanded once and met by all of them).  Measured, us of
+# attention, absorbed and expanded: 16 heads, a latent of 512: 16 rows 95 / 28, 2,048 rows 827 / 93, 16 rows on 1,000 earlier ones
+# 236 / 72; 4 heads, 128: 57 / 26, 218 / 75, 120 / 63; 2 heads, 64: 42 / 26, 167 / 75, 82 / 65.  A whole layer of fewer rows is bound by its
+# launches, of which the expanded form has as many.
 EXPAND_QUERIES = 16
-EXPAND_ELEMENTS = 1 << 29          # the most expanded numbers (1 GB in bfloat16); a longer step keeps the absorbed form
+EXPAND_ELEMENTS = 1 << 29          # the most expanded numbers at a time (1 GB in bfloat16): more sequences go in turns, a longer one stays absorbed
 
 
 def expanded_rows(past, new, window: int) -> tuple[list[int], list[int]]:
@@ -53,35 +54,70 @@ def expanded_rows(past, new, window: int) -> tuple[list[int], list[int]]:
     return lo, [p + n - a for p, n, a in zip(past, new, lo)]
 
 
-def expands(past, new, window: int, H: int, per_head: int) -> bool:
-    """Whether a step's latent attention runs over expanded keys and values (per_head numbers for each head and key)."""
-    if max(new) == 1:
-        return False
+def expanded_turns(past, new, window: int, H: int, per_head: int) -> list[list[int]]:
+    """The sequences of a step whose latent attention runs over expanded keys and values (per_head numbers for each head and key), in
+    turns that share one set of buffers.  Whether a sequence is among them is a matter of its own rows, not of its neighbours."""
+    if max(new) < EXPAND_QUERIES:
+        return []
     _, rows = expanded_rows(past, new, window)
-    pairs = sum(n * r for n, r in zip(new, rows))
-    return pairs >= EXPAND_QUERIES * sum(rows) and sum(rows) * H * per_head <= EXPAND_ELEMENTS
+    turns, held = [], 0
+    for b, (n, r) in enumerate(zip(new, rows)):
+        each = r * H * per_head
+        if n < EXPAND_QUERIES or each > EXPAND_ELEMENTS:
+            continue
+        if not turns or held + each > EXPAND_ELEMENTS:
+            turns.append([])
+            held = 0
+        turns[-1].append(b)
+        held += each
+    return turns
+
+
+def expanded_blocks(new, turn: list[int]) -> int:
+    """Blocks of one turn: two chains of at most 128 rows each."""
+    return sum((-(-new[b] // 128) + 1) // 2 for b in turn)
 
 
 def expanded_work(H: int, per_head: int, window: int, sms: int):
-    """Builder of lq_latent_prefill's step array: blocks [7, n] (sequence, then first row, rows and first position of two chains of
-    at most 128 rows), where every sequence's expanded rows start [B + 1], the position of its first one [B]; empty for a step that
-    keeps the absorbed form."""
+    """Builder of lq_latent_prefill's step array.  For every turn: blocks [7, n] (sequence, then first row, rows and first position of
+    two chains of at most 128 rows), where every sequence's expanded rows start [B + 1] (no rows for those of other turns), the position
+    of its first one [B]; empty for a step without any."""
     def build(step) -> np.ndarray:
-        if not expands(step.past, step.new, window, H, per_head):
-            return np.zeros(0, dtype=np.int32)
         lo, rows = expanded_rows(step.past, step.new, window)
-        tiles = [[(step.cu[b] + r, min(128, n - r), p + r) for r in range(0, n, 128)] for b, (p, n) in enumerate(zip(step.past, step.new))]
-        # Chains of neighbouring rows share all their tiles of keys.  A step whose blocks all run at once is as long as its longest
-        # block: there the first rows go with the last ones, so that all blocks have the same work (not under a window, where
-        # two such chains would have no keys in common).
-        level = window <= 0 and sum((len(t) + 1) // 2 for t in tiles) * H <= sms
-        none, blocks = (0, 0, 0), []
-        for b, t in enumerate(tiles):
-            for i in range((len(t) + 1) // 2):
-                first, second = (i, len(t) - 1 - i) if level else (2 * i, 2 * i + 1)
-                blocks.append((b, *t[first], *(t[second] if first < second < len(t) else none)))
-        blocks.sort(key=lambda e: -sum((e[k + 2] + e[k + 1]) // 128 + 1 for k in (1, 4) if e[k + 1]))
-        return np.concatenate([np.asarray(blocks, dtype=np.int32).T.reshape(-1), np.cumsum([0] + rows), lo]).astype(np.int32)
+        parts = [np.zeros(0, dtype=np.int32)]
+        for turn in expanded_turns(step.past, step.new, window, H, per_head):
+            tiles = {b: [(step.cu[b] + r, min(128, step.new[b] - r), step.past[b] + r) for r in range(0, step.new[b], 128)] for b in turn}
+            # Chains of neighbouring rows share all their tiles of keys.  A turn whose blocks all run at once is as long as its longest
+            # block: there the first rows go with the last ones, so that all blocks have the same work (not under a window, where
+            # two such chains would have no keys in common).
+            level = window <= 0 and expanded_blocks(step.new, turn) * H <= sms
+            none, blocks = (0, 0, 0), []
+            for b, t in tiles.items():
+                for i in range((len(t) + 1) // 2):
+                    first, second = (i, len(t) - 1 - i) if level else (2 * i, 2 * i + 1)
+                    blocks.append((b, *t[first], *(t[second] if first < second < len(t) else none)))
+            blocks.sort(key=lambda e: -sum((e[k + 2] + e[k + 1]) // 128 + 1 for k in (1, 4) if e[k + 1]))
+            held = [r if b in tiles else 0 for b, r in enumerate(rows)]
+            parts += [np.asarray(blocks, dtype=np.int32).T.reshape(-1), np.cumsum([0] + held), lo]
+        return np.concatenate(parts).astype(np.int32)
+    return build
+
+
+def absorbed_rest(size: int, H: int, per_head: int, window: int):
+    """Builder of the absorbed kernel's work list (query_blocks(size)) for the sequences that are not expanded: their blocks, over their
+    rows side by side, then which rows of the step these are.  A step without expanded sequences: the blocks alone."""
+    every = query_blocks(size)
+
+    def build(step) -> np.ndarray:
+        expanded = {b for turn in expanded_turns(step.past, step.new, window, H, per_head) for b in turn}
+        rest = [b for b in range(step.B) if b not in expanded]
+        if not expanded or not rest:
+            return every(step).reshape(-1) if rest else np.zeros(0, dtype=np.int32)
+        new = tuple(step.new[b] for b in rest)
+        cu = tuple(int(c) for c in np.cumsum((0,) + new))
+        blocks = every(type(step)(B=len(rest), T=cu[-1], past=tuple(step.past[b] for b in rest), new=new, cu=cu)).reshape(4, -1)
+        blocks[0] = np.asarray(rest, dtype=np.int32)[blocks[0]]
+        return np.concatenate([blocks.reshape(-1)] + [np.arange(step.cu[b], step.cu[b + 1]) for b in rest]).astype(np.int32)
     return build
 
 

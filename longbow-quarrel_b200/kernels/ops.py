@@ -797,11 +797,12 @@ def latent_turn(q: torch.Tensor, cos, sin, tok_pos, H: int) -> torch.Tensor:
 
 
 def latent_prefill(q: torch.Tensor, qr: torch.Tensor, kv: torch.Tensor, kr: torch.Tensor, blocks: torch.Tensor, first_row, lo, kv_len, H: int,
-                   scale: float, window: int | None, sink: torch.Tensor | None = None) -> torch.Tensor:
+                   scale: float, window: int | None, sink: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """Attention of a prompt over expanded keys and values (csrc/latent_prefill.cu): q bfloat16 [T, H 192] (a head's first 128 are
     read), qr [T, H 64] its rotated parts, kv [rows, H 256] the heads' keys, then their values, kr of
     latent_gather the shared key part: a row that sees a marked key comes out as NaN.  blocks int32 [7, n]; sequence b's keys stand
-    at rows first_row[b] .. and begin at position lo[b].  Returns bfloat16 [T, H 128]."""
+    at rows first_row[b] .. and begin at position lo[b].  Returns bfloat16 [T, H 128] (out, if given, the
+    rows of other sequences as they were)."""
     T, rows = q.shape[0], kv.shape[0]
     for t, width in ((q, H * 192), (qr, H * 64), (kv, H * 256), (kr, 64)):
         if t.dtype != torch.bfloat16 or t.shape[1] != width or not t.is_contiguous():
@@ -811,7 +812,10 @@ def latent_prefill(q: torch.Tensor, qr: torch.Tensor, kv: torch.Tensor, kr: torc
     if kr.shape[0] != rows + _mark_rows(rows):
         raise KernelError("latent_prefill: kr as latent_gather made it for kv's rows")
     _check_sink(sink, H)
-    out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
+    if out is None:
+        out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
+    elif out.dtype != torch.bfloat16 or tuple(out.shape) != (T, H * 128) or not out.is_contiguous():
+        raise KernelError("latent_prefill: out must be contiguous bfloat16 [T, H 128]")
     fn = _fn("latent_prefill", "lq_latent_prefill", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                                      c_void_p, c_void_p, c_int, c_float, c_int, c_void_p, c_void_p])
     _check(fn(_p(q), _p(qr), _p(kv), _p(kr), T, rows, _p(blocks), blocks.shape[1], _p(first_row), _p(lo), _p(kv_len), _p(out), H, float(scale),

@@ -8,8 +8,8 @@
 Only c and the rotated k_r are cached: one row of `kv_rank + rot_dim` numbers per token for all
 heads (`KVNeed` with one kv head and no value pool).  Keys and values are never expanded per
 cached token: the per-head maps go to the query's side, (W_uk,h^T q_h) . c_j and W_uv,h (sum_j p_j c_j),
-so the attention is multi-query attention over the latent rows (`csrc/latent_attn.cu`).  A step with many query
-rows per key (prompts; heads of 128 + 64 and values of 128 in bfloat16) expands the keys and values of the positions it sees
+so the attention is multi-query attention over the latent rows (`csrc/latent_attn.cu`).  A sequence that
+brings many rows (prompts; heads of 128 + 64 and values of 128 in bfloat16) has the keys and values of the positions it sees expanded
 instead, for the length of the step: three and a half times fewer operations per pair (`csrc/latent_prefill.cu`).
 
 Norms, angles, scores and the softmax are 32-bit; in bfloat16 runs the projections' outputs that
@@ -22,7 +22,8 @@ the softmax denominator, with no key and no value).
 """
 from __future__ import annotations
 
-import numpy as np
+from dataclasses import replace
+
 import torch
 
 from ..kernels import attention as attention_kernels
@@ -68,8 +69,8 @@ class LatentAttention(Mixer):
         self.w_o: linear.LinearWeight | None = None
         self.w_uk = self.w_uv = self.w_uk_t = self.w_uv_t = self.g_q = self.g_kv = None
         self.tc_heads = False
-        # Sizes whose prompts may run over expanded keys and values (w_kv, made at load); whether a step's do is
-        # attention_kernels.expands' answer.  (That kernel takes the maximum ahead of the scale, which must be positive for it.)
+        # Sizes whose prompts may run over expanded keys and values (w_kv, made at load); which sequences of a step do is
+        # attention_kernels.expanded_turns' answer.  (That kernel takes the maximum ahead of the scale, which must be positive for it.)
         self.expandable = (runtime.dtype == torch.bfloat16 and (head_dim, rot_dim, value_dim) == ops.LATENT_EXPANDED and kv_rank % 8 == 0
                            and self.rot in (0, rot_dim) and self.scale > 0)
         self.w_kv: linear.LinearWeight | None = None
@@ -82,13 +83,15 @@ class LatentAttention(Mixer):
         if self.runtime.dtype != torch.bfloat16 or (self.R + self.dr) % 8:
             return {}
         size = ops.latent_tc_tokens(self.H)
-        blocks = attention_kernels.query_blocks(size)
         if self.w_kv is None:                    # sizes or weights that keep the absorbed form throughout
-            return {f"latent_blocks{size}": blocks}
+            return {self._blocks_name(): attention_kernels.query_blocks(size)}
         H, each, window = self.H, self.dn + self.dv, int(self.window or 0)
-        absorbed = lambda step: np.zeros(0, dtype=np.int32) if attention_kernels.expands(step.past, step.new, window, H, each) else blocks(step)
-        return {f"latent_blocks{size}:{H}:{window}": absorbed,
+        return {self._blocks_name(): attention_kernels.absorbed_rest(size, H, each, window),
                 f"latent_expanded:{H}:{window}": attention_kernels.expanded_work(H, each, window, ops.sm_count(self.runtime.device))}
+
+    def _blocks_name(self) -> str:
+        name = f"latent_blocks{ops.latent_tc_tokens(self.H)}"
+        return name if self.w_kv is None else f"{name}:{self.H}:{int(self.window or 0)}"
 
     def weights(self):
         n, H = self.names, self.H
@@ -142,22 +145,34 @@ class LatentAttention(Mixer):
         if self.expandable and self.tc_heads and tensors[n["uv"]].dtype == torch.bfloat16:
             self.w_kv = linear.LinearWeight(torch.cat([tensors[n["uk"]], tensors[n["uv"]]], dim=0))
 
-    def _expanded(self, q, pages, ctx: StepContext, cache_view, cos, sin):
-        """Attention of a prompt over the keys and values of the positions it sees, expanded here: [T, H dv], or None where the
-        step keeps the absorbed form."""
-        flat = ctx.extra.get(f"latent_expanded:{self.H}:{int(self.window or 0)}")
-        if self.w_kv is None or flat is None or flat.numel() == 0 or q.dtype != torch.bfloat16 or \
-                not ops.latent_attention_tc_takes(pages, cache_view.page_size):
+    def _prompts(self, q, pages, ctx: StepContext, cache_view, cos, sin):
+        """Attention of a step with prompts, [T, H dv]: sequences with enough rows over keys and values expanded here, the rest in the
+        absorbed form; None where no sequence is expanded."""
+        H, window, each = self.H, int(self.window or 0), self.dn + self.dv
+        flat = ctx.extra.get(f"latent_expanded:{H}:{window}")
+        if self.w_kv is None or flat is None or flat.numel() == 0 or not ops.latent_attention_tc_takes(pages, cache_view.page_size):
             return None
-        B = ctx.B
-        n = (flat.numel() - 2 * B - 1) // 7
-        blocks, first_row, lo = flat[:7 * n].view(7, n), flat[7 * n:7 * n + B + 1], flat[7 * n + B + 1:]
+        out = torch.empty((ctx.T, H * self.dv), dtype=self.runtime.act_dtype, device=q.device)
         # Host lists: steps with prompts are never captured (the part stays graph-safe for steps of single tokens).
-        _, rows = attention_kernels.expanded_rows(ctx.h_past, ctx.h_new, int(self.window or 0))
-        c, kr = ops.latent_gather(pages, cache_view.page_table, ctx.slots, first_row, lo, B, sum(rows), self.R, cache_view.page_size)
-        kv = linear.linear(c, self.w_kv, torch.bfloat16)
-        qr = ops.latent_turn(q, cos, sin, ctx.tok_pos, self.H)
-        return ops.latent_prefill(q, qr, kv, kr, blocks, first_row, lo, ctx.kv_len, self.H, self.scale, self.window, self.sinks)
+        turns, B, at = attention_kernels.expanded_turns(ctx.h_past, ctx.h_new, window, H, each), ctx.B, 0
+        rest = sorted(set(range(B)).difference(*turns))
+        if rest:
+            blocks = ctx.extra[self._blocks_name()]
+            T = sum(ctx.h_new[b] for b in rest)
+            blocks, rows = blocks[:blocks.numel() - T], blocks[blocks.numel() - T:].long()
+            those = replace(ctx, T=T, tok_seq=ctx.tok_seq[rows], tok_pos=ctx.tok_pos[rows], max_new=max(ctx.h_new[b] for b in rest),
+                            extra={self._blocks_name(): blocks})
+            out[rows] = self._absorbed(q[rows], pages, those, cache_view, cos, sin)
+        _, lengths = attention_kernels.expanded_rows(ctx.h_past, ctx.h_new, window)
+        qr = ops.latent_turn(q, cos, sin, ctx.tok_pos, H)
+        for turn in turns:
+            n = attention_kernels.expanded_blocks(ctx.h_new, turn)
+            blocks, first_row, lo = flat[at:at + 7 * n].view(7, n), flat[at + 7 * n:at + 7 * n + B + 1], flat[at + 7 * n + B + 1:at + 7 * n + 2 * B + 1]
+            at += 7 * n + 2 * B + 1
+            c, kr = ops.latent_gather(pages, cache_view.page_table, ctx.slots, first_row, lo, B, sum(lengths[b] for b in turn), self.R, cache_view.page_size)
+            kv = linear.linear(c, self.w_kv, torch.bfloat16)
+            ops.latent_prefill(q, qr, kv, kr, blocks, first_row, lo, ctx.kv_len, H, self.scale, self.window, self.sinks, out=out)
+        return out
 
     def _splits(self, ctx: StepContext, blocks_per_token: int, places_per_sm: int = 1) -> int:
         """Slices per row for a step of single tokens: as many as fill the multiprocessors, none shorter than
@@ -179,8 +194,7 @@ class LatentAttention(Mixer):
                 return ops.latent_attention_tc(wide, pages, cache_view.page_table, ctx.slots, H, R, cache_view.page_size,
                                                self.scale, self.window, tok_pos=ctx.tok_pos, tok_seq=ctx.tok_seq,
                                                splits=self._splits(ctx, -(-H // 64) * chunks), **more)
-            name = f"latent_blocks{ops.latent_tc_tokens(H)}"
-            flat = ctx.extra.get(f"{name}:{H}:{int(self.window or 0)}", ctx.extra.get(name))
+            flat = ctx.extra.get(self._blocks_name())
             if flat is not None and flat.numel():
                 return ops.latent_attention_tc(wide, pages, cache_view.page_table, ctx.slots, H, R, cache_view.page_size,
                                                self.scale, self.window, blocks=tuple(flat.view(4, -1)), **more)
@@ -200,7 +214,7 @@ class LatentAttention(Mixer):
         ops.latent_kv_store(down, 0, R, self.g_kv, self.eps, cos, sin, self.rot, ctx.tok_pos, ctx.tok_seq, ctx.slots,
                             cache_view.page_table, pages, R, dr, cache_view.page_size)
         q = linear.linear(cq, self.w_uq, act if self.tc_heads else torch.float32)     # [T, H (dn + dr)]
-        out = None if ctx.decode else self._expanded(q, pages, ctx, cache_view, cos, sin)
+        out = None if ctx.decode else self._prompts(q, pages, ctx, cache_view, cos, sin)
         if out is None:
             out = self._absorbed(q, pages, ctx, cache_view, cos, sin)
         if self.gate is not None:

@@ -71,6 +71,32 @@ def test_expanded_prompts_agree_with_32_bit_and_with_the_absorbed_form(H, window
         assert float((g - w).abs().max()) < 0.06 * float(w.abs().max())
 
 
+@pytest.mark.parametrize("H,window,portions,expanded", [
+    (2, None, [(200, 600, 5), (1, 1, 1), (1, 130, 9)], [1, 0, 1]), (16, None, [(700, 300), (1, 33)], [1, 1]), (3, 90, [(9, 260, 1), (40, 7, 15)], [1, 1])])
+def test_a_step_of_long_and_short_portions_runs_in_both_forms(H, window, portions, expanded):
+    gen = torch.Generator().manual_seed(H)
+    h = [torch.randn(sum(s[i] for s in portions), D, generator=gen).to(torch.bfloat16).to(DEV) for i in range(len(portions[0]))]
+    part, weights = _part(torch.bfloat16, H, window, True)
+    got, routes = _run(part, portions, h)
+    assert routes == expanded
+    want, _ = _run(_part(torch.float32, H, window, True, weights)[0], portions, h)
+    for g, w in zip(got, want):
+        assert float((g - w).norm() / w.norm()) < 3 * 2.0 ** -8 and float((g - w).abs().max()) < 0.06 * float(w.abs().max())
+
+
+def test_sequences_in_turns(monkeypatch):
+    """Buffers that hold two of the four sequences: the same result as all at once, bit for bit."""
+    from longbow_quarrel_b200.kernels import attention as kernels
+    gen = torch.Generator().manual_seed(9)
+    h = [torch.randn(n, D, generator=gen).to(torch.bfloat16).to(DEV) for n in (300, 200, 270, 1)]
+    part, _ = _part(torch.bfloat16, 2, None, False)
+    want, routes = _run(part, [(300, 200, 270, 1)], h)
+    assert routes == [1]
+    monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", 500 * 2 * 256)
+    got, routes = _run(part, [(300, 200, 270, 1)], h)
+    assert routes == [2] and all(torch.equal(g, w) for g, w in zip(got, want))
+
+
 def test_few_queries_per_key_keep_the_absorbed_form():
     gen = torch.Generator().manual_seed(1)
     part, weights = _part(torch.bfloat16, 2, None, False)
