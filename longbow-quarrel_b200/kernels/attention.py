@@ -45,7 +45,10 @@ EXPAND_TILE = 128
 # 236 / 72; 4 heads, 128: 57 / 26, 218 / 75, 120 / 63; 2 heads, 64: 42 / 26, 167 / 75, 82 / 65.  A whole layer of fewer rows is bound by its
 # launches, of which the expanded form has as many.
 EXPAND_QUERIES = 16
-EXPAND_ELEMENTS = 1 << 29          # the most expanded numbers at a time (1 GB in bfloat16): more sequences go in turns, a longer one stays absorbed
+# The most numbers (bfloat16) in a turn's buffers: 256 MB, or what the absorbed form's queries and means would take for the rows of a
+# sequence that is alone in its turn (any prompt without earlier rows has at least as much there).  More sequences go in turns; one
+# that needs more than both, a short portion on a very long past, stays absorbed.
+EXPAND_ELEMENTS = 1 << 27
 
 
 def expanded_rows(past, new, window: int) -> tuple[list[int], list[int]]:
@@ -54,16 +57,16 @@ def expanded_rows(past, new, window: int) -> tuple[list[int], list[int]]:
     return lo, [p + n - a for p, n, a in zip(past, new, lo)]
 
 
-def expanded_turns(past, new, window: int, H: int, per_head: int) -> list[list[int]]:
-    """The sequences of a step whose latent attention runs over expanded keys and values (per_head numbers for each head and key), in
-    turns that share one set of buffers.  Whether a sequence is among them is a matter of its own rows, not of its neighbours."""
+def expanded_turns(past, new, window: int, H: int, per_head: int, R: int) -> list[list[int]]:
+    """The sequences of a step whose latent attention runs over expanded keys and values (per_head numbers for each head and key, next
+    to the key's gathered row of R + 64), in turns that share one set of buffers.  Whether a sequence is among them is a matter of its own rows, not of its neighbours."""
     if max(new) < EXPAND_QUERIES:
         return []
     _, rows = expanded_rows(past, new, window)
     turns, held = [], 0
     for b, (n, r) in enumerate(zip(new, rows)):
-        each = r * H * per_head
-        if n < EXPAND_QUERIES or each > EXPAND_ELEMENTS:
+        each = r * (H * per_head + R + 64)
+        if n < EXPAND_QUERIES or each > max(EXPAND_ELEMENTS, n * H * (2 * (R + 64) + R)):      # float32 queries, bfloat16 means
             continue
         if not turns or held + each > EXPAND_ELEMENTS:
             turns.append([])
@@ -78,14 +81,14 @@ def expanded_blocks(new, turn: list[int]) -> int:
     return sum((-(-new[b] // 128) + 1) // 2 for b in turn)
 
 
-def expanded_work(H: int, per_head: int, window: int, sms: int):
+def expanded_work(H: int, per_head: int, R: int, window: int, sms: int):
     """Builder of lq_latent_prefill's step array.  For every turn: blocks [7, n] (sequence, then first row, rows and first position of
     two chains of at most 128 rows), where every sequence's expanded rows start [B + 1] (no rows for those of other turns), the position
     of its first one [B]; empty for a step without any."""
     def build(step) -> np.ndarray:
         lo, rows = expanded_rows(step.past, step.new, window)
         parts = [np.zeros(0, dtype=np.int32)]
-        for turn in expanded_turns(step.past, step.new, window, H, per_head):
+        for turn in expanded_turns(step.past, step.new, window, H, per_head, R):
             tiles = {b: [(step.cu[b] + r, min(128, step.new[b] - r), step.past[b] + r) for r in range(0, step.new[b], 128)] for b in turn}
             # Chains of neighbouring rows share all their tiles of keys.  A turn whose blocks all run at once is as long as its longest
             # block: there the first rows go with the last ones, so that all blocks have the same work (not under a window, where
@@ -103,13 +106,13 @@ def expanded_work(H: int, per_head: int, window: int, sms: int):
     return build
 
 
-def absorbed_rest(size: int, H: int, per_head: int, window: int):
+def absorbed_rest(size: int, H: int, per_head: int, R: int, window: int):
     """Builder of the absorbed kernel's work list (query_blocks(size)) for the sequences that are not expanded: their blocks, over their
     rows side by side, then which rows of the step these are.  A step without expanded sequences: the blocks alone."""
     every = query_blocks(size)
 
     def build(step) -> np.ndarray:
-        expanded = {b for turn in expanded_turns(step.past, step.new, window, H, per_head) for b in turn}
+        expanded = {b for turn in expanded_turns(step.past, step.new, window, H, per_head, R) for b in turn}
         rest = [b for b in range(step.B) if b not in expanded]
         if not expanded or not rest:
             return every(step).reshape(-1) if rest else np.zeros(0, dtype=np.int32)

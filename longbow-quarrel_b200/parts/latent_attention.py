@@ -86,12 +86,15 @@ class LatentAttention(Mixer):
         if self.w_kv is None:                    # sizes or weights that keep the absorbed form throughout
             return {self._blocks_name(): attention_kernels.query_blocks(size)}
         H, each, window = self.H, self.dn + self.dv, int(self.window or 0)
-        return {self._blocks_name(): attention_kernels.absorbed_rest(size, H, each, window),
-                f"latent_expanded:{H}:{window}": attention_kernels.expanded_work(H, each, window, ops.sm_count(self.runtime.device))}
+        return {self._blocks_name(): attention_kernels.absorbed_rest(size, H, each, self.R, window),
+                self._expanded_name(): attention_kernels.expanded_work(H, each, self.R, window, ops.sm_count(self.runtime.device))}
 
     def _blocks_name(self) -> str:
         name = f"latent_blocks{ops.latent_tc_tokens(self.H)}"
-        return name if self.w_kv is None else f"{name}:{self.H}:{int(self.window or 0)}"
+        return name if self.w_kv is None else f"{name}:{self.H}:{self.R}:{int(self.window or 0)}"
+
+    def _expanded_name(self) -> str:
+        return f"latent_expanded:{self.H}:{self.R}:{int(self.window or 0)}"
 
     def weights(self):
         n, H = self.names, self.H
@@ -144,17 +147,20 @@ class LatentAttention(Mixer):
                          and (self.dn + self.dr) % 8 == 0 and self.R % 8 == 0)
         if self.expandable and self.tc_heads and tensors[n["uv"]].dtype == torch.bfloat16:
             self.w_kv = linear.LinearWeight(torch.cat([tensors[n["uk"]], tensors[n["uv"]]], dim=0))
+            # The same numbers as two of the absorbed form's matrices: held once.
+            self.w_uk = self.w_kv.tensor[:H * self.dn].view(H, self.dn, self.R)
+            self.w_uv_t = self.w_kv.tensor[H * self.dn:].view(H, self.dv, self.R)
 
     def _prompts(self, q, pages, ctx: StepContext, cache_view, cos, sin):
         """Attention of a step with prompts, [T, H dv]: sequences with enough rows over keys and values expanded here, the rest in the
         absorbed form; None where no sequence is expanded."""
         H, window, each = self.H, int(self.window or 0), self.dn + self.dv
-        flat = ctx.extra.get(f"latent_expanded:{H}:{window}")
+        flat = ctx.extra.get(self._expanded_name())
         if self.w_kv is None or flat is None or flat.numel() == 0 or not ops.latent_attention_tc_takes(pages, cache_view.page_size):
             return None
         out = torch.empty((ctx.T, H * self.dv), dtype=self.runtime.act_dtype, device=q.device)
         # Host lists: steps with prompts are never captured (the part stays graph-safe for steps of single tokens).
-        turns, B, at = attention_kernels.expanded_turns(ctx.h_past, ctx.h_new, window, H, each), ctx.B, 0
+        turns, B, at = attention_kernels.expanded_turns(ctx.h_past, ctx.h_new, window, H, each, self.R), ctx.B, 0
         rest = sorted(set(range(B)).difference(*turns))
         if rest:
             blocks = ctx.extra[self._blocks_name()]

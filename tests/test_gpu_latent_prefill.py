@@ -92,7 +92,7 @@ def test_sequences_in_turns(monkeypatch):
     part, _ = _part(torch.bfloat16, 2, None, False)
     want, routes = _run(part, [(300, 200, 270, 1)], h)
     assert routes == [1]
-    monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", 500 * 2 * 256)
+    monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", 500 * (2 * 256 + R + 64))
     got, routes = _run(part, [(300, 200, 270, 1)], h)
     assert routes == [2] and all(torch.equal(g, w) for g, w in zip(got, want))
 

@@ -28,21 +28,35 @@ def _turns(flat, new, turns):
     ((4000,), (10,), 0, []), ((4000,), (100,), 0, [[0]]), ((0, 4000), (200, 1), 0, [[0]]), ((4000, 0), (1, 200), 128, [[1]]),
     ((0, 9, 70, 3), (16, 15, 40, 1), 0, [[0, 2]])])
 def test_a_sequence_expands_by_its_own_rows(past, new, window, expected):
-    assert expanded_turns(past, new, window, 16, 256) == expected
-    assert (len(expanded_work(16, 256, window, 148)(_step(past, new))) > 0) is bool(expected)
+    assert expanded_turns(past, new, window, 16, 256, 512) == expected
+    assert (len(expanded_work(16, 256, 512, window, 148)(_step(past, new))) > 0) is bool(expected)
 
 
-def test_more_than_the_buffers_hold_goes_in_turns_and_a_longer_sequence_stays_absorbed(monkeypatch):
-    monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", 1000 * 2 * 256)
-    assert expanded_turns((0, 0, 0, 0, 900), (400, 600, 1001, 30, 100), 0, 2, 256) == [[0, 1], [3], [4]]
-    assert EXPAND_ELEMENTS >= 16 * 256 * 2048
+def test_more_than_the_buffers_hold_goes_in_turns_and_a_portion_on_a_longer_past_stays_absorbed(monkeypatch):
+    each = 2 * 256 + 64 + 64
+    monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", 1000 * each)
+    assert expanded_turns((0, 0, 970, 0, 900), (400, 600, 31, 30, 100), 0, 2, 256, 64) == [[0, 1], [3], [4]]
+    # A prompt has at least what the absorbed form's queries and means would take, alone in its turn.
+    assert expanded_turns((0, 0, 0), (400, 5000, 300), 0, 2, 256, 64) == [[0], [1], [2]]
+
+
+@pytest.mark.parametrize("H,R", [(2, 64), (16, 512), (32, 512), (128, 512)])
+def test_expanded_buffers_stay_within_what_the_absorbed_form_takes_or_256_mb(H, R):
+    for past, new in [((0,), (100000,)), ((0, 0, 0), (30000, 8000, 16)), ((30000,) * 40, (16,) * 40), ((100000, 500), (512, 9000)), ((10 ** 6,), (100,))]:
+        _, rows = expanded_rows(past, new, 0)
+        for turn in expanded_turns(past, new, 0, H, 256, R):
+            bytes_ = sum(rows[b] * (H * 256 + R + 64) * 2 for b in turn)
+            absorbed = sum(new[b] * H * ((R + 64) * 4 + R * 2) for b in turn)
+            assert bytes_ <= max(256 << 20, absorbed)
+        if past == (0,):
+            assert expanded_turns(past, new, 0, H, 256, R) == [[0]]
 
 
 @pytest.mark.parametrize("past,new", [((0, 4000, 5), (200, 1, 9)), ((7, 0, 30, 2), (3, 40, 15, 100)), ((0, 8), (50, 60)), ((9, 8), (1, 6)), ((100, 3), (1, 30))])
 def test_the_rest_of_a_step_is_listed_for_the_absorbed_form(past, new):
     step, size = _step(past, new), 4
-    flat = absorbed_rest(size, 16, 256, 0)(step)
-    expanded = {b for t in expanded_turns(past, new, 0, 16, 256) for b in t}
+    flat = absorbed_rest(size, 16, 256, 512, 0)(step)
+    expanded = {b for t in expanded_turns(past, new, 0, 16, 256, 512) for b in t}
     rest = [b for b in range(step.B) if b not in expanded]
     if not expanded:
         assert np.array_equal(flat, kernels.query_blocks(size)(step).reshape(-1))
@@ -62,15 +76,15 @@ def test_the_rest_of_a_step_is_listed_for_the_absorbed_form(past, new):
 
 @pytest.mark.parametrize("past,new,window", [((0,), (500,), 0), ((0, 130, 7), (128, 700, 129), 0), ((300,), (1000,), 100), ((90, 1000), (257, 65), 300)])
 @pytest.mark.parametrize("sms", [2, 148])
-@pytest.mark.parametrize("held", [EXPAND_ELEMENTS, 1400 * 2 * 256])
+@pytest.mark.parametrize("held", [EXPAND_ELEMENTS, 1200 * 640])
 def test_every_row_is_in_one_chain_and_every_key_it_sees_among_its_tiles(past, new, window, sms, held, monkeypatch):
     monkeypatch.setattr(kernels, "EXPAND_ELEMENTS", held)
     step = _step(past, new)
     firsts, rows = expanded_rows(past, new, window)
-    turns = expanded_turns(past, new, window, 2, 256)
+    turns = expanded_turns(past, new, window, 2, 256, 64)
     assert sorted(b for t in turns for b in t) == list(range(step.B))
     seen, listed = np.zeros(step.T, dtype=int), []
-    for turn, (blocks, first_row, lo) in zip(turns, _turns(expanded_work(2, 256, window, sms)(step), new, turns)):
+    for turn, (blocks, first_row, lo) in zip(turns, _turns(expanded_work(2, 256, 64, window, sms)(step), new, turns)):
         assert lo.tolist() == firsts and np.diff(first_row).tolist() == [r if b in turn else 0 for b, r in enumerate(rows)]
         assert set(blocks[:, 0]) == set(turn)
         work = [sum((e[k + 2] + e[k + 1]) // 128 + 1 for k in (1, 4) if e[k + 1]) for e in blocks]
