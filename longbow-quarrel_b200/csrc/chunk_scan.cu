@@ -90,6 +90,8 @@ __device__ __forceinline__ void copy4(void* dst, const void* src, bool in) {
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// Whether one of two bfloat16 is an infinity or a NaN.
+__device__ __forceinline__ bool not_finite(uint32_t v) { return (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u; }
 __device__ __forceinline__ float low_f32(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float high_f32(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 // (x, y) as three pairs of bfloat16 whose sums are x and y to 24 bits.
@@ -158,7 +160,8 @@ __global__ void __launch_bounds__(256) chunk_gates_kernel(const __grid_constant_
             const double up = __shfl_up_sync(0xffffffffu, run, o);
             if (lane >= o) run += up;
         }
-        const double F[2] = {run - f[1], run};
+        const double ahead = __shfl_up_sync(0xffffffffu, run, 1);
+        const double F[2] = {(lane ? ahead : 0.0) + f[0], run};         // (not run - f[1]: a NaN at a token stays behind it)
         const double down[2] = {(double)i[0] - F[0], (double)i[1] - F[1]};
         double top = fmax(down[0], down[1]);
 #pragma unroll
@@ -948,6 +951,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     // ---- S_0^T q, then the rows' decays, then the triangle times v
     const int wn = warp % WN, wm = warp / WN, col = wn * 32 + 4 * g;
     float acc[MTB][4][4] = {};
+    int odd = 0;                                   // bit kk: a value of the tokens 16 kk .. is an infinity or a NaN
     float4 sx[2][4];
     auto fetch_s = [&](int kk, float4 (&x)[4]) {
 #pragma unroll
@@ -1007,10 +1011,16 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < 2; ++j)
             ldsm_x4_t(vp + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + wn * 32 + j * 16 + (lane >> 4) * 8, vb[j]);
+        bool odd_v = false;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) odd_v = odd_v || not_finite(vb[j][e]);
+        if (__any_sync(0xffffffffu, odd_v)) odd |= 1 << kk;
 #pragma unroll
         for (int i = 0; i < MTB; ++i) {
             const int mi = i * WM + wm;
-            if (kk > mi) continue;                 // above the diagonal
+            if (kk > mi || (kk == mi && odd >> kk & 1)) continue;      // above the diagonal; see below
             uint32_t pf[3][4];
 #pragma unroll
             for (int p = 0; p < 3; ++p)
@@ -1024,6 +1034,31 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
+        }
+    }
+    // A value that is not finite must not meet the zeros above the diagonal (0 x NaN is NaN, in rows ahead of its token): such blocks
+    // on the diagonal are added up pair by pair.
+    if (odd) {
+#pragma unroll
+        for (int i = 0; i < MTB; ++i) {
+            const int mi = i * WM + wm;
+            if (!(odd >> mi & 1)) continue;
+#pragma unroll 1
+            for (int s = 0; s < 16; ++s)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int tt = mi * 16 + g + e * 8;
+                    if (s > g + e * 8) continue;
+                    float p = 0.f;
+#pragma unroll
+                    for (int x = 2; x >= 0; --x) p += __bfloat162float(pp[((size_t)x * CC + tt) * LP + mi * 16 + s]);
+                    const bf* v = vp + (size_t)(mi * 16 + s) * LV + wn * 32 + 2 * t;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[i][j][2 * e] = fmaf(p, __bfloat162float(v[8 * j]), acc[i][j][2 * e]);
+                        acc[i][j][2 * e + 1] = fmaf(p, __bfloat162float(v[8 * j + 1]), acc[i][j][2 * e + 1]);
+                    }
+                }
         }
     }
     // ---- out

@@ -28,11 +28,16 @@ def _scan64(q, k, v, a, b, S):
     return torch.stack(out), S
 
 
-def _case(kind, lens, H, dk, dv, pad=0, seed=0):
-    """A step's rows, the call's options and the float64 result."""
+def _case(kind, lens, H, dk, dv, pad=0, seed=0, spoil=None):
+    """A step's rows, the call's options and the float64 result.  spoil = (row, what): a number of that row that is not finite."""
+    bad = lambda what: spoil is not None and spoil[1] == what
     gen = torch.Generator().manual_seed(seed + dk * dv)
     T, X = sum(lens), int(kind == "mlstm")
     x = torch.randn(T, 2 * H * dk + H * dv + pad, generator=gen).to(torch.bfloat16)
+    if bad("v"):
+        x[spoil[0], 2 * H * dk + 3] = float("inf")
+    if bad("k"):
+        x[spoil[0], H * dk + 3] = float("nan")
     slots = [2 * i + 1 for i in range(len(lens))][::-1]
     state = torch.randn(2 * len(lens) + 1, H, dk + X, dv + X, generator=gen)
     pos = np.concatenate([np.arange(n) + 3 * i for i, n in enumerate(lens)])
@@ -54,6 +59,8 @@ def _case(kind, lens, H, dk, dv, pad=0, seed=0):
         cap = 8.0
         pre, bias = torch.randn(T, 2 * H, generator=gen) * 2 * cap, torch.randn(2 * H, generator=gen)
         pre[T // 2:T // 2 + 5, H:] = -4 * cap                 # forget nearly everything
+        if bad("gate") or bad("forget"):
+            pre[spoil[0], 1 if bad("gate") else H + 1] = float("nan")
         opts["gates"] = (pre.to(DEV), bias.to(DEV), cap)
         g = pre.double() + bias.double()
         li, lf = cap * torch.tanh(g[:, :H] / cap), torch.nn.functional.logsigmoid(cap * torch.tanh(g[:, H:] / cap))
@@ -64,6 +71,8 @@ def _case(kind, lens, H, dk, dv, pad=0, seed=0):
         pre[T // 3:T // 3 + 3] = -60.0
         bias, tau = torch.randn(H * dk, generator=gen) * 2, 2.0
         bias[::5], bias[1::7] = 60.0, -12.0
+        if bad("decay"):
+            pre[spoil[0], 5] = float("nan")
         dev = torch.zeros(T, H * dk + 3, device=DEV)
         dev[:, 1:1 + H * dk] = pre.to(DEV)
         opts["channel_decay"] = (dev[:, 1:1 + H * dk], bias.to(DEV), tau)
@@ -78,7 +87,7 @@ def _case(kind, lens, H, dk, dv, pad=0, seed=0):
         if kind == "mlstm":
             m, aa, bb = S[:, dk, 0], [], []
             for t in range(row, row + n):
-                m, old = torch.maximum(lf[t] + m, li[t]), m
+                m, old = (torch.fmax if bad("gate") else torch.maximum)(lf[t] + m, li[t]), m      # the kernels' maxima pass a NaN gate over
                 aa.append(torch.exp(lf[t] + old - m)[:, None])
                 bb.append(torch.exp(li[t] - m)[:, None])
             o, S = _scan64(q[rows], k[rows], v[rows], torch.stack(aa), torch.stack(bb), S[:, :dk])
@@ -141,3 +150,25 @@ def test_other_sizes_keep_the_walk_by_tokens(why, lens, H, dk, dv, pad):
     got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
     assert chunks == 0
     _check(got, st, want, finals, state, slots)
+
+
+@pytest.mark.parametrize("kind,what", [("plain", "v"), ("plain", "k"), ("rotated", "v"), ("mlstm", "v"), ("mlstm", "gate"), ("mlstm", "forget"), ("channels", "v"),
+                                       ("channels", "decay"), ("channels", "k")])
+@pytest.mark.parametrize("dk,dv,row", [(64, 64, 0), (64, 64, 13), (128, 128, 63), (64, 128, 85), (128, 64, 190)])
+def test_a_number_that_is_not_finite_spoils_only_later_tokens(kind, what, dk, dv, row, monkeypatch):
+    """A NaN (an infinity as a value) at one token of the first of two sequences: the same numbers are finite as in the recurrence, and those that
+    are agree with it."""
+    ops = _ops()
+    monkeypatch.setattr(ops, "CHUNK_SCAN_ROWS_CHANNELS", ops.CHUNK_SCAN_ROWS)
+    lens, H = [200, 70], 2
+    x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv, spoil=(row, what))
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    assert chunks == 1
+    fine = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), fine) and not fine[row:200].all() and fine[:row].all() and fine[200:].all()
+    assert float((got - want)[fine].abs().max()) < TOL * float(want[fine].abs().max())
+    for slot, S in zip(slots, finals):
+        fine = torch.isfinite(S)
+        assert torch.equal(torch.isfinite(st[slot]), fine)
+        if fine.any():
+            assert float((st[slot].double() - S)[fine].abs().max()) < TOL * float(S[fine].abs().max())
