@@ -63,6 +63,7 @@ struct ChunkArgs {
     float* prep;                 // VEC, scratch [places][H][vec_floats(dk)]: see prepare
     int H, dk, dv, ld, B;
     int first, places;           // the chunk places that this set of launches works on
+    int fewest;                  // sequences of fewer rows are walked token by token (recurrent.cu): left out here
 };
 
 // Where the chunks of sequence b lie: unique and never overlapping, whatever the sequences' lengths are.
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(256) chunk_gates_kernel(const __grid_constant_
     pdl_wait();
     const int row0 = a.cu_rows[b], row1 = a.cu_rows[b + 1], base = first_place(a.cu_rows, b);
     const int c_lo = max(0, a.first - base), c_hi = min((row1 - row0 + CC - 1) / CC, a.first + a.places - base);
-    if (c_lo >= c_hi) return;
+    if (c_lo >= c_hi || row1 - row0 < a.fewest) return;
     float m = a.state[(long long)a.slots[b] * a.slot_stride + ((size_t)h * (a.dk + 1) + a.dk) * (a.dv + 1)];
     const float cap = a.gate_cap, bias_i = a.gate_bias[h], bias_f = a.gate_bias[H + h];
     for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) chunk_prepare_kernel(const __
         else hi = mid - 1;
     }
     const int row = a.cu_rows[lo] + (place - first_place(a.cu_rows, lo)) * CC, n = min(CC, a.cu_rows[lo + 1] - row);
-    if (n <= 0) return;
+    if (n <= 0 || a.cu_rows[lo + 1] - a.cu_rows[lo] < a.fewest) return;
     float* kw = a.prep + ((size_t)blockIdx.x * H + h) * vec_floats(dk);
     float* qw = kw + CC * dk;
     float* tri = qw + CC * dk;
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
     pdl_wait();
     const int row0 = a.cu_rows[b], row1 = a.cu_rows[b + 1], base = first_place(a.cu_rows, b);
     const int c_lo = max(0, a.first - base), c_hi = min((row1 - row0 + CC - 1) / CC, a.first + a.places - base);
-    if (c_lo >= c_hi) return;
+    if (c_lo >= c_hi || row1 - row0 < a.fewest) return;
     float* st = a.state + (long long)a.slots[b] * a.slot_stride + (size_t)h * (dk + X) * (dv + X);
     const GateRecord* gates = reinterpret_cast<const GateRecord*>(a.gates) + (ptrdiff_t)(base - a.first) * H + h;     // chunk c's: gates[c * H]
     const float* prep = a.prep + ((ptrdiff_t)(base - a.first) * H + h) * vec_floats(dk);       // chunk c's: prep + c * H * vec_floats
@@ -752,7 +753,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
         else hi = mid - 1;
     }
     const int row = a.cu_rows[lo] + (place - first_place(a.cu_rows, lo)) * CC, n = min(CC, a.cu_rows[lo + 1] - row);
-    if (n <= 0) return;
+    if (n <= 0 || a.cu_rows[lo + 1] - a.cu_rows[lo] < a.fewest) return;
     const float* s0 = a.s0 + ((size_t)blockIdx.x * H + h) * dk * a.ld;
 
     // ---- q (which 0) or k (1) of the tokens s_lo .. s_lo + count - 1, split where they are rotated
@@ -1154,11 +1155,12 @@ LQ_EXPORT long long lq_chunk_place_floats(int H, int dk, int dv, int kind) {
 
 // As lq_linear_scan for steps with prompts in bfloat16: dk and dv multiples of 8 up to 128, offsets and stride in whole eights;
 // with a fixed decay, rotation over whole heads (dk a multiple of 16) or none.  `places` chunks of scratch are worked on at a time.
+// Sequences of fewer than `fewest` rows are left out (their rows of out and exp_neg_m and their state stay as they are).
 LQ_EXPORT int lq_chunk_scan(const void* qkv, int stride, int q_off, int k_off, int v_off, const float* cos_t, const float* sin_t,
                             const int* tok_pos, const float* gate_pre, const float* gate_bias, float gate_cap, const float* decay,
                             const float* decay_pre, int decay_stride, const float* decay_bias, float inv_tau, float q_scale,
                             float k_scale, float* state, long long slot_stride, const int* cu_rows, const int* slots, float* out,
-                            float* exp_neg_m, float* scratch, int places, int rows, int B, int H, int dk, int dv, cudaStream_t stream) {
+                            float* exp_neg_m, float* scratch, int places, int rows, int fewest, int B, int H, int dk, int dv, cudaStream_t stream) {
     if (B <= 0 || rows <= 0) return LQ_OK;
     const bool gated = gate_pre != nullptr;
     if (dk < 8 || dv < 8 || dk > 128 || dv > 128 || dk % 8 || dv % 8 || places < 1) return LQ_BAD_SIZE;
@@ -1168,7 +1170,7 @@ LQ_EXPORT int lq_chunk_scan(const void* qkv, int stride, int q_off, int k_off, i
     if (gated ? (!gate_bias || !exp_neg_m || decay_pre) : (!decay && !decay_pre)) return LQ_BAD_SIZE;
     ChunkArgs a{(const bf*)qkv, stride, q_off, k_off, v_off, cos_t, sin_t, tok_pos, gate_pre, gate_bias, gate_cap, decay, q_scale, k_scale,
                 state, slot_stride, cu_rows, slots, out, exp_neg_m, scratch, nullptr, decay_pre, decay_stride, decay_bias, inv_tau, nullptr,
-                H, dk, dv, (dv + 31) / 32 * 32 + (gated ? 4 : 0), B, 0, 0};
+                H, dk, dv, (dv + 31) / 32 * 32 + (gated ? 4 : 0), B, 0, 0, fewest};
     a.gates = a.prep = scratch + (size_t)places * H * dk * a.ld;      // 16-byte aligned: dk and ld are whole eights and fours
     const int all = rows / CC + B;
     for (a.first = 0; a.first < all; a.first += places) {

@@ -11,9 +11,10 @@
 //
 // State, products and gates are float32 whatever the activations' storage is; q and k are rotated (optionally)
 // and scaled in float32 as they are staged, so nothing that enters the recurrence is rounded on the way.
-// A sequence's tokens are walked in order from the state that the step before left in the sequence's slot, so a
-// prompt gives the same bits however it is cut into portions; steps of one token per sequence have a form of
-// their own (the same recurrence, sums in another order).
+// A sequence's tokens are walked in order from the state that the step before left in the sequence's slot, so what this
+// kernel makes of a prompt has the same bits however it is cut into portions; steps of one token per sequence have a form of
+// their own (the same recurrence, sums in another order), and so have longer portions in bfloat16 (chunk_scan.cu).  Which form a
+// sequence takes is a matter of its own rows, not of the sequences beside it.
 #include "common.cuh"
 #include <math_constants.h>
 
@@ -48,6 +49,7 @@ struct ScanArgs {
     int decay_stride;
     const float* decay_bias;     // channel decays: [H * dk] or null
     float inv_tau;               // channel decays: a = exp(logsigmoid(pre + bias) * inv_tau)
+    int most;                    // sequences of more rows run by chunks (chunk_scan.cu): left out here (0: none)
 };
 
 __device__ __forceinline__ float scan_in(float x, int act) { return act ? x / (1.f + expf(-x)) : x; }
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(SC_THREADS) linear_scan_kernel(ScanArgs a) {
     constexpr int RF = (KR + 1) / 2;             // a thread's share of a chunk's rotated pairs
     pdl_wait();
     const int row0 = a.cu_rows[b], row1 = a.cu_rows[b + 1];
+    if (a.most && row1 - row0 > a.most) return;
     float m = 0.f;
     float q_pf[KR], k_pf[KR], d_pf[VEC ? KR : 1], cs_pf[RF], sn_pf[RF], v_pf = 0.f, gi_pf = 0.f, gf_pf = 0.f;
     // Element e of a chunk's q (k) is token e / dk, dimension e % dk; thread tid holds e = tid + i * THREADS.
@@ -399,7 +402,7 @@ LQ_EXPORT int lq_linear_scan(const void* qkv, int dtype, int stride, int q_off, 
                              const float* gate_bias, float gate_cap, const float* decay, float q_scale, float k_scale,
                              float* state, long long slot_stride, const int* cu_rows, const int* slots, float* out,
                              float* exp_neg_m, int B, int H, int dk, int dv, int mlstm, int single, int in_act,
-                             const float* decay_pre, int decay_stride, const float* decay_bias, float inv_tau,
+                             const float* decay_pre, int decay_stride, const float* decay_bias, float inv_tau, int most,
                              cudaStream_t stream) {
     if (B <= 0) return LQ_OK;
     if (in_act < 0 || in_act > 1) return LQ_BAD_SIZE;
@@ -408,7 +411,7 @@ LQ_EXPORT int lq_linear_scan(const void* qkv, int dtype, int stride, int q_off, 
     if (mlstm ? (!gate_pre || !gate_bias || !exp_neg_m || vec) : (!decay && !vec)) return LQ_BAD_SIZE;
     ScanArgs a{qkv, stride, q_off, k_off, v_off, cos_t, sin_t, rot, tok_pos, gate_pre, gate_bias, gate_cap, decay,
                q_scale, k_scale, state, slot_stride, cu_rows, slots, out, exp_neg_m, H, dk, dv, in_act,
-               decay_pre, decay_stride, decay_bias, inv_tau};
+               decay_pre, decay_stride, decay_bias, inv_tau, most};
     typedef __nv_bfloat16 bf;
     if (dtype != LQ_F32 && dtype != LQ_BF16) return LQ_BAD_DTYPE;
     const bool f32 = dtype == LQ_F32;

@@ -1013,26 +1013,33 @@ def moe_down(u: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, weights: 
 
 
 # ------------------------------------------------------------------ mixers with a matrix state per head
-# Rows a sequence, on average, from which the scan runs by chunks: its two or three launches pay from one whole chunk on (32 heads
-# of 64 / of 128, one sequence, us by tokens and by chunks: 32 rows 11.5 / 22 and 16 / 24, 64 rows 19 / 39 and 18 / 26, 256 rows
-# 67 / 136 and 23 / 37).  With decays per key channel a third launch prepares every chunk: 128 rows (26 / 88 and 27 / 52).
+# Rows of a sequence from which it is scanned by chunks: their two or three launches pay from one whole chunk on (32 heads of 32 / of 64 /
+# of 128, one sequence, us by tokens and by chunks: 64 rows 20 13 / 25 17 / 49 28, 256 rows 56 17 / 78 19 / 164 32; with gates 64 rows
+# 20 26 / 37 26 / 56 40, 96 rows 27 26 / 51 27 / 78 42).  With decays per key channel a third launch prepares every chunk: 128 rows
+# 33 38 / 41 42 / 111 70, 192 rows 44 40 / 57 44 / 161 73.  Heads of up to 48, whose chunks are padded to 64 channels, wait half as
+# long again with either.
 CHUNK_SCAN_ROWS = 64
 CHUNK_SCAN_ROWS_CHANNELS = 128
 CHUNK_SCRATCH_FLOATS = 1 << 27        # the most scratch that the scan by chunks takes at a time (512 MB); longer steps run in turns
 
 
-def _scan_takes_chunks(qkv: torch.Tensor, offsets: tuple, fewest: int, dk: int, dv: int, turns: bool, cos, sin, dims: int) -> bool:
-    """Whether lq_chunk_scan takes a step's rows (sizes, types and alignment; turns: a form that it also takes rotated) and is the
-    faster kernel for them."""
-    return (qkv.dtype == torch.bfloat16 and qkv.shape[0] >= fewest and dk % 8 == 0 and dv % 8 == 0 and dk <= 128 and dv <= 128
+def _scan_takes_chunks(qkv: torch.Tensor, offsets: tuple, dk: int, dv: int, turns: bool, cos, sin, dims: int) -> bool:
+    """Whether lq_chunk_scan takes a step's rows: sizes, types and alignment (turns: a form that it also takes rotated)."""
+    return (qkv.dtype == torch.bfloat16 and dk % 8 == 0 and dv % 8 == 0 and dk <= 128 and dv <= 128
             and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and all(o % 8 == 0 for o in offsets)
             and (not dims or (turns and dims == dk and dk % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (cos, sin)))))
+
+
+def chunk_scan_rows(dk: int, gates: bool, channels: bool) -> int:
+    """Rows of a sequence from which the scan by chunks is the faster one."""
+    rows = CHUNK_SCAN_ROWS_CHANNELS if channels else CHUNK_SCAN_ROWS
+    return rows * 3 // 2 if (gates or channels) and dk <= 48 else rows
 
 
 def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_rows, slots, tok_pos,
                 B: int, H: int, dk: int, dv: int, q_scale: float = 1.0, k_scale: float = 1.0,
                 decay: torch.Tensor | None = None, gates: tuple | None = None, rot: tuple | None = None,
-                single: bool = False, in_act: str | None = None, channel_decay: tuple | None = None):
+                single: bool = False, in_act: str | None = None, channel_decay: tuple | None = None, lens: list | None = None):
     """S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t for the rows of B sequences (rows cu_rows[b] ..
     cu_rows[b+1] of qkv belong to the sequence in slot slots[b]), from and into `state` (float32
     [slots, H, dk (+1), dv (+1)]).  decay: float32 [H] (a_t fixed, b_t = 1).  gates = (pre [rows, 2H] float32,
@@ -1043,6 +1050,8 @@ def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: to
     they are read.  channel_decay = (pre, bias, tau): a decay for every key channel and token instead of one per head,
     a_t[h, r] = sigmoid(pre[t, h * dk + r] + bias[h * dk + r])^(1 / tau), the rows of the state that belong to channel r
     decaying by it; pre is a float32 [rows, H * dk] view (rows may be strided), bias float32 [H * dk] or None.
+    Long sequences in bfloat16 run by chunks (csrc/chunk_scan.cu), the others token by token; lens, the sequences' rows on the host,
+    spares the launches for a kind that the step has none of.
     Returns the raw outputs float32 [rows, H, dv (+1)] and, with gates, exp(-maximum) float32 [rows, H]."""
     rows = qkv.shape[0]
     mlstm = gates is not None
@@ -1069,9 +1078,11 @@ def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: to
     if decay is not None and (decay.dtype != torch.float32 or decay.numel() != H):
         raise KernelError("linear_scan: decay must be float32 [H]")
     cos, sin, dims = rot if rot is not None else (None, None, 0)
-    if in_act is None and not (single and rows == B) and \
-            _scan_takes_chunks(qkv, (q_off, k_off, v_off), B * (CHUNK_SCAN_ROWS if d_pre is None else CHUNK_SCAN_ROWS_CHANNELS),
-                               dk, dv, decay is not None, cos, sin, dims):
+    most = 0                         # rows of the longest sequence that is left to the walk by tokens (0: all are)
+    fewest = chunk_scan_rows(dk, mlstm, d_pre is not None)
+    longest, shortest = (max(lens), min(lens)) if lens else (rows, rows if B == 1 else 0)
+    if in_act is None and not (single and rows == B) and longest >= fewest and \
+            _scan_takes_chunks(qkv, (q_off, k_off, v_off), dk, dv, decay is not None, cos, sin, dims):
         count = build.load("chunk_scan").lq_chunk_place_floats
         count.argtypes, count.restype = [c_int] * 4, c_longlong
         kind = 1 if mlstm else 2 if d_pre is not None else 0
@@ -1080,21 +1091,23 @@ def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: to
         scratch = torch.empty(places * each, dtype=torch.float32, device=qkv.device)
         fn = _fn("chunk_scan", "lq_chunk_scan", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                  c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_float, c_void_p, c_longlong,
-                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
         _check(fn(_p(qkv), qkv.stride(0), q_off, k_off, v_off, _p(cos), _p(sin), _p(tok_pos), _p(pre), _p(bias), float(cap), _p(decay),
                   _p(d_pre), d_pre.stride(0) if d_pre is not None else 0, _p(d_bias), 1.0 / float(tau), float(q_scale), float(k_scale), _p(state),
-                  state.stride(0), _p(cu_rows), _p(slots), _p(out), _p(enm), _p(scratch), places, rows, B, H, dk, dv, _stream()),
+                  state.stride(0), _p(cu_rows), _p(slots), _p(out), _p(enm), _p(scratch), places, rows, fewest, B, H, dk, dv, _stream()),
                "linear_scan", (3 if kind else 2) * -(-(rows // 64 + B) // places), "linear_scan:chunks")
-        return out, enm
+        if shortest >= fewest:
+            return out, enm
+        most = fewest - 1
     fn = _fn("recurrent", "lq_linear_scan", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                                              c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_float, c_float, c_void_p,
                                              c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                             c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p])
+                                             c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_int, c_void_p])
     _check(fn(_p(qkv), dtype_code(qkv), qkv.stride(0), q_off, k_off, v_off, _p(cos), _p(sin), int(dims), _p(tok_pos),
               _p(pre), _p(bias), float(cap), _p(decay), float(q_scale), float(k_scale), _p(state), state.stride(0),
               _p(cu_rows), _p(slots), _p(out), _p(enm), B, H, dk, dv, int(mlstm), int(single and rows == B),
               {None: 0, "silu": 1}[in_act], _p(d_pre), d_pre.stride(0) if d_pre is not None else 0, _p(d_bias), 1.0 / float(tau),
-              _stream()),
+              most, _stream()),
            "linear_scan", 1, "linear_scan:single" if single and rows == B else None)
     return out, enm
 

@@ -30,7 +30,7 @@ Gates, decays, the state and the per-head norms are 32-bit in both precisions; t
 gates' pre-activations come from a 32-bit product of their own.  A sequence's tokens
 are walked in order from the state in its slot (`csrc/recurrent.cu`: one kernel for
 prompts and portions, one for steps of a single token per sequence), so a position's
-result does not depend on how its prompt was cut, beyond rounding.  (In bfloat16, prompts of "retention", "mlstm" and
+result does not depend on how its prompt was cut, beyond rounding.  (In bfloat16, sequences that bring many rows to "retention", "mlstm" and
 "channel_decay" run by chunks of 64 tokens on the tensor cores, `csrc/chunk_scan.cu`; "lightning" walks prompts by records of
 four tokens, `csrc/delta.cu`.)
 """
@@ -108,7 +108,7 @@ class Retention(_MatrixStateMixer):
             cos, sin = self.position.tables()
             rot = (cos, sin, self.position.rotary_dims)
         raw, _ = ops.linear_scan(rows, 0, H * dk, 2 * H * dk, cache_view, ctx.cu_rows, ctx.slots, ctx.tok_pos, ctx.B,
-                                 H, dk, dv, k_scale=dk ** -0.5, decay=self.decay, rot=rot, single=ctx.decode)
+                                 H, dk, dv, k_scale=dk ** -0.5, decay=self.decay, rot=rot, single=ctx.decode, lens=ctx.h_new)
         g_off = 2 * H * dk + H * dv
         out = ops.head_norm_gate(raw, dv, self.eps, self.runtime.act_dtype, gate=rows[:, g_off:g_off + H * dv], act="silu")
         return self._finish(out, residual)
@@ -186,7 +186,8 @@ class MLSTM(_MatrixStateMixer):
         rows = linear.linear(h, self.w_in, self.runtime.act_dtype)
         pre = ops.small_proj(h, self.w_gates)         # the gates enter the recurrence: a 32-bit product of their own
         raw, enm = ops.linear_scan(rows, 0, H * dk, 2 * H * dk, cache_view, ctx.cu_rows, ctx.slots, ctx.tok_pos, ctx.B,
-                                   H, dk, dv, q_scale=dk ** -0.5, gates=(pre, self.b_gates, self.cap), single=ctx.decode)
+                                   H, dk, dv, q_scale=dk ** -0.5, gates=(pre, self.b_gates, self.cap), single=ctx.decode,
+                                   lens=ctx.h_new)
         g_off = 2 * H * dk + H * dv
         out = ops.head_norm_gate(raw, dv, self.eps, self.runtime.act_dtype, exp_neg_m=enm, weight=self.head_weight,
                                  gate=rows[:, g_off:g_off + H * dv], act="sigmoid")
@@ -232,7 +233,8 @@ class ChannelDecay(_MatrixStateMixer):
         # product, so that nothing between the first product's sums and the decay itself is rounded.
         pre = ops.gemm_plain(linear.linear(h, self.w_a1, torch.float32), self.w_a2, torch.float32)
         raw, _ = ops.linear_scan(rows, 0, H * dk, 2 * H * dk, cache_view, ctx.cu_rows, ctx.slots, ctx.tok_pos, ctx.B,
-                                 H, dk, dv, q_scale=dk ** -0.5, channel_decay=(pre, self.b_a2, self.tau), single=ctx.decode)
+                                 H, dk, dv, q_scale=dk ** -0.5, channel_decay=(pre, self.b_a2, self.tau), single=ctx.decode,
+                                 lens=ctx.h_new)
         g_off = 2 * H * dk + H * dv
         out = ops.head_norm_gate(raw, dv, self.eps, self.runtime.act_dtype, weight=self.head_weight,
                                  gate=rows[:, g_off:g_off + H * dv], act="silu")

@@ -100,11 +100,11 @@ def _case(kind, lens, H, dk, dv, pad=0, seed=0, spoil=None):
     return x, state, slots, pos, opts, torch.cat(outs), finals
 
 
-def _run(ops, x, state, slots, lens, pos, opts, H, dk, dv):
+def _run(ops, x, state, slots, lens, pos, opts, H, dk, dv, **more):
     before = ops.launches_by_name().get("linear_scan:chunks", 0)
     st = state.to(DEV).contiguous()
     out, enm = ops.linear_scan(x.to(DEV), 0, H * dk, 2 * H * dk, st, _i32(np.concatenate([[0], np.cumsum(lens)])), _i32(slots), _i32(pos),
-                               len(lens), H, dk, dv, **opts)
+                               len(lens), H, dk, dv, **opts, **more)
     return out.cpu().double(), st.cpu(), ops.launches_by_name().get("linear_scan:chunks", 0) - before
 
 
@@ -134,7 +134,7 @@ def test_chunks_follow_the_recurrence(kind, lens, H, dk, dv, monkeypatch):
 def test_scratch_for_a_part_of_the_chunks(kind, monkeypatch):
     """The chunks in turns of two places: the state goes on from turn to turn through its slot."""
     ops = _ops()
-    lens, H, dk, dv = [200, 70, 130], 2, 64, 32         # 133 rows a sequence
+    lens, H, dk, dv = [200, 128, 130], 2, 64, 32
     x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv)
     monkeypatch.setattr(ops, "CHUNK_SCRATCH_FLOATS", 2 * ops.build.load("chunk_scan").lq_chunk_place_floats(H, dk, dv, {"plain": 0, "mlstm": 1, "channels": 2}[kind]))
     got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
@@ -172,3 +172,32 @@ def test_a_number_that_is_not_finite_spoils_only_later_tokens(kind, what, dk, dv
         assert torch.equal(torch.isfinite(st[slot]), fine)
         if fine.any():
             assert float((st[slot].double() - S)[fine].abs().max()) < TOL * float(S[fine].abs().max())
+
+
+@pytest.mark.parametrize("kind", ["plain", "rotated", "mlstm", "channels"])
+@pytest.mark.parametrize("lens", [[400] + [1] * 7, [1, 63, 200, 5], [20, 30], [95, 97, 191, 193]])
+@pytest.mark.parametrize("dk", [64, 32])
+def test_a_sequence_takes_its_form_by_its_own_rows(kind, lens, dk):
+    """Long sequences by chunks and short ones token by token in one step, whether the host knows their lengths or not; every sequence has
+    the bits that it has alone."""
+    ops = _ops()
+    H, dv = 2, 64
+    fewest = ops.chunk_scan_rows(dk, kind == "mlstm", kind == "channels")
+    x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv)
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv, lens=lens)
+    assert chunks == int(max(lens) >= fewest)
+    _check(got, st, want, finals, state, slots)
+    blind, st2, _ = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    assert torch.equal(blind, got) and torch.equal(st2, st)
+    row = 0
+    for n, slot in zip(lens, slots):
+        rows = slice(row, row + n)
+        own = dict(opts)
+        if kind == "mlstm":
+            own["gates"] = (opts["gates"][0][rows].contiguous(), *opts["gates"][1:])
+        if kind == "channels":
+            own["channel_decay"] = (opts["channel_decay"][0][rows], *opts["channel_decay"][1:])
+        alone, st3, chunks = _run(ops, x[rows], state, [slot], [n], pos[rows], own, H, dk, dv, lens=[n])
+        assert chunks == int(n >= fewest)
+        assert torch.equal(alone, got[rows]) and torch.equal(st3[slot], st[slot])
+        row += n
