@@ -719,7 +719,8 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
 // ------------------------------------------------------------------ output
 // Four warps: first 16 rows of the chunk's triangle each, then 32 value columns and 16 MTB rows of the output each.  The state
 // goes from global memory straight into the products' fragments; shared memory holds q, v, and k and then the triangle in one
-// place, so that three blocks share a multiprocessor (two where q and k are rotated heads of 128, whose k comes in two halves).
+// place, so that three blocks share a multiprocessor, or two where q is three terms of 128 channels (rotated, and then k comes in two
+// halves, or with decays per channel).
 template <int DK, int DV, Mode MODE, bool ROT>
 struct OutSizes {
     static constexpr int NQ = ROT || MODE == VEC ? 3 : 1;     // rotated q and k, and q with its decays, are float32: three terms
@@ -727,7 +728,9 @@ struct OutSizes {
     static constexpr int HALVES = ROT && DK == 128 ? 2 : 1;
     static constexpr size_t q = (size_t)NQ * CC * LK * sizeof(bf), k = MODE == VEC ? 0 : q / HALVES, p = (size_t)3 * CC * LP * sizeof(bf);
     static constexpr size_t v = (size_t)CC * LV * sizeof(bf), rows_out = MODE == GATED ? (size_t)CC * (DV + 4) * sizeof(float) : 0;
-    static constexpr size_t work = q + v + (HALVES == 1 ? (k > p ? k : p) : k + p), bytes = work > rows_out ? work : rows_out;
+    static constexpr size_t work = q + v + (k > p ? k : p), bytes = work > rows_out ? work : rows_out;
+    static constexpr int BLOCKS = DK == 128 && NQ == 3 ? 2 : 3;
+    static_assert(BLOCKS * (bytes + 2560 + 1024) <= 228 * 1024, "blocks of a multiprocessor, with their static and reserved shared memory");
 };
 
 template <int DK, int DV, Mode MODE, bool ROT>
@@ -740,7 +743,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     bf* qp = reinterpret_cast<bf*>(smem);          // [NQ][CC][LK]
     bf* vp = qp + Z::q / sizeof(bf);               // [CC][LV]
     bf* kp = vp + Z::v / sizeof(bf);               // [NQ][HC][LK]
-    bf* pp = HALVES == 1 ? kp : kp + Z::k / sizeof(bf);    // [3][CC][LP]
+    bf* pp = kp;                                   // [3][CC][LP], once k has been read
     __shared__ float pw[CC + 1], f_row[CC], n_row[CC], n_part[2][CC], n0[DK];
     __shared__ double up[CC], down[CC];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -916,7 +919,7 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
                 }
             }
         }
-        if (HALVES == 1) __syncthreads();          // k has been read: the triangle takes its place
+        __syncthreads();                           // k has been read: the triangle takes its place
         const float scale = a.q_scale * a.k_scale;
         float sums[2] = {0.f, 0.f};
 #pragma unroll
