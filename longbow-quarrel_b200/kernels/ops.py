@@ -1020,7 +1020,7 @@ def moe_down(u: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, weights: 
 # long again with either.
 CHUNK_SCAN_ROWS = 64
 CHUNK_SCAN_ROWS_CHANNELS = 128
-CHUNK_SCRATCH_FLOATS = 1 << 27        # the most scratch that the scan by chunks takes at a time (512 MB); longer steps run in turns
+CHUNK_SCRATCH_FLOATS = 1 << 26        # the most scratch that the scan by chunks takes at a time (256 MB); longer steps run in turns
 
 
 def _scan_takes_chunks(qkv: torch.Tensor, offsets: tuple, dk: int, dv: int, turns: bool, cos, sin, dims: int) -> bool:
@@ -1034,6 +1034,16 @@ def chunk_scan_rows(dk: int, gates: bool, channels: bool) -> int:
     """Rows of a sequence from which the scan by chunks is the faster one."""
     rows = CHUNK_SCAN_ROWS_CHANNELS if channels else CHUNK_SCAN_ROWS
     return rows * 3 // 2 if (gates or channels) and dk <= 48 else rows
+
+
+def _chunk_scratch(places: int, each: int, device) -> tuple:
+    """(scratch for as many of `places` chunks as there is memory for, that many); (None, 0) where there is none for one."""
+    while places:
+        try:
+            return torch.empty(places * each, dtype=torch.float32, device=device), places
+        except torch.cuda.OutOfMemoryError:
+            places //= 2
+    return None, 0
 
 
 def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_rows, slots, tok_pos,
@@ -1087,8 +1097,10 @@ def linear_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, state: to
         count.argtypes, count.restype = [c_int] * 4, c_longlong
         kind = 1 if mlstm else 2 if d_pre is not None else 0
         each = count(H, dk, dv, kind)
-        places = max(1, min(rows // 64 + B, CHUNK_SCRATCH_FLOATS // each))
-        scratch = torch.empty(places * each, dtype=torch.float32, device=qkv.device)
+        scratch, places = _chunk_scratch(max(1, min(rows // 64 + B, CHUNK_SCRATCH_FLOATS // each)), each, qkv.device)
+    else:
+        places = 0
+    if places:
         fn = _fn("chunk_scan", "lq_chunk_scan", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                  c_float, c_void_p, c_void_p, c_int, c_void_p, c_float, c_float, c_float, c_void_p, c_longlong,
                                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])

@@ -154,6 +154,14 @@ class LatentAttention(Mixer):
     def _prompts(self, q, pages, ctx: StepContext, cache_view, cos, sin):
         """Attention of a step with prompts, [T, H dv]: sequences with enough rows over keys and values expanded here, the rest in the
         absorbed form; None where no sequence is expanded."""
+        try:
+            return self._in_both_forms(q, pages, ctx, cache_view, cos, sin)
+        except torch.cuda.OutOfMemoryError:
+            pass                                 # (what was allocated goes back as the exception does)
+        # No room for the expansion: the absorbed form, row by row (the step's work list has the rest alone).
+        return self._absorbed(q, pages, replace(ctx, extra={}), cache_view, cos, sin)
+
+    def _in_both_forms(self, q, pages, ctx: StepContext, cache_view, cos, sin):
         H, window, each = self.H, int(self.window or 0), self.dn + self.dv
         flat = ctx.extra.get(self._expanded_name())
         if self.w_kv is None or flat is None or flat.numel() == 0 or not ops.latent_attention_tc_takes(pages, cache_view.page_size):

@@ -142,6 +142,29 @@ def test_scratch_for_a_part_of_the_chunks(kind, monkeypatch):
     _check(got, st, want, finals, state, slots)
 
 
+@pytest.mark.parametrize("kind", ["plain", "channels"])
+@pytest.mark.parametrize("room", [3, 0])
+def test_no_memory_for_the_scratch(kind, room, monkeypatch):
+    """Room for three of the step's chunks: in turns, with the same bits.  For none: token by token."""
+    ops = _ops()
+    lens, H, dk, dv = [300, 140], 2, 64, 64
+    x, state, slots, pos, opts, want, finals = _case(kind, lens, H, dk, dv)
+    full, st_full, _ = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    most = room * ops.build.load("chunk_scan").lq_chunk_place_floats(H, dk, dv, {"plain": 0, "channels": 2}[kind])
+    empty = torch.empty
+
+    def limited(*size, **kw):
+        if kw.get("dtype") == torch.float32 and size and isinstance(size[0], int) and size[0] > most:
+            raise torch.cuda.OutOfMemoryError("test")
+        return empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", limited)
+    got, st, chunks = _run(ops, x, state, slots, lens, pos, opts, H, dk, dv)
+    monkeypatch.undo()
+    assert chunks == int(room > 0)
+    _check(got, st, want, finals, state, slots)
+    assert not room or (torch.equal(got, full) and torch.equal(st, st_full))
+
+
 @pytest.mark.parametrize("why,lens,H,dk,dv,pad", [("few rows", [63], 2, 64, 64, 0), ("odd head", [100], 2, 24, 20, 0), ("odd stride", [100], 2, 16, 16, 3),
                                                   ("a head of 136", [100], 1, 136, 16, 0)])
 def test_other_sizes_keep_the_walk_by_tokens(why, lens, H, dk, dv, pad):

@@ -97,6 +97,22 @@ def test_sequences_in_turns(monkeypatch):
     assert routes == [2] and all(torch.equal(g, w) for g, w in zip(got, want))
 
 
+def test_no_memory_for_the_expansion(monkeypatch):
+    from longbow_quarrel_b200.kernels import ops
+    gen = torch.Generator().manual_seed(4)
+    h = [torch.randn(n, D, generator=gen).to(torch.bfloat16).to(DEV) for n in (200, 3)]
+    part, weights = _part(torch.bfloat16, 2, None, True)
+
+    def full(*args):
+        raise torch.cuda.OutOfMemoryError("test")
+    monkeypatch.setattr(ops, "latent_gather", full)
+    got, routes = _run(part, [(200, 3)], h)
+    assert routes == [0]
+    want, _ = _run(_part(torch.float32, 2, None, True, weights)[0], [(200, 3)], h)
+    for g, w in zip(got, want):
+        assert float((g - w).norm() / w.norm()) < 3 * 2.0 ** -8
+
+
 def test_few_queries_per_key_keep_the_absorbed_form():
     gen = torch.Generator().manual_seed(1)
     part, weights = _part(torch.bfloat16, 2, None, False)
