@@ -1467,10 +1467,9 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
                        const float* __restrict__ slope) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float sm[];
-    float* qs = sm;              // [hd]
-    float* sc = sm + hd;         // [ATT_CHUNK]
-    int* at = (int*)(sc + ATT_CHUNK);  // [ATT_CHUNK] where each key of the chunk lies, in rows of the pages
+    extern __shared__ long long at[];  // [ATT_CHUNK] where each key of the chunk lies, in rows of the pages (which may be 2^31 and more)
+    float* qs = (float*)(at + ATT_CHUNK);  // [hd]
+    float* sc = qs + hd;         // [ATT_CHUNK]
     const bool vec = hd % 4 == 0 && (uintptr_t)k_pages % (4 * sizeof(T)) == 0;
     int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     int pos = tok_pos[t];
@@ -1490,9 +1489,9 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
         float s = -CUDART_INF_F;
         if (tid < n) {
             int key = vbase + tid < head ? vbase + tid : start + (vbase + tid - head);
-            const int row = (pt[key / page_size] * Hkv + kvh) * page_size + key % page_size;
+            const long long row = ((long long)pt[key / page_size] * Hkv + kvh) * page_size + key % page_size;
             at[tid] = row;
-            const T* kr = k_pages + (size_t)row * hd;
+            const T* kr = k_pages + row * hd;
             float d = 0.f;
             if (vec) {
 #pragma unroll 8
@@ -1528,7 +1527,7 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
             if (d >= vd) break;
             float a = 0.f;
 #pragma unroll 16
-            for (int j = 0; j < n; ++j) a = fmaf(sc[j], to_f32(v_pages[(size_t)at[j] * vd + d]), a);
+            for (int j = 0; j < n; ++j) a = fmaf(sc[j], to_f32(v_pages[at[j] * vd + d]), a);
             if (rep == 0) acc0 = acc0 * corr + a; else acc1 = acc1 * corr + a;
         }
         m = cm;
@@ -1569,7 +1568,7 @@ LQ_EXPORT int lq_attention_plain(const void* q, int q_stride, int dtype, const v
     if (vd <= 0) vd = hd;
     if (vd > 2 * ATT_CHUNK || H % Hkv) return LQ_BAD_SIZE;
     dim3 grid(T, H);
-    size_t smem = (hd + 2 * ATT_CHUNK) * sizeof(float);
+    size_t smem = ATT_CHUNK * sizeof(long long) + (hd + ATT_CHUNK) * sizeof(float);
     if (dtype == LQ_F32)
         return launch_pdl(attention_plain_kernel<float, float>, grid, dim3(ATT_CHUNK), smem, stream, (const float*)q, q_stride, (const float*)k_pages,
             (const float*)v_pages, page_table, pt_stride, tok_pos, tok_seq, slots, (float*)out, H, Hkv, hd, page_size, scale, window,
