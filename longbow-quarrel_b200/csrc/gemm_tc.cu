@@ -87,7 +87,8 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&r)[32], void* Cout,
         return;
     }
     const bool whole = n + 32 <= n_lim;
-    if (EPI == EPI_BF16 || EPI == EPI_ACT) {
+    static_assert(EPI != EPI_ACT, "sums leave through an activation by staged stores only");
+    if (EPI == EPI_BF16) {
         __nv_bfloat16* dst = (__nv_bfloat16*)Cout + (size_t)m * N + n;
         if (whole && (N & 7) == 0) {
             uint4* d4 = reinterpret_cast<uint4*>(dst);
@@ -276,7 +277,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                              (splits > 1 ? range * plane_rows : 0) + m0 + quarter * 32, n0, N, lane, qkv.glu_limit,
                                              qkv.act);
                 }
-            } else {
+            } else if constexpr (EPI != EPI_ACT) {      // (which has staged stores only: see launch_epi)
 #pragma unroll 1
                 for (int c = 0; c < (BN + 31) / 32; ++c) {      // a last half chunk reads columns that are not stored
                     uint32_t r[32];

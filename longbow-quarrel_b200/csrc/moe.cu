@@ -109,18 +109,6 @@ LQ_EXPORT int lq_moe_route(const float* z, int z_stride, int* ids, float* weight
                       weights, T, E, groups, keep, top, route_scale, score_fn, correction, group_rule, normalize);
 }
 
-// act: 0 none, 1 gelu (erf), 2 gelu (tanh form), 3 silu, 4 relu, 5 the square of relu
-__device__ __forceinline__ float moe_act(float v, int act) {
-    switch (act) {
-        case 1: return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-        case 2: return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-        case 3: return v / (1.f + expf(-v));
-        case 4: return fmaxf(v, 0.f);
-        case 5: { const float r = fmaxf(v, 0.f); return r * r; }
-        default: return v;
-    }
-}
-
 // sum_k x[k] * w[k] over a row of n numbers, by one warp (x float32 in shared memory).  bfloat16 rows whose length is a
 // multiple of 8 are read 16 bytes a lane at a time (rows then start on 16-byte boundaries), two loads in flight.
 // (The lane's share of the sum: the caller adds the lanes with warp_sum, once for all that it has to add.)
@@ -195,7 +183,7 @@ __global__ void __launch_bounds__(MX_WARPS * 32) moe_up_kernel(const T* __restri
         const float s = warp_sum(part[i]);
         const float up = gated ? warp_sum(part_up[i]) : 1.f;
         // gated: the activated gate is rounded as a product's output would be before it meets the up value
-        if (lane == 0 && f < F) u[(size_t)pair * F + f] = from_f32<T>(gated ? moe_act(s, act) * up : moe_act(s, act));
+        if (lane == 0 && f < F) u[(size_t)pair * F + f] = from_f32<T>(gated ? lq_expert_act(s, act) * up : lq_expert_act(s, act));
     }
 }
 
@@ -320,7 +308,7 @@ __global__ void __launch_bounds__(MX_WARPS * 32, 4) moe_up_rows_kernel(const __n
     for (int i = 0; i < OUT; ++i) {
         const int f = (blockIdx.y * OUT + i) * MX_WARPS + warp;
         const float s = warp_sum(part[i]), up = GATED ? warp_sum(part[R - OUT + i]) : 1.f;
-        if (lane == 0 && f < F) u[(size_t)pair * F + f] = __float2bfloat16_rn(GATED ? moe_act(s, act) * up : moe_act(s, act));
+        if (lane == 0 && f < F) u[(size_t)pair * F + f] = __float2bfloat16_rn(GATED ? lq_expert_act(s, act) * up : lq_expert_act(s, act));
     }
 }
 
