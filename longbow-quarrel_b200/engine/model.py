@@ -110,9 +110,10 @@ class Model:
         seen, total = set(), 0
         for _, part in self._named_parts():
             for t in _tensors_of(part):
-                if t.data_ptr() not in seen:
-                    seen.add(t.data_ptr())
-                    total += t.numel() * t.element_size()
+                memory = t.untyped_storage()         # matrices that are views of one another are held once
+                if memory.data_ptr() not in seen:
+                    seen.add(memory.data_ptr())
+                    total += memory.nbytes()
         return total
 
     # ------------------------------------------------------------------ forward

@@ -104,3 +104,19 @@ def test_every_row_is_in_one_chain_and_every_key_it_sees_among_its_tiles(past, n
         if len(spans) == 2:                    # the tiles that a block walks have no gap
             assert max(s[0] for s in spans) <= min(s[1] for s in spans)
     assert (seen == 1).all()
+
+
+def test_matrices_that_are_views_of_one_another_are_weighed_once():
+    import torch
+
+    from longbow_quarrel_b200.engine.model import Model
+
+    class Part:
+        def __init__(self):
+            self.both = torch.zeros(6, 4)
+            self.first, self.second, self.other = self.both[:2].view(1, 2, 4), self.both[2:], torch.zeros(3, dtype=torch.bfloat16)
+
+    model = object.__new__(Model)
+    part = Part()
+    model._named_parts = lambda: [("a", part), ("b", part)]
+    assert model.weight_bytes() == 6 * 4 * 4 + 3 * 2
