@@ -1116,7 +1116,7 @@ int launch_state(const ChunkArgs& a, cudaStream_t stream) {
         return launch_pdl(kernel, dim3(a.B, a.H, (a.dv + cols - 1) / cols), dim3(STATE_THREADS), smem, stream, a);
     };
     // 32 columns a block read the keys' terms least often; 16 where that leaves more than half of the multiprocessors idle.
-    if ((long long)a.B * a.H * ((a.dv + 31) / 32) > 74) return go(chunk_state_kernel<DK, 4, MODE, ROT>, 32, StateSizes<DK, 4, MODE, ROT>::bytes);
+    if ((long long)a.B * a.H * ((a.dv + 31) / 32) * 2 > lq_sm_count()) return go(chunk_state_kernel<DK, 4, MODE, ROT>, 32, StateSizes<DK, 4, MODE, ROT>::bytes);
     return go(chunk_state_kernel<DK, 2, MODE, ROT>, 16, StateSizes<DK, 2, MODE, ROT>::bytes);
 }
 

@@ -27,6 +27,14 @@ static inline int lq_launch_status() {
     return e == cudaSuccess ? LQ_OK : (int)e;
 }
 
+// Multiprocessors of the current device.
+static inline int lq_sm_count() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+}
+
 // The first key that a row at position p sees under a mask given as one integer: w > 0, a sliding window of the
 // last w positions; w < 0, the row's own block of -w positions (blocks are counted from the sequence's first
 // position); 0, every earlier position.  It never decreases as p grows.

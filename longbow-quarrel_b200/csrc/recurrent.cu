@@ -758,7 +758,7 @@ static int small_proj_bf16(const __nv_bfloat16* x, const __nv_bfloat16* w, float
     };
     // Few rows: as many warps as possible; many: as many products from every number that is read and unpacked.
     if (rows <= 2) return go(small_proj_bf16_kernel<2, 1>, 2, 1);
-    if ((long long)((rows + 3) / 4) * ((N + 3) / 4) < 148 * 4) return go(small_proj_bf16_kernel<4, 1>, 4, 1);
+    if ((long long)((rows + 3) / 4) * ((N + 3) / 4) < 4 * lq_sm_count()) return go(small_proj_bf16_kernel<4, 1>, 4, 1);
     return go(small_proj_bf16_kernel<4, 4>, 4, 4);
 }
 
