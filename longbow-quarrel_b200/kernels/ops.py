@@ -154,17 +154,13 @@ def _contig(t: torch.Tensor, what: str) -> torch.Tensor:
     return t
 
 
-# Libraries that take some of another one's calls in bfloat16: they are set up together.
-_BESIDE = {"recurrent": ("chunk_scan",)}
-
-
 def prepare(dtype: torch.dtype, verbose: bool = True, extra: tuple = ()) -> None:
     """Build and load the libraries a model of this dtype uses, before the first step.  extra: libraries
     that parts of the model name beyond the common ones (`Part.kernel_libraries`)."""
     from concurrent.futures import ThreadPoolExecutor
     names = ["plain_kernels", *extra]
     if dtype == torch.bfloat16:
-        names += ["gemm_skinny", "gemm_tc", "gemm_pair", *(b for n in extra for b in _BESIDE.get(n, ()))]
+        names += ["gemm_skinny", "gemm_tc", "gemm_pair"]
     names = [n for n in dict.fromkeys(names) if not build.loaded(n)]
     if not names:
         return

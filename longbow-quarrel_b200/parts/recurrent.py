@@ -38,7 +38,7 @@ from __future__ import annotations
 
 import torch
 
-from ..kernels import linear, ops
+from ..kernels import build, linear, ops
 from ..weights.spec import WeightSpec
 from .base import Mixer, Runtime, StateNeed, StepContext
 from .registry import make_part, register_part
@@ -72,6 +72,11 @@ class _MatrixStateMixer(Mixer):
         self.w_in = linear.LinearWeight(torch.cat(rows, dim=0))       # q, k, v and the gate in one product
         self.w_o = linear.LinearWeight(tensors[n["o"]])
 
+    def _load_scan(self):
+        """What ops.linear_scan runs long sequences with, made ready before the first step."""
+        if self.runtime.dtype == torch.bfloat16 and self.w_in.tensor.is_cuda:
+            build.load("chunk_scan")
+
     def _finish(self, out, residual):
         if residual is None:
             return linear.linear(out, self.w_o, torch.float32)
@@ -98,6 +103,7 @@ class Retention(_MatrixStateMixer):
 
     def load(self, tensors):
         self._load_base(tensors)
+        self._load_scan()
         self.decay = torch.tensor(self.decay_values, dtype=torch.float32, device=self.runtime.device)
 
     def forward(self, h, ctx: StepContext, cache_view, residual, writes_cache: bool = True):
@@ -176,6 +182,7 @@ class MLSTM(_MatrixStateMixer):
 
     def load(self, tensors):
         self._load_base(tensors)
+        self._load_scan()
         n = self.names
         self.w_gates = torch.cat([tensors[n["i"]], tensors[n["f"]]], dim=0).contiguous()
         self.b_gates = torch.cat([tensors[n["i_bias"]], tensors[n["f_bias"]]]).to(torch.float32).contiguous()
@@ -218,6 +225,7 @@ class ChannelDecay(_MatrixStateMixer):
 
     def load(self, tensors):
         self._load_base(tensors)
+        self._load_scan()
         n = self.names
         self.w_a1, self.w_a2 = linear.LinearWeight(tensors[n["a1"]]), tensors[n["a2"]].contiguous()
         if self.w_a1.N != self.w_a2.shape[1]:
