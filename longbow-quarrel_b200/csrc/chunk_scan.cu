@@ -91,8 +91,6 @@ __device__ __forceinline__ void copy4(void* dst, const void* src, bool in) {
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// Whether one of two bfloat16 is an infinity or a NaN.
-__device__ __forceinline__ bool not_finite(uint32_t v) { return (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u; }
 __device__ __forceinline__ float low_f32(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float high_f32(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 // (x, y) as three pairs of bfloat16 whose sums are x and y to 24 bits.
@@ -955,7 +953,6 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     // ---- S_0^T q, then the rows' decays, then the triangle times v
     const int wn = warp % WN, wm = warp / WN, col = wn * 32 + 4 * g;
     float acc[MTB][4][4] = {};
-    int odd = 0;                                   // bit kk: a value of the tokens 16 kk .. is an infinity or a NaN
     float4 sx[2][4];
     auto fetch_s = [&](int kk, float4 (&x)[4]) {
 #pragma unroll
@@ -967,7 +964,16 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
     fetch_s(0, sx[0]);
     fetch_s(1, sx[1]);
     copy_wait<0>();
-    __syncthreads();
+    // Whether a value of the chunk is an infinity or a NaN: times zero it leaves a NaN in what is added up over this thread's copies.
+    __nv_bfloat162 zeros = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int j = tid; j < CC * (DV / 8); j += 128) {
+        const uint4 v4 = *reinterpret_cast<const uint4*>(vp + j / (DV / 8) * LV + (j % (DV / 8)) * 8);
+        const __nv_bfloat162* v2 = reinterpret_cast<const __nv_bfloat162*>(&v4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) zeros = __hfma2(v2[e], __floats2bfloat162_rn(0.f, 0.f), zeros);
+    }
+    const int odd = __syncthreads_or((*reinterpret_cast<const uint32_t*>(&zeros) & 0x7fff7fffu) != 0);
 #pragma unroll 2
     for (int kk = 0; kk < DK / 16; ++kk) {
         uint32_t sb[3][4][2];
@@ -1015,16 +1021,10 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < 2; ++j)
             ldsm_x4_t(vp + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + wn * 32 + j * 16 + (lane >> 4) * 8, vb[j]);
-        bool odd_v = false;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) odd_v = odd_v || not_finite(vb[j][e]);
-        if (__any_sync(0xffffffffu, odd_v)) odd |= 1 << kk;
 #pragma unroll
         for (int i = 0; i < MTB; ++i) {
             const int mi = i * WM + wm;
-            if (kk > mi || (kk == mi && odd >> kk & 1)) continue;      // above the diagonal; see below
+            if (kk > mi || (kk == mi && odd)) continue;      // above the diagonal; see below
             uint32_t pf[3][4];
 #pragma unroll
             for (int p = 0; p < 3; ++p)
@@ -1040,13 +1040,12 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
                 for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
         }
     }
-    // A value that is not finite must not meet the zeros above the diagonal (0 x NaN is NaN, in rows ahead of its token): such blocks
-    // on the diagonal are added up pair by pair.
+    // A value that is not finite must not meet the zeros above the diagonal (0 x NaN is NaN, in rows ahead of its token): the
+    // blocks on the diagonal of such a chunk are added up pair by pair.
     if (odd) {
 #pragma unroll
         for (int i = 0; i < MTB; ++i) {
             const int mi = i * WM + wm;
-            if (!(odd >> mi & 1)) continue;
 #pragma unroll 1
             for (int s = 0; s < 16; ++s)
 #pragma unroll
