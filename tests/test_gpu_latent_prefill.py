@@ -52,7 +52,8 @@ def _run(part, portions, h):
 
 @pytest.mark.parametrize("H,window,sink,portions", [
     (2, None, False, [(128,)]), (3, None, True, [(129, 257, 40)]), (2, None, False, [(300, 0), (70, 511), (33, 100)]), (1, 100, True, [(450, 130), (200, 64)]),
-    (2, 300, False, [(700,), (129,)]), (16, None, False, [(1100,)])])
+    (2, 300, False, [(700,), (129,)]), (16, None, False, [(1100,)]),
+    (16, None, True, [(1300, 1290)])])           # the last: more blocks than multiprocessors, whose chains are neighbours (2 i, 2 i + 1)
 def test_expanded_prompts_agree_with_32_bit_and_with_the_absorbed_form(H, window, sink, portions, monkeypatch):
     from longbow_quarrel_b200.kernels import attention as kernels
     gen = torch.Generator().manual_seed(H)
@@ -66,8 +67,9 @@ def test_expanded_prompts_agree_with_32_bit_and_with_the_absorbed_form(H, window
     want, _ = _run(_part(torch.float32, H, window, sink, weights)[0], portions, h)
     for g, a, w in zip(got, absorbed, want):
         err, other = float((g - w).norm() / w.norm()), float((a - w).norm() / w.norm())
-        # Both forms round three tensors to bfloat16 on the way (2^-9 each at most, at random); neither may lose against the other.
-        assert err < 3 * 2.0 ** -8 and err < 1.25 * other + 1e-4, (err, other)
+        # Both forms round three tensors to bfloat16 on the way (2^-9 each at most, at random); neither may lose against the other (of
+        # the attention alone, over 2 to 32 heads and latents of 64 to 512, their distances from 64 bits differ by 4 % at most, either way).
+        assert err < 3 * 2.0 ** -8 and err < 1.1 * other, (err, other)
         assert float((g - w).abs().max()) < 0.06 * float(w.abs().max())
 
 
