@@ -1467,7 +1467,8 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
                        const float* __restrict__ slope) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ long long at[];  // [ATT_CHUNK] where each key of the chunk lies, in rows of the pages (which may be 2^31 and more)
+    extern __shared__ __align__(16) uint8_t sm[];
+    const T** at = (const T**)sm;          // [ATT_CHUNK] each key's values
     float* qs = (float*)(at + ATT_CHUNK);  // [hd]
     float* sc = qs + hd;         // [ATT_CHUNK]
     const bool vec = hd % 4 == 0 && (uintptr_t)k_pages % (4 * sizeof(T)) == 0;
@@ -1490,7 +1491,7 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
         if (tid < n) {
             int key = vbase + tid < head ? vbase + tid : start + (vbase + tid - head);
             const long long row = ((long long)pt[key / page_size] * Hkv + kvh) * page_size + key % page_size;
-            at[tid] = row;
+            at[tid] = v_pages + row * vd;
             const T* kr = k_pages + row * hd;
             float d = 0.f;
             if (vec) {
@@ -1527,7 +1528,7 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
             if (d >= vd) break;
             float a = 0.f;
 #pragma unroll 16
-            for (int j = 0; j < n; ++j) a = fmaf(sc[j], to_f32(v_pages[at[j] * vd + d]), a);
+            for (int j = 0; j < n; ++j) a = fmaf(sc[j], to_f32(at[j][d]), a);
             if (rep == 0) acc0 = acc0 * corr + a; else acc1 = acc1 * corr + a;
         }
         m = cm;
@@ -1568,7 +1569,7 @@ LQ_EXPORT int lq_attention_plain(const void* q, int q_stride, int dtype, const v
     if (vd <= 0) vd = hd;
     if (vd > 2 * ATT_CHUNK || H % Hkv) return LQ_BAD_SIZE;
     dim3 grid(T, H);
-    size_t smem = ATT_CHUNK * sizeof(long long) + (hd + ATT_CHUNK) * sizeof(float);
+    size_t smem = ATT_CHUNK * sizeof(void*) + (hd + ATT_CHUNK) * sizeof(float);
     if (dtype == LQ_F32)
         return launch_pdl(attention_plain_kernel<float, float>, grid, dim3(ATT_CHUNK), smem, stream, (const float*)q, q_stride, (const float*)k_pages,
             (const float*)v_pages, page_table, pt_stride, tok_pos, tok_seq, slots, (float*)out, H, Hkv, hd, page_size, scale, window,
