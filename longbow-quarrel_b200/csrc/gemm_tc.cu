@@ -149,11 +149,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // is the float32-store one and Cout the scratch [splits, plane_rows, N] (plane_rows: M rounded up to 32, so
     // that a warp's box of 32 rows stays inside its range's plane).
     const int total = m_tiles * n_tiles * splits;
-    // Row tiles of one column of tiles by turns: neighbours read the same weights.  Grouped: the columns of one row tile by turns, so that
-    // the blocks at work share few groups' rows and weights, each read from memory once, and the tiles without a group lie behind
-    // all others (12,288 rows in 64 groups, 2,048 x 1,408 with gelu and 1,408 x 2,048: 119 and 94 us, 137 and 127 a column at a time).
-    const auto m_of = [&](int tile) { return tile_group ? tile / n_tiles : tile % m_tiles; };
-    const auto n_of = [&](int tile) { return tile_group ? tile % n_tiles : tile / m_tiles; };
+    // Row tiles of one column of tiles by turns: neighbours read the same weights.  Grouped: the columns of one row tile by turns, or
+    // (by_group: see lq_gemm_tc_grouped) group by group, the neighbouring row tiles of a group by columns; tiles without a group
+    // are left out by all roles.
+    struct Walk { int first = 0, end = 0; };       // neighbouring row tiles of the group that a role was at last
+    struct Place { int m, n, group; };
+    const auto place_of = [&](int tile, Walk& w) -> Place {
+        if (!tile_group) return {tile % m_tiles, tile / m_tiles, 0};
+        const int at = tile / n_tiles, group = tile_group[at];
+        if (group < 0 || !qkv.by_group) return {at, tile % n_tiles, group};
+        if (at < w.first || at >= w.end) {
+            w.first = at;
+            w.end = at + 1;
+            while (w.first > 0 && tile_group[w.first - 1] == group) --w.first;
+            while (w.end < m_tiles && tile_group[w.end] == group) ++w.end;
+        }
+        const int local = tile - w.first * n_tiles, rows = w.end - w.first;
+        return {w.first + local % rows, local / rows, group};
+    };
     const int n_kb = (K + BK - 1) / BK;
     constexpr uint32_t STAGE_BYTES = (AROWS + BN) * BK * 2;
     constexpr uint32_t ACC_COLS = BN <= 128 ? 128 : 256;   // columns of tensor memory per accumulator (BN of them used)
@@ -182,12 +195,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
+            Walk walk;
             for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x) {
                 const int tile = piece / splits, range = piece % splits;
-                const int m0 = m_of(tile) * BM, n0 = n_of(tile) * BN;
-                // Grouped products: the rows of a tile all belong to one group, whose weight is rows
-                // group * N .. of W; a tile without a group (padding behind the last one) is left out by all roles.
-                const int group = tile_group ? tile_group[m_of(tile)] : 0;
+                // Grouped products: the rows of a tile all belong to one group, whose weight is rows group * N .. of W.
+                const auto [mt, nt, group] = place_of(tile, walk);
+                const int m0 = mt * BM, n0 = nt * BN;
                 if (group < 0) continue;
                 const int kb_lo = (int)((long)n_kb * range / splits), kb_hi = (int)((long)n_kb * (range + 1) / splits);
                 for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
@@ -214,8 +227,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             constexpr uint32_t idesc = idesc_bf16(BM, BN, false);
             uint32_t it = 0, t = 0;
             bool ok = true;
+            Walk walk;
             for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x, ++t) {
-                if (tile_group && tile_group[m_of(piece / splits)] < 0) { --t; continue; }
+                if (place_of(piece / splits, walk).group < 0) { --t; continue; }
                 const int range = piece % splits;
                 const int kb_lo = (int)((long)n_kb * range / splits), kb_hi = (int)((long)n_kb * (range + 1) / splits);
                 const uint32_t acc = t & 1;
@@ -242,10 +256,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         uint32_t t = 0;
         int stage_buf = 0;
         bool ok = true;
+        Walk walk;
         for (int piece = blockIdx.x; piece < total && ok; piece += gridDim.x, ++t) {
             const int tile = piece / splits, range = piece % splits;
-            if (tile_group && tile_group[m_of(tile)] < 0) { --t; continue; }
-            const int m0 = m_of(tile) * BM, n0 = n_of(tile) * BN;
+            const auto [mt, nt, group] = place_of(tile, walk);
+            if (group < 0) { --t; continue; }
+            const int m0 = mt * BM, n0 = nt * BN;
             void* dst = splits > 1 ? (void*)((float*)Cout + (size_t)range * plane_rows * N) : Cout;
             const uint32_t acc = t & 1;
             const int m = m0 + quarter * 32 + lane;
@@ -577,14 +593,21 @@ LQ_EXPORT int lq_gemm_tc_grouped(const void* A, const void* W, void* C, int out_
     if (rc != LQ_OK) return rc;
     rc = make_map(&mb, W, G * N, K, 256);
     if (rc != LQ_OK) return rc;
-    if (out_f32 == 2) return launch_epi<256, 4, EPI_SWIGLU, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, QkvArgs{}, stream, tile_group);
+    QkvArgs more{};
+    // Row tile by row tile a group's weights are read once for every row tile that is not at work beside another of its group; group by
+    // group they are read once.  Long contractions gain by that; short ones with the gated epilogue lose by blocks that work in step.
+    // us, gated first product / second one, by row tiles and by groups: 8 groups of 512 rows, 4,096 x 14,336: 1,181 846 / 427 387;
+    // 4 such: 610 420 / 197 197; 8 of 512, 3,072 x 8,192: 485 438 / 182 178; 16 of 256, 4,096 x 6,400: 541 455 / 252 244;
+    // 64 of 192, 4,096 x 2,048: 520 490, 2,048 x 1,408: 248 288 / 105 106; 16 of 512, 2,048 x 8,192: 688 740 / 240 238; 8 of 512,
+    // 2,048 x 5,632: 212 256 / 94 92.  (By columns over all row tiles: 905 / 503, 513 / 281, 420 / 234, 563 / 295, 701, 322 / 140, 792 / 318, 238 / 127.)
+    more.by_group = K >= 3072;
+    if (out_f32 == 2) return launch_epi<256, 4, EPI_SWIGLU, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, more, stream, tile_group);
     if (out_f32 > 2) {
-        QkvArgs more{};
         more.act = out_f32 - 2;
         return launch_epi<256, 4, EPI_ACT, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, more, stream, tile_group);
     }
-    if (out_f32) return launch_epi<256, 4, EPI_F32, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, QkvArgs{}, stream, tile_group);
-    return launch_epi<256, 4, EPI_BF16, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, QkvArgs{}, stream, tile_group);
+    if (out_f32) return launch_epi<256, 4, EPI_F32, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, more, stream, tile_group);
+    return launch_epi<256, 4, EPI_BF16, BM>(ma, mb, C, nullptr, M, N, K, sm_count(), 1, more, stream, tile_group);
 }
 
 LQ_EXPORT int lq_gemm_tc_splits(int M, int N, int K) {

@@ -119,6 +119,7 @@ struct QkvArgs {
     int pt_stride, H, Hkv, hd, page_size;
     float glu_limit;          // EPI_SWIGLU: see Glu
     int act;                  // EPI_ACT: see lq_expert_act
+    int by_group;             // grouped products: the order of their tiles
 };
 
 // Where elements j .. of head `head` of row m go: q_out, or the row's place in a cache page.

@@ -79,3 +79,20 @@ def test_a_grouped_product_behind_an_activation(act, T, E, D, F):
     # half a unit of bfloat16, and a few float32 roundings of the factor (1 + erf or tanh), which cancels for negative sums
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 16 * 2.0 ** -24 * sums.abs()).all())
     ops.check_status()
+
+
+@pytest.mark.parametrize("groups", [[0], [0, 0, 0, -1], [1, 1, 2, 2, 2, 3, -1, -1], [3, 3, 0, 0, 0, -1, 3, 1, -1, 1], list(range(5)) * 2 + [4] * 160])
+@pytest.mark.parametrize("N,K", [(8, 64), (600, 72), (8, 3072), (600, 3080)])      # tiles by row tiles, then by groups
+def test_grouped_products_walk_every_tile_once_in_whatever_order_the_groups_come(groups, N, K):
+    """One to three columns of tiles, runs of one group and groups that come back; more tiles than multiprocessors.  Integers small enough
+    that every sum is exact."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(len(groups))
+    a = torch.randint(-3, 4, (len(groups) * 128, K), generator=g).to(torch.bfloat16).to(DEV)
+    w = torch.randint(-3, 4, (5, N, K), generator=g).to(torch.bfloat16).to(DEV)
+    tiles = torch.tensor(groups, dtype=torch.int32, device=DEV)
+    got = ops.gemm_tc_grouped(a, w, tiles, torch.float32).view(len(groups), 128, N)
+    for i, group in enumerate(groups):
+        if group >= 0:
+            assert torch.equal(got[i], (a[i * 128:(i + 1) * 128].float() @ w[group].float().T))
+    ops.check_status()
