@@ -14,9 +14,9 @@
 //   output  a block per (chunk, head), all at once
 // The state kernel is bound by what a block does per chunk (its products where heads are of 128, its stagers' copies of cosines
 // and sines where they are rotated), the output kernel by the latencies of eight to twelve warps a multiprocessor (tensor cores
-// busy a quarter of the time).  2,048 tokens of 32 heads, both kernels (and gates), us: heads of 64 rotated 491 token by token
-// (recurrent.cu), 75 here; with gates 731 and 87; with decays per key channel 397 and 157; heads of
-// 128: 1,165 and 236, 1,264 and 160, 1,915 and 333 (of which prepare 147: exponentials and logarithms, then the halves' sums).
+// busy a third of the time).  2,048 tokens of 32 heads, both kernels (and gates), us: heads of 64 rotated 491 token by token
+// (recurrent.cu), 87 here (50 not rotated); with gates 731 and 87; with decays per key channel 397 and 157; heads of
+// 128: 1,165 and 195, 1,264 and 160, 1,915 and 333 (of which prepare 147: exponentials and logarithms, then the halves' sums).
 //
 // Precision: what the recurrence holds in 32 bits stays so.  A float32 operand enters the products as three bfloat16 terms
 // (its 24 bits), a pair of such operands as the six products that reach 2^-24; bfloat16 operands enter as they are.  The
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(STATE_THREADS, 1) chunk_state_kernel(const __g
 // Four warps: first 16 rows of the chunk's triangle each, then 32 value columns and 16 MTB rows of the output each.  The state
 // goes from global memory straight into the products' fragments; shared memory holds q, v, and k and then the triangle in one
 // place, so that three blocks share a multiprocessor, or two where q is three terms of 128 channels (rotated, and then k comes in two
-// halves, or with decays per channel).
+// halves, or with decays per channel).  (One block for rotated heads of 128, whose triangle lay behind k: the scan 241 us, now 195.)
 template <int DK, int DV, Mode MODE, bool ROT>
 struct OutSizes {
     static constexpr int NQ = ROT || MODE == VEC ? 3 : 1;     // rotated q and k, and q with its decays, are float32: three terms

@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(1024) group_rows_padded_kernel(const int* __re
 }
 
 // out[p, :] = a[src[p] / div, :] (zeros where src[p] < 0): the rows of a product's input in the padded order.  With tile_group,
-// rows of tiles without a group (a quarter of `cap` at 2,048 tokens of 6 among 64) are left as they are: no product reads them.
+// rows of tiles without a group (a fifth of `cap` at 2,048 tokens of 6 among 64) are left as they are: no product reads them.
 // A block takes GATHER_ROWS rows and asks for all of them before it stores one: 20,480 places for
 // 12,288 rows of 2,048 numbers take 15 us, 23 with a row a block.
 constexpr int GATHER_ROWS = 4;
