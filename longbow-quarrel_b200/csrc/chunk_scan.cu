@@ -15,7 +15,7 @@
 // The state kernel is bound by what a block does per chunk (its products where heads are of 128, its stagers' copies of cosines
 // and sines where they are rotated), the output kernel by the latencies of eight to twelve warps a multiprocessor (tensor cores
 // busy a third of the time).  2,048 tokens of 32 heads, both kernels (and gates), us: heads of 64 rotated 491 token by token
-// (recurrent.cu), 87 here (50 not rotated); with gates 731 and 87; with decays per key channel 397 and 157; heads of
+// (recurrent.cu), 85 here (50 not rotated); with gates 731 and 87; with decays per key channel 397 and 157; heads of
 // 128: 1,165 and 195, 1,264 and 160, 1,915 and 333 (of which prepare 147: exponentials and logarithms, then the halves' sums).
 //
 // Precision: what the recurrence holds in 32 bits stays so.  A float32 operand enters the products as three bfloat16 terms
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) chunk_gates_kernel(const __grid_constant_
             if (lane >= o) run += up;
         }
         const double ahead = __shfl_up_sync(0xffffffffu, run, 1);
-        const double F[2] = {(lane ? ahead : 0.0) + f[0], run};         // (not run - f[1]: a NaN at a token stays behind it)
+        const double F[2] = {f[1] == f[1] ? run - f[1] : (lane ? ahead : 0.0) + f[0], run};      // a NaN at a token stays behind it
         const double down[2] = {(double)i[0] - F[0], (double)i[1] - F[1]};
         double top = fmax(down[0], down[1]);
 #pragma unroll
@@ -1007,55 +1007,60 @@ __global__ void __launch_bounds__(128, 3) chunk_out_kernel(const __grid_constant
                 for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
         }
     }
+    auto row_decays = [&] {
 #pragma unroll
-    for (int i = 0; i < MTB; ++i)
+        for (int i = 0; i < MTB; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float f = MODE == VEC ? 1.f : f_row[(i * WM + wm) * 16 + g + (e >> 1) * 8];
+            for (int e = 0; e < 4; ++e) {
+                const float f = MODE == VEC ? 1.f : f_row[(i * WM + wm) * 16 + g + (e >> 1) * 8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j][e] *= f;
+                for (int j = 0; j < 4; ++j) acc[i][j][e] *= f;
+            }
+    };
+    if (!odd) {
+        row_decays();
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t vb[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                ldsm_x4_t(vp + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + wn * 32 + j * 16 + (lane >> 4) * 8, vb[j]);
+#pragma unroll
+            for (int i = 0; i < MTB; ++i) {
+                const int mi = i * WM + wm;
+                if (kk > mi) continue;             // above the diagonal
+                uint32_t pf[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    ldsm_x4(pp + ((size_t)p * CC + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LP + kk * 16 + (lane >> 4) * 8, pf[p]);
+                float d[4][4] = {};
+#pragma unroll
+                for (int p = 2; p >= 0; --p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) mma_bf16(d[j], pf[p], vb[j / 2][2 * (j & 1)], vb[j / 2][2 * (j & 1) + 1]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
+            }
         }
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-        uint32_t vb[2][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-            ldsm_x4_t(vp + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + wn * 32 + j * 16 + (lane >> 4) * 8, vb[j]);
+    } else {
+        // A value that is not finite must not meet the zeros above the diagonal (0 x NaN is NaN, in rows ahead of its token): the
+        // triangle of such a chunk is added up pair by pair.
+        row_decays();
 #pragma unroll
         for (int i = 0; i < MTB; ++i) {
-            const int mi = i * WM + wm;
-            if (kk > mi || (kk == mi && odd)) continue;      // above the diagonal; see below
-            uint32_t pf[3][4];
-#pragma unroll
-            for (int p = 0; p < 3; ++p)
-                ldsm_x4(pp + ((size_t)p * CC + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LP + kk * 16 + (lane >> 4) * 8, pf[p]);
-            float d[4][4] = {};
-#pragma unroll
-            for (int p = 2; p >= 0; --p)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) mma_bf16(d[j], pf[p], vb[j / 2][2 * (j & 1)], vb[j / 2][2 * (j & 1) + 1]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[i][j][e] += d[j][e];
-        }
-    }
-    // A value that is not finite must not meet the zeros above the diagonal (0 x NaN is NaN, in rows ahead of its token): the
-    // blocks on the diagonal of such a chunk are added up pair by pair.
-    if (odd) {
-#pragma unroll
-        for (int i = 0; i < MTB; ++i) {
-            const int mi = i * WM + wm;
+            const int t0 = (i * WM + wm) * 16 + g;
 #pragma unroll 1
-            for (int s = 0; s < 16; ++s)
+            for (int s = 0; s <= t0 + 8; ++s)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int tt = mi * 16 + g + e * 8;
-                    if (s > g + e * 8) continue;
+                    const int tt = t0 + e * 8;
+                    if (s > tt) continue;
                     float p = 0.f;
 #pragma unroll
-                    for (int x = 2; x >= 0; --x) p += __bfloat162float(pp[((size_t)x * CC + tt) * LP + mi * 16 + s]);
-                    const bf* v = vp + (size_t)(mi * 16 + s) * LV + wn * 32 + 2 * t;
+                    for (int x = 2; x >= 0; --x) p += __bfloat162float(pp[((size_t)x * CC + tt) * LP + s]);
+                    const bf* v = vp + (size_t)s * LV + wn * 32 + 2 * t;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         acc[i][j][2 * e] = fmaf(p, __bfloat162float(v[8 * j]), acc[i][j][2 * e]);
